@@ -13,10 +13,17 @@
 // consumers run without boundary branches.  Consumer warps keep the axis-0
 // neighbours in a register queue whose rotation is resolved at compile time
 // (the plane loop is unrolled by 2H+1), read the in-plane neighbours from the
-// slot with 16-byte loads at offsets fixed per thread, take the stencil
-// coefficients from the kernel-parameter bank, and hand each slot back
+// slot with 16-byte loads at offsets fixed per thread, hold the coefficients
+// of symmetric stencils in registers (star_core.cuh), and hand each slot back
 // through an mbarrier when its last reader is done.  All waits are bounded
 // (tma.cuh).
+//
+// Bound by issue slots more than by HBM: 78 instructions per 32 FP64 points
+// (19 points, radius 3), 94 before the coefficients stayed in registers, the
+// stores and epilogue loads became predicated and the loads moved ahead of
+// the wait.  256 x 96^3 FP64 803 -> 715 us (5.1 of the measured 6.55 TB/s),
+// with a potential 1557 -> 1030 us; 160 x 56^3 FP32 with a potential 120 ->
+// 81 us.  One row per thread instead of two (more warps) was 11 % slower.
 #include <algorithm>
 #include <cstring>
 #include <cstdio>
@@ -26,7 +33,7 @@
 #include <string>
 #include <type_traits>
 #include <cudaTypedefs.h>
-#include "internal.cuh"
+#include "star_core.cuh"
 #include "tma.cuh"
 
 namespace gb {
@@ -99,13 +106,6 @@ struct TmaArgs {
   double alpha, beta, gamma;
 };
 
-// coefficients straight from the kernel-parameter bank (no registers held)
-template <typename R>
-__device__ __forceinline__ R coef(const TmaArgs& a, int c, int m) {
-  if constexpr (sizeof(R) == 8) return a.a[c][m];
-  else return a.af[c][m];
-}
-
 // Slot layout: ROWS rows of `pitch` bytes, logical row r = grid row y0 - H + r
 // (wrapped on a periodic axis 1).  Columns [n2, pitch) of every row are TMA
 // out-of-bounds fill (zeros); on a zero-boundary axis 2 the pitch keeps at
@@ -129,46 +129,42 @@ __device__ __forceinline__ void ldv(const T* p, T (&v)[N]) {
   }
 }
 
-// N consecutive elements from global memory: 16-byte loads when N elements
-// make whole 16-byte chunks (the caller guarantees the alignment), else
-// element loads
+// N consecutive elements from global memory, zeros if !on: 16-byte loads when
+// N elements make whole 16-byte chunks (the caller guarantees the alignment)
 template <typename V, int N>
-__device__ __forceinline__ void ldg_run(const V* __restrict__ p, V (&v)[N]) {
-  if constexpr ((N * sizeof(V)) % 16 == 0) {
+__device__ __forceinline__ void ld_run_if(const V* p, V (&v)[N], bool on) {
+  if constexpr ((N * sizeof(V)) % 16 == 0 && sizeof(V) == 4) {
     constexpr int E = 16 / (int)sizeof(V);
 #pragma unroll
     for (int h = 0; h < N / E; ++h) {
-      const float4 x = __ldg(reinterpret_cast<const float4*>(p) + h);
+      const float4 x = ld4_if(p + h * E, on);
       const V* e = reinterpret_cast<const V*>(&x);
 #pragma unroll
       for (int k = 0; k < E; ++k) v[h * E + k] = e[k];
     }
   } else {
 #pragma unroll
-    for (int c = 0; c < N; ++c) v[c] = p[c];
+    for (int c = 0; c < N; ++c) v[c] = ld_if(p + c, on);
   }
 }
 
-// FP32 taps on two neighbouring points at once (packed f32x2 arithmetic,
-// sm_100): one pair of offsets +k / -k with coefficients cp / cm.  SYM = 1
-// (cp == cm, the Laplacian): c ((vp + vm) - 2 xc), 3 packed operations and
-// exactly zero on a constant; SYM = -1 (cp == -cm, first derivatives):
-// c (vp - vm); SYM = 0: the difference form c (v - xc) per offset.
-template <int SYM>
-__device__ __forceinline__ float2 tap2(float2 acc, float cp, float cm, float2 vp, float2 vm, float2 xc) {
-  const float2 m1 = make_float2(-1.f, -1.f);
-  if constexpr (SYM == 1) {
-    const float2 d = __ffma2_rn(make_float2(-2.f, -2.f), xc, __fadd2_rn(vp, vm));
-    return __ffma2_rn(make_float2(cp, cp), d, acc);
-  } else if constexpr (SYM == -1) {
-    return __ffma2_rn(make_float2(cp, cp), __ffma2_rn(vm, m1, vp), acc);
-  } else {
-    acc = __ffma2_rn(make_float2(cp, cp), __ffma2_rn(xc, m1, vp), acc);
-    return __ffma2_rn(make_float2(cm, cm), __ffma2_rn(xc, m1, vm), acc);
+// predicated streaming store of N elements in 16-byte pieces
+template <typename T, int N>
+__device__ __forceinline__ void st_run_if(T* p, const T (&v)[N], bool on) {
+  constexpr int E = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int h = 0; h < N; h += E) {
+    float4 w;
+    T* e = reinterpret_cast<T*>(&w);
+#pragma unroll
+    for (int k = 0; k < E; ++k) e[k] = v[h + k];
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %5, 0;\n@p st.global.cs.v4.f32 [%0], {%1, %2, %3, %4};\n}\n" ::"l"(p + h),
+                 "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w), "r"((int)on)
+                 : "memory");
   }
 }
 
-template <typename T, int H, int R1, int R2, int VB, int SYM = 0>
+template <typename T, int H, int R1, int R2, int VB, int SYM, int EPI>
 __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ CUtensorMap tmA,
                                                         const __grid_constant__ CUtensorMap tmH,
                                                         const __grid_constant__ CUtensorMap tmB,
@@ -281,13 +277,8 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
     lcol[ch] = own_row + zl * (int)sizeof(T);
     rcol[ch] = own_row + zr * (int)sizeof(T);
   }
-  // FP32: the difference form sum_p c_p (x_p - x_c) + (sum c) x_c keeps the
-  // operator exactly constant-annihilating after the coefficients are rounded
-  // (otherwise every eigenvalue shifts by ~|c0| 2^-24)
-  constexpr bool DIFF = sizeof(R) == 4;
-  constexpr bool PACK = std::is_same<T, float>::value && R2 % 2 == 0;
-  const bool epi = a.alpha != 1.0 || a.beta != 0.0 || a.y != nullptr || a.vpot != nullptr;
-  const R* __restrict__ vpot = reinterpret_cast<const R*>(a.vpot);
+  StarCoef<R, H, SYM> ck;
+  if (SYM == 1) ck.init(a);
 
   T q[NQ][R1][R2];
   int slot = 0;          // ring slot of the current step
@@ -301,9 +292,14 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
     const int64_t band = col / a.ytiles;
     const int y0 = (int)(col % a.ytiles) * T1;
     const int L = p_end - p_start + 2 * H;
-    T* dst = reinterpret_cast<T*>(a.out) + band * n12 * n0;
-    const T* ybase = a.y ? reinterpret_cast<const T*>(a.y) + band * n12 * n0 : nullptr;
     const int yrow = y0 + ty * R1;
+    const int64_t own_g = (int64_t)p_start * n12 + (int64_t)yrow * n2 + tz * R2;
+    T* o = reinterpret_cast<T*>(a.out) + band * n12 * n0 + own_g;
+    const T* yp = EPI == 2 && a.y ? reinterpret_cast<const T*>(a.y) + band * n12 * n0 + own_g : nullptr;
+    const R* vp = EPI && a.vpot ? reinterpret_cast<const R*>(a.vpot) + own_g : nullptr;
+    bool on[R1];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) on[r] = active && yrow + r < n1;
 
     for (int tb = 0; tb < L; tb += NQ) {
 #pragma unroll
@@ -312,6 +308,15 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
         if (t < L) {
         int cslot = slot - H;  // slot of the centre plane (step t - H)
         if (cslot < 0) cslot += NS;
+        T yv[R1][R2];
+        R vv[R1][R2];
+        if (EPI && t >= 2 * H) {
+#pragma unroll
+          for (int r = 0; r < R1; ++r) {
+            if (EPI == 2) ld_run_if<T, R2>(yp + r * n2, yv[r], a.y && on[r]);
+            ld_run_if<R, R2>(vp + r * n2, vv[r], a.vpot && on[r]);
+          }
+        }
         if (!mbar_wait(&full[slot], fph)) {
           raise_device_error(102);
           return;
@@ -323,217 +328,44 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
 
         if (t >= 2 * H) {
           const int cu = (u + NQ - H) % NQ;     // centre plane in the queue (static after unrolling)
-          const int cpl = p_start + t - 2 * H;
           const unsigned char* Pc = slots + (int64_t)cslot * a.slot_bytes;
           T acc[R1][R2];
-          if constexpr (PACK) {
-          // FP32: two points per instruction (f32x2), pairs of columns
-          float2 acc2[R1][R2 / 2];
-          // centre + axis 0 (register queue)
+          star_points<T, H, R1, R2, HZ, SYM>(
+              acc, q, u, ck, a,
+              [&](int r, T(&w)[HZ]) {
 #pragma unroll
-          for (int r = 0; r < R1; ++r)
+                for (int ch = 0; ch < HZ / VEC; ++ch)
+                  ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + lcol[ch] + r * pitch),
+                                  *reinterpret_cast<T(*)[VEC]>(&w[ch * VEC]));
+              },
+              [&](int r, T(&w)[HZ]) {
 #pragma unroll
-            for (int p = 0; p < R2 / 2; ++p) {
-              const float2 xc = make_float2(q[cu][r][2 * p], q[cu][r][2 * p + 1]);
-              float2 x = __fmul2_rn(make_float2(a.c0difff, a.c0difff), xc);
-#pragma unroll
-              for (int k = 1; k <= H; ++k) {
-                const int mp = (u + 1 + H + k) % NQ, mm = (u + 1 + H - k) % NQ;
-                x = tap2<SYM>(x, coef<R>(a, 0, HMAX + k), coef<R>(a, 0, HMAX - k),
-                              make_float2(q[mp][r][2 * p], q[mp][r][2 * p + 1]),
-                              make_float2(q[mm][r][2 * p], q[mm][r][2 * p + 1]), xc);
-              }
-              acc2[r][p] = x;
-            }
-          // axis 2: the row with its halo chunks
-#pragma unroll
-          for (int r = 0; r < R1; ++r) {
-            float w[HZ + R2 + HZ];
-#pragma unroll
-            for (int ch = 0; ch < HZ / VEC; ++ch) {
-              T tl[VEC], tr[VEC];
-              ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + lcol[ch] + r * pitch), tl);
-              ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + rcol[ch] + r * pitch), tr);
-#pragma unroll
-              for (int v = 0; v < VEC; ++v) {
-                w[ch * VEC + v] = tl[v];
-                w[HZ + R2 + ch * VEC + v] = tr[v];
-              }
-            }
-#pragma unroll
-            for (int c = 0; c < R2; ++c) w[HZ + c] = q[cu][r][c];
-#pragma unroll
-            for (int p = 0; p < R2 / 2; ++p) {
-              const int c = HZ + 2 * p;
-              const float2 xc = make_float2(w[c], w[c + 1]);
-              float2 x = acc2[r][p];
-#pragma unroll
-              for (int k = 1; k <= H; ++k)
-                x = tap2<SYM>(x, coef<R>(a, 2, HMAX + k), coef<R>(a, 2, HMAX - k),
-                              make_float2(w[c + k], w[c + 1 + k]), make_float2(w[c - k], w[c + 1 - k]), xc);
-              acc2[r][p] = x;
-            }
-          }
-          // axis 1: rows of the centre slot, streamed (difference form)
-#pragma unroll
-          for (int rr = -H; rr < R1 + H; ++rr) {
-            T v[R2];
-            if (rr >= 0 && rr < R1) {
-#pragma unroll
-              for (int c = 0; c < R2; ++c) v[c] = q[cu][rr][c];
-            } else {
-              ldv<T, R2, VB>(reinterpret_cast<const T*>(Pc + own_row + rr * pitch + own_col), v);
-            }
-#pragma unroll
-            for (int r = 0; r < R1; ++r) {
-              const int d = rr - r;
-              if (d < -H || d > H || d == 0) continue;
-              const float cc = coef<R>(a, 1, HMAX + d);
-#pragma unroll
-              for (int p = 0; p < R2 / 2; ++p) {
-                const float2 xc = make_float2(q[cu][r][2 * p], q[cu][r][2 * p + 1]);
-                const float2 dv = __ffma2_rn(xc, make_float2(-1.f, -1.f), make_float2(v[2 * p], v[2 * p + 1]));
-                acc2[r][p] = __ffma2_rn(make_float2(cc, cc), dv, acc2[r][p]);
-              }
-            }
-          }
-#pragma unroll
-          for (int r = 0; r < R1; ++r)
-#pragma unroll
-            for (int p = 0; p < R2 / 2; ++p) {
-              acc[r][2 * p] = acc2[r][p].x;
-              acc[r][2 * p + 1] = acc2[r][p].y;
-            }
-          } else {
-          // centre + axis 0 (register queue)
-#pragma unroll
-          for (int r = 0; r < R1; ++r)
-#pragma unroll
-            for (int c = 0; c < R2; ++c) {
-              const T xc = q[cu][r][c];
-              T x = scale(DIFF ? (R)a.c0difff : (R)a.c0, xc);
-#pragma unroll
-              for (int m = 0; m < NQ; ++m) {
-                if (m == H) continue;
-                const T v = q[(u + 1 + m) % NQ][r][c];
-                x = fmadd(x, coef<R>(a, 0, m + HMAX - H), DIFF ? sub(v, xc) : v);
-              }
-              acc[r][c] = x;
-            }
-          // axis 2 (halo chunks of the own rows)
-#pragma unroll
-          for (int r = 0; r < R1; ++r) {
-            T wl[HZ], wr[HZ];
-#pragma unroll
-            for (int ch = 0; ch < HZ / VEC; ++ch) {
-              T tl[VEC], tr[VEC];
-              ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + lcol[ch] + r * pitch), tl);
-              ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + rcol[ch] + r * pitch), tr);
-#pragma unroll
-              for (int v = 0; v < VEC; ++v) {
-                wl[ch * VEC + v] = tl[v];
-                wr[ch * VEC + v] = tr[v];
-              }
-            }
-#pragma unroll
-            for (int c = 0; c < R2; ++c) {
-              const T xc = q[cu][r][c];
-#pragma unroll
-              for (int m = 0; m < NQ; ++m) {
-                if (m == H) continue;
-                const int cc = c + m - H;
-                const T v = cc < 0 ? wl[HZ + cc] : (cc >= R2 ? wr[cc - R2] : q[cu][r][cc]);
-                acc[r][c] = fmadd(acc[r][c], coef<R>(a, 2, m + HMAX - H), DIFF ? sub(v, xc) : v);
-              }
-            }
-          }
-          // axis 1 (rows of the centre slot)
-#pragma unroll
-          for (int rr = -H; rr < R1 + H; ++rr) {
-            T v[R2];
-            if (rr >= 0 && rr < R1) {
-#pragma unroll
-              for (int c = 0; c < R2; ++c) v[c] = q[cu][rr][c];
-            } else {
-              ldv<T, R2, VB>(reinterpret_cast<const T*>(Pc + own_row + rr * pitch + own_col), v);
-            }
-#pragma unroll
-            for (int r = 0; r < R1; ++r) {
-              const int m = rr - r + H;
-              if (m < 0 || m > 2 * H || m == H) continue;
-#pragma unroll
-              for (int c = 0; c < R2; ++c)
-                acc[r][c] = fmadd(acc[r][c], coef<R>(a, 1, m + HMAX - H), DIFF ? sub(v[c], q[cu][r][c]) : v[c]);
-            }
-          }
-          }  // PACK
+                for (int ch = 0; ch < HZ / VEC; ++ch)
+                  ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + rcol[ch] + r * pitch),
+                                  *reinterpret_cast<T(*)[VEC]>(&w[ch * VEC]));
+              },
+              [&](int rr, T(&v)[R2]) {
+                if (rr < 0 || rr >= R1) ldv<T, R2, VB>(reinterpret_cast<const T*>(Pc + own_row + rr * pitch + own_col), v);
+              },
+              [](int, int, T v) { return v; });
           // epilogue + streaming stores
-          if (active) {
-            const int64_t pbase = (int64_t)cpl * n12 + (int64_t)yrow * n2 + tz * R2;
 #pragma unroll
-            for (int r = 0; r < R1; ++r) {
-              if (yrow + r >= n1) continue;
-              const int64_t p = pbase + (int64_t)r * n2;
-              if (epi) {
-                if constexpr (sizeof(T) == 4) {
-                  // FP32: y and the potential as 16-byte loads of this
-                  // thread's R2 points (p is a multiple of R2, both bases
-                  // 16-byte aligned); the FP64 kernels run faster, epilogue
-                  // or not, with the element loads below
-                  T yv[R2];
-                  R vv[R2];
-                  if (ybase) ldg_run<T, R2>(ybase + p, yv);
-                  if (vpot) ldg_run<R, R2>(vpot + p, vv);
-                  if constexpr (PACK) {
-                    const float2 al = make_float2((float)a.alpha, (float)a.alpha);
-                    const float2 be = make_float2((float)a.beta, (float)a.beta);
-                    const float2 ga = make_float2((float)a.gamma, (float)a.gamma);
+          for (int r = 0; r < R1; ++r) {
 #pragma unroll
-                    for (int c = 0; c < R2; c += 2) {
-                      const float2 xc = make_float2(q[cu][r][c], q[cu][r][c + 1]);
-                      float2 v = __ffma2_rn(be, xc, __fmul2_rn(al, make_float2(acc[r][c], acc[r][c + 1])));
-                      if (ybase) v = __ffma2_rn(ga, make_float2(yv[c], yv[c + 1]), v);
-                      if (vpot) v = __ffma2_rn(make_float2(vv[c], vv[c + 1]), xc, v);
-                      acc[r][c] = v.x;
-                      acc[r][c + 1] = v.y;
-                    }
-                  } else {
-#pragma unroll
-                  for (int c = 0; c < R2; ++c) {
-                    T v = fmadd(scale((R)a.alpha, acc[r][c]), (R)a.beta, q[cu][r][c]);
-                    if (ybase) v = fmadd(v, (R)a.gamma, yv[c]);
-                    if (vpot) v = fmadd(v, vv[c], q[cu][r][c]);
-                    acc[r][c] = v;
-                  }
-                  }
-                } else {
-#pragma unroll
-                  for (int c = 0; c < R2; ++c) {
-                    T v = fmadd(scale((R)a.alpha, acc[r][c]), (R)a.beta, q[cu][r][c]);
-                    if (ybase) v = fmadd(v, (R)a.gamma, ybase[p + c]);
-                    if (vpot) v = fmadd(v, vpot[p + c], q[cu][r][c]);
-                    acc[r][c] = v;
-                  }
-                }
+            for (int c = 0; c < R2; ++c) {
+              T v = acc[r][c];
+              if (EPI == 2) {
+                v = fmadd(scale((R)a.alpha, v), (R)a.beta, q[cu][r][c]);
+                if (a.y) v = fmadd(v, (R)a.gamma, yv[r][c]);
               }
-#pragma unroll
-              for (int c = 0; c < R2; c += VEC) {
-                if constexpr (VB == 16) {
-                  float4 w4;
-                  T* e = reinterpret_cast<T*>(&w4);
-#pragma unroll
-                  for (int v = 0; v < VEC; ++v) e[v] = acc[r][c + v];
-                  __stcs(reinterpret_cast<float4*>(dst + p + c), w4);
-                } else {
-                  float2 w2;
-                  T* e = reinterpret_cast<T*>(&w2);
-#pragma unroll
-                  for (int v = 0; v < VEC; ++v) e[v] = acc[r][c + v];
-                  __stcs(reinterpret_cast<float2*>(dst + p + c), w2);
-                }
-              }
+              if (EPI && a.vpot) v = fmadd(v, vv[r][c], q[cu][r][c]);
+              acc[r][c] = v;
             }
+            st_run_if<T, R2>(o + r * n2, acc[r], on[r]);
           }
+          o += n12;
+          if (EPI == 2) yp += yp ? n12 : 0;
+          if (EPI) vp += vp ? n12 : 0;
         }
         // hand back the slot read as centre plane (its last reader was this step)
         if (t >= H) {
@@ -558,13 +390,13 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
 }
 
 // ------------------------------------------------------------------ host
-template <typename T, int H, int R1, int R2, int VB = 16, int SYM = 0>
+template <typename T, int H, int R1, int R2, int VB, int SYM, int EPI>
 static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int64_t nin, cudaStream_t st,
                           const Epilogue& ep) {
   using R = typename Elem<T>::R;
   const int n0 = (int)op->n[0], n1 = (int)op->n[1], n2 = (int)op->n[2];
   const int TZ = n2 / R2;
-  auto kern = star_tma_kernel<T, H, R1, R2, VB, SYM>;
+  auto kern = star_tma_kernel<T, H, R1, R2, VB, SYM, EPI>;
   static int regs = -1;
   if (regs < 0) {
     cudaFuncAttributes fa;
@@ -756,6 +588,46 @@ static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int6
   return launch(choice);
 }
 
+// Instantiations: symmetric stencils of the radii the path uses (1 and 3: the
+// kinetic operators of the three multigrid levels) with each epilogue (none,
+// potential, general); first derivatives in FP32; everything else general.
+template <typename T, int R2>
+static int dispatch_tma(const gb_operator* op, const void* in, void* out, int64_t nin, cudaStream_t st,
+                        const Epilogue& ep) {
+  bool sym = true, anti = std::is_same<T, float>::value;
+  for (int c = 0; c < 3; ++c)
+    for (int k = 1; k <= HMAX; ++k) {
+      using R = typename Elem<T>::R;
+      const R p = (R)op->a[c][HMAX + k], m = (R)op->a[c][HMAX - k];
+      sym = sym && p == m;
+      anti = anti && p == -m;
+    }
+  const int epi = ep.y || ep.alpha != 1.0 || ep.beta != 0.0 ? 2 : ep.vpot ? 1 : 0;
+  if (sym && (op->H == 1 || op->H == 3)) {
+    if (op->H == 1)
+      return epi == 2 ? launch_tma_cfg<T, 1, 2, R2, 16, 1, 2>(op, in, out, nin, st, ep)
+                      : launch_tma_cfg<T, 1, 2, R2, 16, 1, 1>(op, in, out, nin, st, ep);
+    switch (epi) {
+      case 0: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 0>(op, in, out, nin, st, ep);
+      case 1: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 1>(op, in, out, nin, st, ep);
+      default: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 2>(op, in, out, nin, st, ep);
+    }
+  }
+  if constexpr (std::is_same<T, float>::value)
+    if (anti) switch (op->H) {
+        case 1: return launch_tma_cfg<T, 1, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
+        case 2: return launch_tma_cfg<T, 2, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
+        case 3: return launch_tma_cfg<T, 3, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
+        default: return launch_tma_cfg<T, 4, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
+      }
+  switch (op->H) {
+    case 1: return launch_tma_cfg<T, 1, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
+    case 2: return launch_tma_cfg<T, 2, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
+    case 3: return launch_tma_cfg<T, 3, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
+    default: return launch_tma_cfg<T, 4, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
+  }
+}
+
 static int g_stencil_path = 0;   // 0 auto, 1 cp.async only, 2 TMA required
 const char* tma_reason() { return g_tma_reason; }
 
@@ -779,51 +651,10 @@ int star_tma_apply(const gb_operator* op, const void* in, void* out, int64_t nin
   if (ep.vpot && (reinterpret_cast<uintptr_t>(ep.vpot) & 15)) { g_tma_reason = "unaligned potential"; return 1; }
   if (op->n[0] < op->H || op->n[1] < op->H || op->n[2] < 8) { g_tma_reason = "grid shorter than the stencil"; return 1; }
   switch (dtype) {
-    case GB_DTYPE_F64:
-      switch (op->H) {
-        case 1: return launch_tma_cfg<double, 1, 2, 2>(op, in, out, nin, st, ep);
-        case 2: return launch_tma_cfg<double, 2, 2, 2>(op, in, out, nin, st, ep);
-        case 3: return launch_tma_cfg<double, 3, 2, 2>(op, in, out, nin, st, ep);
-        default: return launch_tma_cfg<double, 4, 2, 2>(op, in, out, nin, st, ep);
-      }
-    case GB_DTYPE_F32: {
-      // coefficient symmetry of every axis, in FP32: symmetric pairs (the
-      // Laplacian) and antisymmetric pairs (derivatives) take fewer
-      // operations in the packed kernel
-      bool sym = true, anti = true;
-      for (int c = 0; c < 3; ++c)
-        for (int k = 1; k <= HMAX; ++k) {
-          const float p = (float)op->a[c][HMAX + k], m = (float)op->a[c][HMAX - k];
-          sym = sym && p == m;
-          anti = anti && p == -m;
-        }
-      const int kind = sym ? 1 : (anti ? -1 : 0);
-#define GB_F32_TMA(HH)                                                                      \
-  return kind == 1 ? launch_tma_cfg<float, HH, 2, 4, 16, 1>(op, in, out, nin, st, ep)       \
-                   : kind == -1 ? launch_tma_cfg<float, HH, 2, 4, 16, -1>(op, in, out, nin, st, ep) \
-                                : launch_tma_cfg<float, HH, 2, 4, 16, 0>(op, in, out, nin, st, ep)
-      switch (op->H) {
-        case 1: GB_F32_TMA(1);
-        case 2: GB_F32_TMA(2);
-        case 3: GB_F32_TMA(3);
-        default: GB_F32_TMA(4);
-      }
-#undef GB_F32_TMA
-    }
-    case GB_DTYPE_C128:
-      switch (op->H) {
-        case 1: return launch_tma_cfg<double2, 1, 2, 1>(op, in, out, nin, st, ep);
-        case 2: return launch_tma_cfg<double2, 2, 2, 1>(op, in, out, nin, st, ep);
-        case 3: return launch_tma_cfg<double2, 3, 2, 1>(op, in, out, nin, st, ep);
-        default: return launch_tma_cfg<double2, 4, 2, 1>(op, in, out, nin, st, ep);
-      }
-    default:
-      switch (op->H) {
-        case 1: return launch_tma_cfg<float2, 1, 2, 2>(op, in, out, nin, st, ep);
-        case 2: return launch_tma_cfg<float2, 2, 2, 2>(op, in, out, nin, st, ep);
-        case 3: return launch_tma_cfg<float2, 3, 2, 2>(op, in, out, nin, st, ep);
-        default: return launch_tma_cfg<float2, 4, 2, 2>(op, in, out, nin, st, ep);
-      }
+    case GB_DTYPE_F64: return dispatch_tma<double, 2>(op, in, out, nin, st, ep);
+    case GB_DTYPE_F32: return dispatch_tma<float, 4>(op, in, out, nin, st, ep);
+    case GB_DTYPE_C128: return dispatch_tma<double2, 1>(op, in, out, nin, st, ep);
+    default: return dispatch_tma<float2, 2>(op, in, out, nin, st, ep);
   }
 }
 

@@ -52,6 +52,17 @@ struct gb_operator {
 };
 
 
+namespace gb {
+// coefficients equal on both sides of every axis, in the working precision
+template <typename R>
+inline bool symmetric_stencil(const gb_operator* op) {
+  for (int c = 0; c < 3; ++c)
+    for (int k = 1; k <= HMAX; ++k)
+      if ((R)op->a[c][HMAX + k] != (R)op->a[c][HMAX - k]) return false;
+  return true;
+}
+}  // namespace gb
+
 struct gb_transformer {
   int64_t nin_c[3], nout_c[3];
   int k;              // 2 * nn
