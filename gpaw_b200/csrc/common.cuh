@@ -67,12 +67,14 @@ __device__ __forceinline__ float2  sub(float2 a, float2 b)   { return make_float
 // arrays, c/operators.c:270-273).
 __device__ __forceinline__ double  phase_mul(double a, double, double)  { return a; }
 __device__ __forceinline__ float   phase_mul(float a, double, double)   { return a; }
+// (explicit operations: every kernel rounds a wrapped cell alike, whatever the
+// compiler would contract around it)
 __device__ __forceinline__ double2 phase_mul(double2 a, double pr, double pi) {
-  return make_double2(a.x * pr - a.y * pi, a.x * pi + a.y * pr);
+  return make_double2(__fma_rn(a.x, pr, -__dmul_rn(a.y, pi)), __fma_rn(a.x, pi, __dmul_rn(a.y, pr)));
 }
 __device__ __forceinline__ float2 phase_mul(float2 a, double pr, double pi) {
-  float r = (float)pr, i = (float)pi;
-  return make_float2(a.x * r - a.y * i, a.x * i + a.y * r);
+  const float r = (float)pr, i = (float)pi;
+  return make_float2(__fmaf_rn(a.x, r, -__fmul_rn(a.y, i)), __fmaf_rn(a.x, i, __fmul_rn(a.y, r)));
 }
 
 // ---------------------------------------------------------------- async copies
@@ -105,6 +107,19 @@ __device__ __forceinline__ void st_cs(double* p, double v) { __stcs(p, v); }
 __device__ __forceinline__ void st_cs(float* p, float v) { __stcs(p, v); }
 __device__ __forceinline__ void st_cs(double2* p, double2 v) { __stcs(p, v); }
 __device__ __forceinline__ void st_cs(float2* p, float2 v) { __stcs(p, v); }
+
+// a / b and a % b for 0 <= a, 0 < b: 32-bit division when it fits (a 64-bit
+// one costs as much as a whole point of the kernels that index with it)
+__device__ __forceinline__ int64_t div_mod(int64_t a, int b, int& r) {
+  if ((a >> 31) == 0) {
+    const unsigned q = (unsigned)a / (unsigned)b;
+    r = (int)((unsigned)a - q * (unsigned)b);
+    return q;
+  }
+  const int64_t q = a / b;
+  r = (int)(a - q * b);
+  return q;
+}
 
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 

@@ -1,18 +1,17 @@
 // FD stencil operator (replaces _gpaw.Operator: c/operators.c, c/bmgs/fd.c,
-// c/bc.c).  Two kernels:
+// c/bc.c).  Stencils whose points all lie on the three axes (the reference's
+// "cfd" case: Laplace on orthorhombic cells, Gradient) take, in this order,
+// the TMA kernel of fd_stencil_tma.cu, the row kernel of fd_stencil_rows.cu
+// and the kernel here:
 //
-//  * star_kernel  -- stencils whose points all lie on the three axes (the
-//    reference's "cfd" case: Laplace on orthorhombic cells, Gradient).  A
-//    persistent CTA owns a (T1 x T2) tile of the (axis1, axis2) plane of one
-//    grid and marches along axis 0.  Planes (tile + halo) stream through a
-//    ring of NS shared-memory slots filled by cp.async (LDGSTS, no register
-//    staging, D planes in flight); every thread keeps a register queue of
-//    2H+1 values of its own R1 x R2 points along axis 0, so each input
-//    element is read from HBM once and from shared memory ~5-7 times.
-//    Zero and periodic boundaries (with Bloch phases) are resolved while
-//    filling the tile: out-of-range cells become zeros or wrapped copies,
-//    wrapped copies of complex data are multiplied by the phase in a short
-//    fix-up pass (only tiles that touch a periodic face pay it).
+//  * march_star_kernel -- any layout, boundary mix, phases and radius up to 6.
+//    One thread per (axis1, axis2) column marches along axis 0 with a
+//    register queue; its in-plane neighbours are read through L1.  There is
+//    no staging and no barrier, so it is the fastest form while a call is too
+//    small to fill the pipelines of the other two (every SM busy for less
+//    than ~16 plane tiles), and with 7-point FP32 stencils, which read too
+//    few neighbours to be bound by L1 (four 31^3 FP64 grids 13 us against
+//    33 us in the row kernel; 160 x 37^3 FP32, radius 1: 33 against 37 us).
 //
 //  * box_kernel   -- any stencil (off-axis points of GUC Laplacians /
 //    non-orthogonal gradients, c/bmgs/fd.c generic loop).  3-D tile with a
@@ -26,6 +25,7 @@
 #include <cmath>
 #include <cstring>
 #include <algorithm>
+#include <type_traits>
 #include "internal.cuh"
 
 namespace gb {
@@ -37,7 +37,7 @@ struct StarArgs {
   int64_t nbatch;
   int n0, n1, n2;
   int pbc0, pbc1, pbc2;
-  int tiles1, tiles2;
+  int tiles, chunks;          // column tiles of a plane, chunks of planes
   double c0;
   double c0diff;              // c0 + sum of the neighbour coefficients (difference form)
   double a[3][2 * HMAX + 1];  // a[axis][m + HMAX]: coefficient of offset m (m != 0)
@@ -48,26 +48,6 @@ struct StarArgs {
   const void* vpot;
 };
 
-template <typename T_, int H_, int R1_, int R2_, int TY_, int TZ_, int D_>
-struct StarCfg {
-  using T = T_;
-  static constexpr int H = H_, R1 = R1_, R2 = R2_, TY = TY_, TZ = TZ_, D = D_;
-  static constexpr int VEC = 16 / (int)sizeof(T);
-  static constexpr int HZ = ((H + VEC - 1) / VEC) * VEC;
-  static constexpr int T1 = TY * R1, T2 = TZ * R2;
-  static constexpr int W = T2 + 2 * HZ;
-  static constexpr int ROWS = T1 + 2 * H;
-  static constexpr int PLANE = ROWS * W;
-  static constexpr int NS = H + D;
-  static constexpr int NT = TY * TZ;
-  static constexpr int KH = T2 / VEC;       // chunks in a halo row
-  static constexpr int KC = W / VEC;        // chunks in a centre row
-  static constexpr int NCHUNK = 2 * H * KH + T1 * KC;
-  static constexpr size_t SMEM = (size_t)NS * PLANE * sizeof(T);
-  static_assert(R2 % VEC == 0, "R2 must be a multiple of the 16-byte vector");
-  static_assert((W * sizeof(T)) % 16 == 0, "row pitch must keep 16-byte alignment");
-};
-
 // true modulo: partial tiles of small grids can reach several periods away
 // (those cells feed no valid output, but their loads must stay in bounds)
 __device__ __forceinline__ int wrap_index(int i, int n) {
@@ -75,283 +55,191 @@ __device__ __forceinline__ int wrap_index(int i, int n) {
   return r < 0 ? r + n : r;
 }
 
-template <class C>
-__global__ void __launch_bounds__(C::NT, 2) star_kernel(const StarArgs args) {
-  using T = typename C::T;
+// One term of the stencil, in the order and form of star_core.cuh: centre,
+// axis 0, axis 2, axis 1, offsets ascending; FP32 as differences, axes 0 and 2
+// in pairs of offsets.  A band's result is then the same, bit for bit, in this
+// kernel and in the row kernel, so it does not depend on how many bands a call
+// has.
+template <typename T>
+__device__ __forceinline__ T star_term(T acc, typename Elem<T>::R c, T v, T xc) {
+  return fmadd(acc, c, sizeof(typename Elem<T>::R) == 4 ? sub(v, xc) : v);
+}
+
+template <bool SYM>
+__device__ __forceinline__ float star_pair(float acc, float cp, float cm, float vp, float vm, float xc) {
+  if constexpr (SYM) return fmaf(cp, fmaf(-2.f, xc, vp + vm), acc);
+  acc = fmaf(cp, vp - xc, acc);
+  return fmaf(cm, vm - xc, acc);
+}
+
+__device__ __forceinline__ double ld_nc(const double* p) { return __ldg(p); }
+__device__ __forceinline__ float ld_nc(const float* p) { return __ldg(p); }
+__device__ __forceinline__ double2 ld_nc(const double2* p) { return __ldg(p); }
+__device__ __forceinline__ float2 ld_nc(const float2* p) { return __ldg(p); }
+
+template <typename T, int H, bool PER, bool SYM>
+__global__ void __launch_bounds__(256, sizeof(T) == 16 ? 2 : 3) march_star_kernel(const __grid_constant__ StarArgs a) {
   using R = typename Elem<T>::R;
-  constexpr int H = C::H, R1 = C::R1, R2 = C::R2, TZ = C::TZ, VEC = C::VEC, HZ = C::HZ;
-  constexpr int T1 = C::T1, T2 = C::T2, W = C::W, PLANE = C::PLANE, NS = C::NS, D = C::D;
   constexpr bool CPLX = Elem<T>::cplx;
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* planes = reinterpret_cast<T*>(smem_raw);
-
-  const int tid = threadIdx.x;
-  const int ty = tid / TZ, tz = tid % TZ;
-  const int n0 = args.n0, n1 = args.n1, n2 = args.n2;
-  const int64_t n12 = (int64_t)n1 * n2;
-  const int64_t n012 = n12 * n0;
-  const int64_t ntiles = (int64_t)args.tiles1 * args.tiles2;
-  const int64_t total = args.nbatch * ntiles * n0;
-  int64_t s = total * blockIdx.x / gridDim.x;
-  const int64_t s_end = total * (blockIdx.x + 1) / gridDim.x;
-
-  const bool epi = args.alpha != 1.0 || args.beta != 0.0 || args.y != nullptr || args.vpot != nullptr;
-  const R* __restrict__ vpot = reinterpret_cast<const R*>(args.vpot);
-  const R ealpha = (R)args.alpha, ebeta = (R)args.beta, egamma = (R)args.gamma;
-  // FP32: the difference form sum_p c_p (x_p - x_c) + (sum c) x_c keeps the
-  // operator exactly constant-annihilating after the coefficients are rounded
   constexpr bool DIFF = sizeof(R) == 4;
-  R c0 = DIFF ? (R)args.c0diff : (R)args.c0;
-  R a0[2 * H + 1], a1[2 * H + 1], a2[2 * H + 1];
-#pragma unroll
-  for (int m = 0; m <= 2 * H; ++m) {
-    a0[m] = (R)args.a[0][m - H + HMAX];
-    a1[m] = (R)args.a[1][m - H + HMAX];
-    a2[m] = (R)args.a[2][m - H + HMAX];
-  }
+  constexpr int R1 = 1;                     // rows per thread (2 and 3 were slower: fewer warps)
+  constexpr int NQ = 2 * H + 2;             // 2H + 1 planes in use, one on its way
+  const int n0 = a.n0, n1 = a.n1, n2 = a.n2;
+  const int64_t n12 = (int64_t)n1 * n2;
+  unsigned u0 = blockIdx.x;
+  const unsigned tile = u0 % a.tiles;
+  u0 /= a.tiles;
+  const int chunk = u0 % a.chunks;
+  const int64_t band = u0 / a.chunks;
+  const int64_t f = (int64_t)tile * 256 + threadIdx.x;
+  int z;
+  const int y0 = (int)div_mod(f, n2, z) * R1;
+  if (y0 >= n1) return;
+  const int p_begin = (int)((int64_t)n0 * chunk / a.chunks), p_end = (int)((int64_t)n0 * (chunk + 1) / a.chunks);
 
-  while (s < s_end) {
-    const int64_t col = s / n0;
-    const int p_start = (int)(s % n0);
-    const int p_end = (int)(s_end - s < (int64_t)(n0 - p_start) ? p_start + (s_end - s) : n0);
-    s += p_end - p_start;
-    const int64_t band = col / ntiles;
-    const int t = (int)(col % ntiles);
-    const int y0 = (t / args.tiles2) * T1;
-    const int z0 = (t % args.tiles2) * T2;
-    const T* __restrict__ src = reinterpret_cast<const T*>(args.in) + band * n012;
-    T* __restrict__ dst = reinterpret_cast<T*>(args.out) + band * n012;
-    const T* __restrict__ ybase = args.y ? reinterpret_cast<const T*>(args.y) + band * n012 : nullptr;
-    const auto& PH = args.phs.ph[phase_set_of(args.phs, band)];
-    const bool edge = (y0 - H < 0) || (y0 + T1 + H > n1) || (z0 - HZ < 0) || (z0 + T2 + HZ > n2);
+  const T* __restrict__ src = reinterpret_cast<const T*>(a.in) + band * n12 * n0 + ((int64_t)y0 * n2 + z);
+  const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
+  const bool phased = CPLX && PER && a.phs.any;
 
-    const int j0 = p_start - H, j1 = p_end + H;   // planes pushed: [j0, j1)
-
-    // plane j -> source plane (or -1 for an all-zero plane) and its phase
-    auto plane_src = [&](int j, double& pr, double& pi) -> int {
-      pr = 1.0; pi = 0.0;
-      if (j >= 0 && j < n0) return j;
-      if (!args.pbc0) return -1;
-      const int side = j < 0 ? 1 : 0;
-      pr = PH[0][side][0]; pi = PH[0][side][1];
-      return wrap_index(j, n0);
-    };
-
-    auto issue = [&](int j) {
-      double pr, pi;
-      const int sp = plane_src(j, pr, pi);
-      if (sp < 0) return;
-      T* P = planes + ((j - j0) % NS) * PLANE;
-      const T* S = src + (int64_t)sp * n12;
-      for (int e = tid; e < C::NCHUNK; e += C::NT) {
-        int Rw, k;
-        if (e < 2 * H * C::KH) {
-          const int hr = e / C::KH;
-          Rw = hr < H ? hr : hr + T1;
-          k = HZ / VEC + e % C::KH;
-        } else {
-          const int e2 = e - 2 * H * C::KH;
-          Rw = H + e2 / C::KC;
-          k = e2 % C::KC;
-        }
-        T* sd = P + Rw * W + k * VEC;
-        int y = y0 - H + Rw;
-        if (y < 0 || y >= n1) {
-          if (!args.pbc1) {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) sd[v] = zero<T>();
-            continue;
-          }
-          y = wrap_index(y, n1);
-        }
-        const T* row = S + (int64_t)y * n2;
-        const int zs = z0 - HZ + k * VEC;
-        if (zs >= 0 && zs + VEC <= n2 && ((reinterpret_cast<uintptr_t>(row + zs) & 15) == 0)) {
-          cp_async16(sd, row + zs);
-        } else {
-#pragma unroll
-          for (int v = 0; v < VEC; ++v) {
-            int z = zs + v;
-            if (z < 0 || z >= n2) {
-              if (!args.pbc2) { sd[v] = zero<T>(); continue; }
-              z = wrap_index(z, n2);
-            }
-            cp_async_elem(sd + v, row + z);
-          }
-        }
-      }
-    };
-
-    // Bloch phase of wrapped in-plane cells (complex data only)
-    auto fixup = [&](T* P) {
-      for (int e = tid; e < C::NCHUNK * VEC; e += C::NT) {
-        const int ec = e / VEC, v = e % VEC;
-        int Rw, k;
-        if (ec < 2 * H * C::KH) {
-          const int hr = ec / C::KH;
-          Rw = hr < H ? hr : hr + T1;
-          k = HZ / VEC + ec % C::KH;
-        } else {
-          const int e2 = ec - 2 * H * C::KH;
-          Rw = H + e2 / C::KC;
-          k = e2 % C::KC;
-        }
-        const int y = y0 - H + Rw, z = z0 - HZ + k * VEC + v;
-        double pr = 1.0, pi = 0.0;
-        bool w = false;
-        if (args.pbc1 && (y < 0 || y >= n1)) { const int sd = y < 0; pr = PH[1][sd][0]; pi = PH[1][sd][1]; w = true; }
-        if (args.pbc2 && (z < 0 || z >= n2)) {
-          const int sd = z < 0;
-          const double qr = PH[2][sd][0], qi = PH[2][sd][1];
-          const double tr = pr * qr - pi * qi, ti = pr * qi + pi * qr;
-          pr = tr; pi = ti; w = true;
-        }
-        if (w) { T* c = P + Rw * W + k * VEC + v; *c = phase_mul(*c, pr, pi); }
-      }
-    };
-
-    T q[2 * H + 1][R1][R2];
-#pragma unroll
-    for (int m = 0; m <= 2 * H; ++m)
-#pragma unroll
-      for (int r = 0; r < R1; ++r)
-#pragma unroll
-        for (int c = 0; c < R2; ++c) q[m][r][c] = zero<T>();
-
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (j0 + d < j1) issue(j0 + d);
-      cp_async_commit();
+  // Row y0 + d relative to the thread's own point: the flat offset (wrapped on
+  // a periodic axis), whether it holds data, and whether it wraps
+  auto row = [&](int d, int64_t& off, bool& ok, int& side) {
+    const int y = y0 + d;
+    off = (int64_t)d * n2;
+    side = y < 0 ? 1 : y >= n1 ? 0 : -1;
+    ok = side < 0;
+    if (PER && a.pbc1 && !ok) {
+      off += side ? n12 : -n12;
+      ok = true;
     }
-
-    for (int j = j0; j < j1; ++j) {
-      cp_async_wait<D - 1>();
-      __syncthreads();
-      double pr, pi;
-      const int sp = plane_src(j, pr, pi);
-      T* P = planes + ((j - j0) % NS) * PLANE;
-      if (CPLX && args.phs.any && edge && sp >= 0) {
-        fixup(P);
-        __syncthreads();
+  };
+  // value of the centre plane's row d (rows of the own block come from the queue)
+  auto ld_row = [&](const T* c, int d) -> T {
+    int64_t off;
+    int side;
+    bool ok;
+    row(d, off, ok, side);
+    T v = zero<T>();
+    if (ok) v = ld_nc(c + off);
+    if (phased && side >= 0) v = phase_mul(v, PH[1][side][0], PH[1][side][1]);
+    return v;
+  };
+  auto ld_col = [&](const T* c, int d) -> T {
+    const int zz = z + d;
+    int off = d;
+    int side = zz < 0 ? 1 : zz >= n2 ? 0 : -1;
+    bool ok = side < 0;
+    if (PER && a.pbc2 && !ok) {
+      off += side ? n2 : -n2;
+      ok = true;
+    }
+    T v = zero<T>();
+    if (ok) v = ld_nc(c + off);
+    if (phased && side >= 0) v = phase_mul(v, PH[2][side][0], PH[2][side][1]);
+    return v;
+  };
+  // own block of plane j (any j; zero or wrapped outside the grid)
+  int64_t ooff[R1];
+  bool ook[R1];
+  int oside[R1];
+#pragma unroll
+  for (int r = 0; r < R1; ++r) row(r, ooff[r], ook[r], oside[r]);
+  auto ld_plane = [&](int j, T (&v)[R1]) {
+    int side = j < 0 ? 1 : j >= n0 ? 0 : -1;
+    bool in = side < 0;
+    if (PER && a.pbc0 && !in) {
+      j += side ? n0 : -n0;
+      in = true;
+    }
+    const T* c = src + (int64_t)j * n12;
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      v[r] = zero<T>();
+      if (in && ook[r]) v[r] = ld_nc(c + ooff[r]);
+      if (phased) {
+        if (oside[r] >= 0) v[r] = phase_mul(v[r], PH[1][oside[r]][0], PH[1][oside[r]][1]);
+        if (side >= 0) v[r] = phase_mul(v[r], PH[0][side][0], PH[0][side][1]);
       }
-      // push own values of plane j into the axis-0 queue
-#pragma unroll
-      for (int m = 0; m < 2 * H; ++m)
-#pragma unroll
-        for (int r = 0; r < R1; ++r)
-#pragma unroll
-          for (int c = 0; c < R2; ++c) q[m][r][c] = q[m + 1][r][c];
-      if (sp >= 0) {
-#pragma unroll
-        for (int r = 0; r < R1; ++r) {
-          T v[R2];
-          lds_vec<T, R2>(P + (H + ty * R1 + r) * W + HZ + tz * R2, v);
-#pragma unroll
-          for (int c = 0; c < R2; ++c) q[2 * H][r][c] = CPLX ? phase_mul(v[c], pr, pi) : v[c];
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R1; ++r)
-#pragma unroll
-          for (int c = 0; c < R2; ++c) q[2 * H][r][c] = zero<T>();
-      }
+    }
+  };
 
-      const int cpl = j - H;   // centre plane computed this iteration
-      if (cpl >= p_start) {
-        const T* Pc = planes + ((cpl - j0) % NS) * PLANE;
-        T acc[R1][R2];
-        // axis 0 (register queue) and axis 2 (row windows)
+  const bool epi = a.alpha != 1.0 || a.beta != 0.0 || a.y != nullptr || a.vpot != nullptr;
+  const R c0 = DIFF ? (R)a.c0diff : (R)a.c0;
+  const int64_t obase = band * n12 * n0 + ((int64_t)y0 * n2 + z);
+  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + obase;
+  const T* __restrict__ ysrc = a.y ? reinterpret_cast<const T*>(a.y) + obase : nullptr;
+  const R* __restrict__ vsrc = a.vpot ? reinterpret_cast<const R*>(a.vpot) + ((int64_t)y0 * n2 + z) : nullptr;
+
+  // q[(s + H) % NQ]: plane p_begin + s
+  T q[NQ][R1];
 #pragma unroll
-        for (int r = 0; r < R1; ++r) {
-          const T* rowp = Pc + (H + ty * R1 + r) * W + tz * R2;
-          T wl[HZ], wr[HZ];
-          lds_vec<T, HZ>(rowp, wl);
-          lds_vec<T, HZ>(rowp + HZ + R2, wr);
+  for (int s = -H; s <= H; ++s) ld_plane(p_begin + s, q[s + H]);
+  for (int pb = p_begin; pb < p_end; pb += NQ) {
 #pragma unroll
-          for (int c = 0; c < R2; ++c) {
-            T x = scale(c0, q[H][r][c]);
-#pragma unroll
-            for (int m = 0; m <= 2 * H; ++m)
-              if (m != H) x = fmadd(x, a0[m], DIFF ? sub(q[m][r][c], q[H][r][c]) : q[m][r][c]);
-#pragma unroll
-            for (int m = 0; m <= 2 * H; ++m) {
-              if (m == H) continue;
-              const int cc = c + m - H;
-              T v;
-              if (cc < 0) v = wl[HZ + cc];
-              else if (cc >= R2) v = wr[cc - R2];
-              else v = q[H][r][cc];
-              x = fmadd(x, a2[m], DIFF ? sub(v, q[H][r][c]) : v);
-            }
-            acc[r][c] = x;
-          }
-        }
-        // axis 1: rows of the own block come from the queue, others from smem
-#pragma unroll
-        for (int rr = -H; rr < R1 + H; ++rr) {
-          T v[R2];
-          if (rr >= 0 && rr < R1) {
-#pragma unroll
-            for (int c = 0; c < R2; ++c) v[c] = q[H][rr][c];
-          } else {
-            lds_vec<T, R2>(Pc + (H + ty * R1 + rr) * W + HZ + tz * R2, v);
-          }
-#pragma unroll
-          for (int r = 0; r < R1; ++r) {
-            const int m = rr - r + H;
-            if (m < 0 || m > 2 * H || m == H) continue;
-#pragma unroll
-            for (int c = 0; c < R2; ++c)
-              acc[r][c] = fmadd(acc[r][c], a1[m], DIFF ? sub(v[c], q[H][r][c]) : v[c]);
-          }
-        }
-        // epilogue (fused axpy passes of the multigrid V-cycle)
+    for (int u = 0; u < NQ; ++u) {
+      const int p = pb + u;
+      if (p < p_end) {
+        if (p + 1 < p_end) ld_plane(p + 1 + H, q[(u + 2 * H + 1) % NQ]);
+        const int64_t po = (int64_t)p * n12;
+        const T* c = src + po;
+        const int cu = (u + H) % NQ;
+        T yv[R1];
+        R vv[R1];
         if (epi) {
-          const T* yp = ybase ? ybase + (int64_t)cpl * n12 : nullptr;
 #pragma unroll
           for (int r = 0; r < R1; ++r) {
-            const int y = y0 + ty * R1 + r;
-#pragma unroll
-            for (int c = 0; c < R2; ++c) {
-              const int z = z0 + tz * R2 + c;
-              T v = fmadd(scale(ealpha, acc[r][c]), ebeta, q[H][r][c]);
-              if (yp && y < n1 && z < n2) v = fmadd(v, egamma, yp[(int64_t)y * n2 + z]);
-              if (vpot && y < n1 && z < n2) v = fmadd(v, vpot[(int64_t)cpl * n12 + (int64_t)y * n2 + z], q[H][r][c]);
-              acc[r][c] = v;
-            }
+            if (ysrc && y0 + r < n1) yv[r] = __ldcs(ysrc + po + r * n2);
+            if (vsrc && y0 + r < n1) vv[r] = __ldg(vsrc + po + r * n2);
           }
         }
-        // store
-        T* outp = dst + (int64_t)cpl * n12;
+        T acc[R1];
 #pragma unroll
         for (int r = 0; r < R1; ++r) {
-          const int y = y0 + ty * R1 + r;
-          if (y >= n1) continue;
-          T* o = outp + (int64_t)y * n2;
-          const int z = z0 + tz * R2;
-          if (z + R2 <= n2 && ((reinterpret_cast<uintptr_t>(o + z) & 15) == 0)) {
+          const T xc = q[cu][r];
+          T x = scale(c0, xc);
 #pragma unroll
-            for (int c = 0; c < R2; c += VEC) {
-              float4 w4;
-              T* e = reinterpret_cast<T*>(&w4);
-#pragma unroll
-              for (int k = 0; k < VEC; ++k) e[k] = acc[r][c + k];
-              __stcs(reinterpret_cast<float4*>(o + z + c), w4);
+          for (int m = -H; m <= H; ++m) {
+            if constexpr (std::is_same<T, float>::value) {
+              if (m > 0)
+                x = star_pair<SYM>(x, (R)a.a[0][HMAX + m], (R)a.a[0][HMAX - m], q[(u + H + m + NQ) % NQ][r],
+                                   q[(u + H - m + NQ) % NQ][r], xc);
+            } else {
+              if (m) x = star_term(x, (R)a.a[0][m + HMAX], q[(u + H + m + NQ) % NQ][r], xc);
             }
-          } else {
-#pragma unroll
-            for (int c = 0; c < R2; ++c)
-              if (z + c < n2) st_cs(o + z + c, acc[r][c]);
           }
+#pragma unroll
+          for (int m = -H; m <= H; ++m) {
+            if constexpr (std::is_same<T, float>::value) {
+              if (m > 0)
+                x = star_pair<SYM>(x, (R)a.a[2][HMAX + m], (R)a.a[2][HMAX - m], ld_col(c + ooff[r], m),
+                                   ld_col(c + ooff[r], -m), xc);
+            } else {
+              if (m) x = star_term(x, (R)a.a[2][m + HMAX], ld_col(c + ooff[r], m), xc);
+            }
+          }
+          acc[r] = x;
+        }
+#pragma unroll
+        for (int d = -H; d < R1 + H; ++d) {
+          const T v = d >= 0 && d < R1 ? q[cu][d < 0 ? 0 : d < R1 ? d : 0] : ld_row(c, d);
+#pragma unroll
+          for (int r = 0; r < R1; ++r)
+            if (d != r && d - r >= -H && d - r <= H)
+              acc[r] = star_term(acc[r], (R)a.a[1][d - r + HMAX], v, q[cu][r]);
+        }
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+          if (y0 + r >= n1) continue;
+          T v = acc[r];
+          if (epi) {
+            v = fmadd(scale((R)a.alpha, v), (R)a.beta, q[cu][r]);
+            if (ysrc) v = fmadd(v, (R)a.gamma, yv[r]);
+            if (vsrc) v = fmadd(v, vv[r], q[cu][r]);
+          }
+          st_cs(dst + po + r * n2, v);
         }
       }
-      __syncthreads();
-      if (j + D < j1) issue(j + D);
-      cp_async_commit();
     }
-    cp_async_wait<0>();
-    __syncthreads();
   }
 }
 
@@ -477,25 +365,13 @@ __global__ void jacobi_kernel(const BoxArgs args, const double* f_in, double* f_
 namespace gb {
 
 
-template <class C>
+template <typename T, int H>
 static int launch_star(const gb_operator* op, const void* in, void* out, int64_t nin,
                        const double* phase_cd, cudaStream_t stream, const Epilogue& ep, int nk) {
-  static int occ = -1;
-  static size_t smem_set = 0;
-  if (smem_set != C::SMEM) {
-    cudaFuncSetAttribute(star_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    smem_set = C::SMEM;
-  }
-  if (occ < 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, star_kernel<C>, C::NT, C::SMEM);
-    if (occ < 1) occ = 1;
-  }
   StarArgs a{};
   a.in = in; a.out = out; a.nbatch = nin;
   a.n0 = (int)op->n[0]; a.n1 = (int)op->n[1]; a.n2 = (int)op->n[2];
   a.pbc0 = op->pbc[0]; a.pbc1 = op->pbc[1]; a.pbc2 = op->pbc[2];
-  a.tiles1 = ceil_div(a.n1, C::T1);
-  a.tiles2 = ceil_div(a.n2, C::T2);
   a.c0 = op->center;
   a.c0diff = op->center;
   for (int c = 0; c < 3; ++c)
@@ -503,131 +379,37 @@ static int launch_star(const gb_operator* op, const void* in, void* out, int64_t
   memcpy(a.a, op->a, sizeof(a.a));
   a.alpha = ep.alpha; a.beta = ep.beta; a.gamma = ep.gamma; a.y = ep.y; a.vpot = ep.vpot;
   fill_phase_sets(a.phs, phase_cd, nk, nin);
-  const int64_t total = nin * (int64_t)a.tiles1 * a.tiles2 * a.n0;
-  int64_t blocks = (int64_t)sm_count() * occ;
-  // keep at least a few planes per CTA so the prologue (2H planes) stays small
-  blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, total / (4 * C::H + 4)));
-  star_kernel<C><<<(unsigned)blocks, C::NT, C::SMEM, stream>>>(a);
-  return check_launch("star_kernel");
-}
-
-// Small real grids (the coarsest multigrid level, 14^3 for a 56^3 grid):
-// the tiles of star_kernel would leave most threads idle and march a few
-// planes per CTA through its staging pipeline, so one thread per point reads
-// its 6H neighbours straight from global memory (the grid stays in L1/L2).
-// Same terms in the same order as star_kernel (axis 0, axis 2, axis 1, m
-// ascending; the FP32 difference form), so both give identical results.
-template <typename T, int H>
-__global__ void __launch_bounds__(256) star_direct_kernel(const StarArgs args) {
-  constexpr bool DIFF = sizeof(T) == 4;
-  const int n0 = args.n0, n1 = args.n1, n2 = args.n2;
-  const int64_t n12 = (int64_t)n1 * n2, n012 = n12 * n0;
-  const int64_t total = args.nbatch * n012;
-  const bool epi = args.alpha != 1.0 || args.beta != 0.0 || args.y != nullptr || args.vpot != nullptr;
-  const T* __restrict__ vpot = reinterpret_cast<const T*>(args.vpot);
-  const T c0 = DIFF ? (T)args.c0diff : (T)args.c0;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t band = e / n012;
-    const int64_t g = e - band * n012;
-    const int i0 = (int)(g / n12);
-    const int i1 = (int)((g - (int64_t)i0 * n12) / n2);
-    const int i2 = (int)(g - (int64_t)i0 * n12 - (int64_t)i1 * n2);
-    const T* __restrict__ src = reinterpret_cast<const T*>(args.in) + band * n012;
-    const T xc = src[g];
-    T x = scale(c0, xc);
-    // axis 0
-#pragma unroll
-    for (int m = 0; m <= 2 * H; ++m) {
-      if (m == H) continue;
-      int j = i0 + m - H;
-      T v = (T)0;
-      if (j >= 0 && j < n0) v = src[g + (int64_t)(m - H) * n12];
-      else if (args.pbc0) v = src[(int64_t)wrap_index(j, n0) * n12 + (g - (int64_t)i0 * n12)];
-      x = fmadd(x, (T)args.a[0][m - H + HMAX], DIFF ? v - xc : v);
+  // chunks of at most 24 planes (the 2H planes before each are read again,
+  // from L2), down to single planes while that gives more blocks than an SM
+  // holds several times over
+  a.tiles = ceil_div((int64_t)a.n1 * a.n2, 256);
+  const int64_t cols = nin * a.tiles;
+  a.chunks = (int)std::max<int64_t>(ceil_div(a.n0, 24),
+                                    std::min<int64_t>(a.n0, ceil_div((int64_t)sm_count() * 16, cols)));
+  const unsigned blocks = (unsigned)(cols * a.chunks);
+  const bool per = a.pbc0 || a.pbc1 || a.pbc2;
+  if constexpr (std::is_same<T, float>::value) {
+    if (symmetric_stencil<float>(op)) {
+      if (per) march_star_kernel<T, H, true, true><<<blocks, 256, 0, stream>>>(a);
+      else march_star_kernel<T, H, false, true><<<blocks, 256, 0, stream>>>(a);
+      return check_launch("march_star_kernel");
     }
-    // axis 2
-#pragma unroll
-    for (int m = 0; m <= 2 * H; ++m) {
-      if (m == H) continue;
-      int j = i2 + m - H;
-      T v = (T)0;
-      if (j >= 0 && j < n2) v = src[g + (m - H)];
-      else if (args.pbc2) v = src[g - i2 + wrap_index(j, n2)];
-      x = fmadd(x, (T)args.a[2][m - H + HMAX], DIFF ? v - xc : v);
-    }
-    // axis 1
-#pragma unroll
-    for (int m = 0; m <= 2 * H; ++m) {
-      if (m == H) continue;
-      int j = i1 + m - H;
-      T v = (T)0;
-      if (j >= 0 && j < n1) v = src[g + (int64_t)(m - H) * n2];
-      else if (args.pbc1) v = src[g + (int64_t)(wrap_index(j, n1) - i1) * n2];
-      x = fmadd(x, (T)args.a[1][m - H + HMAX], DIFF ? v - xc : v);
-    }
-    if (epi) {
-      T v = fmadd(scale((T)args.alpha, x), (T)args.beta, xc);
-      if (args.y) v = fmadd(v, (T)args.gamma, reinterpret_cast<const T*>(args.y)[e]);
-      if (vpot) v = fmadd(v, vpot[g], xc);
-      x = v;
-    }
-    reinterpret_cast<T*>(args.out)[e] = x;
   }
+  if (per) march_star_kernel<T, H, true, false><<<blocks, 256, 0, stream>>>(a);
+  else march_star_kernel<T, H, false, false><<<blocks, 256, 0, stream>>>(a);
+  return check_launch("march_star_kernel");
 }
-
-template <typename T, int H>
-static int launch_star_direct(const gb_operator* op, const void* in, void* out, int64_t nin,
-                              cudaStream_t stream, const Epilogue& ep) {
-  StarArgs a{};
-  a.in = in; a.out = out; a.nbatch = nin;
-  a.n0 = (int)op->n[0]; a.n1 = (int)op->n[1]; a.n2 = (int)op->n[2];
-  a.pbc0 = op->pbc[0]; a.pbc1 = op->pbc[1]; a.pbc2 = op->pbc[2];
-  a.c0 = op->center;
-  a.c0diff = op->center;
-  for (int c = 0; c < 3; ++c)
-    for (int m = 0; m < 2 * HMAX + 1; ++m) a.c0diff += op->a[c][m];
-  memcpy(a.a, op->a, sizeof(a.a));
-  a.alpha = ep.alpha; a.beta = ep.beta; a.gamma = ep.gamma; a.y = ep.y; a.vpot = ep.vpot;
-  const int64_t total = nin * op->n[0] * op->n[1] * op->n[2];
-  const int64_t blocks = std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 8);
-  star_direct_kernel<T, H><<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, stream>>>(a);
-  return check_launch("star_direct_kernel");
-}
-
-// Per-element-size tile shapes.  (R1 x R2) points per thread, (TY x TZ)
-// threads; R2 * sizeof(T) = 16 bytes so row windows are single LDS.128s and a
-// warp's 16 lanes along axis 2 read 256 contiguous bytes (no bank conflicts).
-template <typename T, int H>
-struct StarTile;
-template <int H> struct StarTile<float, H>   { using C = StarCfg<float, H, (H <= 3 ? 4 : 2), 4, 8, 8, 2>; };
-template <int H> struct StarTile<double, H>  { using C = StarCfg<double, H, (H <= 3 ? 4 : 2), 2, 8, 16, 2>; };
-template <int H> struct StarTile<float2, H>  { using C = StarCfg<float2, H, (H <= 3 ? 4 : 2), 2, 8, 16, 2>; };
-template <int H> struct StarTile<double2, H> { using C = StarCfg<double2, H, (H <= 3 ? 4 : 2), 1, 8, 16, 2>; };
 
 template <typename T>
 static int dispatch_star(const gb_operator* op, const void* in, void* out, int64_t nin,
                          const double* ph, cudaStream_t st, const Epilogue& ep, int nk) {
-  if constexpr (!Elem<T>::cplx) {
-    // tiles of star_kernel less than a quarter used: one thread per point
-    using C1 = typename StarTile<T, 1>::C;
-    const int64_t n1 = op->n[1], n2 = op->n[2];
-    const int64_t tiled = (int64_t)ceil_div((int)n1, C1::T1) * C1::T1 * ceil_div((int)n2, C1::T2) * C1::T2;
-    if (op->H <= 3 && 4 * n1 * n2 < tiled) {
-      switch (op->H) {
-        case 1: return launch_star_direct<T, 1>(op, in, out, nin, st, ep);
-        case 2: return launch_star_direct<T, 2>(op, in, out, nin, st, ep);
-        default: return launch_star_direct<T, 3>(op, in, out, nin, st, ep);
-      }
-    }
-  }
   switch (op->H) {
-    case 1: return launch_star<typename StarTile<T, 1>::C>(op, in, out, nin, ph, st, ep, nk);
-    case 2: return launch_star<typename StarTile<T, 2>::C>(op, in, out, nin, ph, st, ep, nk);
-    case 3: return launch_star<typename StarTile<T, 3>::C>(op, in, out, nin, ph, st, ep, nk);
-    case 4: return launch_star<typename StarTile<T, 4>::C>(op, in, out, nin, ph, st, ep, nk);
-    case 5:
-    case 6: return launch_star<typename StarTile<T, 6>::C>(op, in, out, nin, ph, st, ep, nk);
+    case 1: return launch_star<T, 1>(op, in, out, nin, ph, st, ep, nk);
+    case 2: return launch_star<T, 2>(op, in, out, nin, ph, st, ep, nk);
+    case 3: return launch_star<T, 3>(op, in, out, nin, ph, st, ep, nk);
+    case 4: return launch_star<T, 4>(op, in, out, nin, ph, st, ep, nk);
+    case 5: return launch_star<T, 5>(op, in, out, nin, ph, st, ep, nk);
+    case 6: return launch_star<T, 6>(op, in, out, nin, ph, st, ep, nk);
     default: return fail(GB_E_UNSUPPORTED, "star stencil radius > 6");
   }
 }
@@ -681,6 +463,8 @@ int op_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int 
     if (rc != 1) return rc;
     if (stencil_path() == 2)
       return fail(GB_E_UNSUPPORTED, std::string("TMA stencil path required but not applicable: ") + tma_reason());
+    const int rr = star_rows_apply(op, in, out, nin, dtype, ph, st, ep, nk);
+    if (rr != 1) return rr;
     switch (dtype) {
       case GB_DTYPE_F64: return dispatch_star<double>(op, in, out, nin, ph, st, ep, nk);
       case GB_DTYPE_F32: return dispatch_star<float>(op, in, out, nin, ph, st, ep, nk);

@@ -102,6 +102,9 @@ int tr_apply(const gb_transformer* t, const void* in, void* out, int64_t nin, in
 // TMA stencil path: returns 1 when the request is not eligible (caller falls back)
 int star_tma_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype,
                    const double* ph, cudaStream_t st, const Epilogue& ep, int nk = 1);
+// row kernel for the layouts the TMA path does not take; returns 1 likewise
+int star_rows_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype,
+                    const double* ph, cudaStream_t st, const Epilogue& ep, int nk = 1);
 void set_stencil_path(int mode);
 const char* tma_reason();
 int stencil_path();
