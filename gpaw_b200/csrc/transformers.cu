@@ -3,14 +3,15 @@
 //
 // The reference pads each band (c/bc.c), then runs three separable 1-D passes
 // with a transpose after each (restrict.c:136-155, interpolate.c:227-257),
-// i.e. four trips through memory per band.  Here one persistent kernel does
-// all three passes with one read of the input and one write of the output:
-// a CTA owns a 2-D tile of the (axis1, axis2) output plane and marches along
-// axis 0; each input plane (tile + halo, boundary conditions resolved while
-// staging through cp.async) is reduced along axis 2 then axis 1 in shared
-// memory, and the axis-0 pass runs on a per-thread register queue of the 2-D
-// results.  The pass order (axis 2, 1, 0) and the 0.5 factor per pass follow
-// the reference, so real FP64 results agree with it to rounding.
+// i.e. four trips through memory per band.  Here one kernel does all three
+// passes with one read of the input and one write of the output:
+//   k >= 4, and k = 2 on unusual grids: blocks of a few output planes, axis 0
+//     from global loads, axes 2 and 1 in shared memory
+//   k = 2: one thread per coarse column, in-plane values straight from
+//     global memory through L1, marching along axis 0
+//   k = 2, periodic real rows of whole 16-byte chunks: the same march over
+//     planes staged in shared memory
+// Real FP64 results agree with the reference to rounding.
 //
 // Index conventions (single domain, gpaw/transformers.py:31-47):
 //   restriction:   coarse local i  <-> fine local centre 2 i + off,
@@ -51,420 +52,415 @@ __device__ __forceinline__ int floor_div(int a, int b) {
   return (a >= 0) ? a / b : -((-a + b - 1) / b);
 }
 
-// Stage one input plane (rows [ry0, ry0+NR), cols [cx0, cx0+NC)) of `S` into
-// smem (row pitch PITCH), resolving zero / periodic boundaries.  cx0 must be a
-// multiple of VEC so 16-byte chunks line up.
-template <typename T, int NR, int NC, int PITCH, int NT>
-__device__ __forceinline__ void stage_plane(T* P, const T* S, int ry0, int cx0, int n1, int n2,
-                                            int pbc1, int pbc2, int tid) {
-  constexpr int VEC = 16 / sizeof(T);
-  constexpr int KC = NC / VEC;
-  static_assert(NC % VEC == 0, "");
-  for (int e = tid; e < NR * KC; e += NT) {
-    const int r = e / KC, k = e % KC;
-    T* sd = P + r * PITCH + k * VEC;
-    int y = ry0 + r;
-    if (y < 0 || y >= n1) {
-      if (!pbc1) {
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) sd[v] = zero<T>();
-        continue;
-      }
-      y = tr_mod(y, n1);
-    }
-    const T* row = S + (int64_t)y * n2;
-    const int zs = cx0 + k * VEC;
-    if (zs >= 0 && zs + VEC <= n2 && ((reinterpret_cast<uintptr_t>(row + zs) & 15) == 0)) {
-      cp_async16(sd, row + zs);
-    } else {
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) {
-        int z = zs + v;
-        if (z < 0 || z >= n2) {
-          if (!pbc2) { sd[v] = zero<T>(); continue; }
-          z = tr_mod(z, n2);
-        }
-        cp_async_elem(sd + v, row + z);
-      }
-    }
-  }
-}
-
-// multiply wrapped cells of a staged plane by the Bloch phase
-template <typename T, int NR, int NC, int PITCH, int NT>
-__device__ __forceinline__ void phase_fixup(T* P, int ry0, int cx0, int n1, int n2,
-                                            const TrArgs& a, const double (&PH)[3][2][2], int tid) {
-  for (int e = tid; e < NR * NC; e += NT) {
-    const int r = e / NC, c = e % NC;
-    const int y = ry0 + r, z = cx0 + c;
-    double pr = 1.0, pi = 0.0;
-    bool w = false;
-    if (a.pbc[1] && (y < 0 || y >= n1)) { const int s = y < 0; pr = PH[1][s][0]; pi = PH[1][s][1]; w = true; }
-    if (a.pbc[2] && (z < 0 || z >= n2)) {
-      const int s = z < 0;
-      const double qr = PH[2][s][0], qi = PH[2][s][1];
-      const double tr = pr * qr - pi * qi, ti = pr * qi + pi * qr;
-      pr = tr; pi = ti; w = true;
-    }
-    if (w) P[r * PITCH + c] = phase_mul(P[r * PITCH + c], pr, pi);
-  }
-}
-
-// ---------------------------------------------------------------- restriction
-template <typename T_, int K_, int CY_, int CZ_, int D_>
-struct RCfg {
+// ---------------------------------------------------------------- any k
+// Restriction with k taps per axis, any geometry, boundary and element type.
+// A CTA owns T1 x T2 points of IB coarse planes.  The axis-0 pass runs first,
+// on values read straight from global memory (2 IB + k - 1 independent,
+// coalesced loads per fine column, all boundary rules resolved there); the
+// axis-2 and axis-1 passes follow in shared memory.  Nothing marches, so one
+// small grid (the density's 112^3 -> 56^3) already fills the GPU: it is
+// bound by L2 reads, (2 IB + k - 1) / 2 IB times the halo factor of the tile.
+template <typename T_, int K_, int IB_, int T1_, int T2_>
+struct RXCfg {
   using T = T_;
-  static constexpr int K = K_, CY = CY_, CZ = CZ_, D = D_;
-  static constexpr int NT = CY * CZ;
-  static constexpr int VEC = 16 / (int)sizeof(T);
-  static constexpr int FR = 2 * CY + 2 * K - 3;
-  static constexpr int FC = 2 * CZ + 2 * K - 3;
-  static constexpr int FCW = ((FC + VEC - 1 + VEC - 1) / VEC) * VEC;   // room for the alignment shift
-  static constexpr int PITCH = FCW;
-  static constexpr int PLANE = FR * PITCH;
-  static constexpr int NS = D + 1;
-  static constexpr int TB = FR * CZ;                                  // pass-A buffer
-  static constexpr size_t SMEM = ((size_t)NS * PLANE + TB) * sizeof(T);
-  static constexpr int NQ = 2 * K - 1;
+  static constexpr int K = K_, IB = IB_, T1 = T1_, T2 = T2_, NT = 256;
+  static constexpr int FR = 2 * T1 + 2 * K - 3, FC = 2 * T2 + 2 * K - 3;
+  static constexpr size_t SMEM = (size_t)IB * FR * (FC + T2) * sizeof(T);
 };
 
+// index i of an axis of n points: the wrapped index (periodic), or -1
+__device__ __forceinline__ int tr_index(int i, int n, int pbc, int& side) {
+  side = i < 0 ? 1 : i >= n ? 0 : -1;
+  if (side < 0) return i;
+  return pbc ? tr_mod(i, n) : -1;
+}
+
 template <class C>
-__global__ void __launch_bounds__(C::NT) restrict_kernel(const TrArgs a) {
+__global__ void __launch_bounds__(C::NT) restrict_x_kernel(const __grid_constant__ TrArgs a) {
   using T = typename C::T;
   using R = typename Elem<T>::R;
-  constexpr int K = C::K, CY = C::CY, CZ = C::CZ, D = C::D, NT = C::NT, VEC = C::VEC;
-  constexpr int FR = C::FR, PITCH = C::PITCH, PLANE = C::PLANE, NS = C::NS, NQ = C::NQ;
+  constexpr int K = C::K, IB = C::IB, T1 = C::T1, T2 = C::T2, FR = C::FR, FC = C::FC, KH = K / 2;
+  constexpr int NO = IB + K - 1;                       // odd-offset planes
   constexpr bool CPLX = Elem<T>::cplx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);
-  T* tbuf = ring + NS * PLANE;
-
-  const int tid = threadIdx.x, ty = tid / CZ, tz = tid % CZ;
+  T* X = reinterpret_cast<T*>(smem_raw);               // [IB][FR][FC]
+  T* Z = X + IB * FR * FC;                             // [IB][FR][T2]
   const int nf0 = a.ni[0], nf1 = a.ni[1], nf2 = a.ni[2];
   const int nc0 = a.no[0], nc1 = a.no[1], nc2 = a.no[2];
   const int64_t nf12 = (int64_t)nf1 * nf2, nc12 = (int64_t)nc1 * nc2;
-  const int64_t ntiles = (int64_t)a.tiles1 * a.tiles2;
-  const int64_t total = a.nbatch * ntiles * nc0;
-  int64_t s = total * blockIdx.x / gridDim.x;
-  const int64_t s_end = total * (blockIdx.x + 1) / gridDim.x;
-  R w[K / 2];
-#pragma unroll
-  for (int m = 0; m < K / 2; ++m) w[m] = (R)a.w[m];
-  const R half = (R)0.5, alpha = (R)a.alpha;
-
-  while (s < s_end) {
-    const int64_t col = s / nc0;
-    const int Is = (int)(s % nc0);
-    const int Ie = (int)((s_end - s) < (int64_t)(nc0 - Is) ? Is + (s_end - s) : nc0);
-    s += Ie - Is;
-    const int64_t band = col / ntiles;
-    const int t = (int)(col % ntiles);
-    const int Y0 = (t / a.tiles2) * CY, Z0 = (t % a.tiles2) * CZ;
-    const T* src = reinterpret_cast<const T*>(a.in) + band * nf12 * nf0;
-    T* dst = reinterpret_cast<T*>(a.out) + band * nc12 * nc0;
-    const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
-    const int ry0 = 2 * Y0 + a.off[1] - (K - 1);
-    const int s0 = 2 * Z0 + a.off[2] - (K - 1);
-    const int cx0 = floor_div(s0, VEC) * VEC;
-    const int sh = s0 - cx0;
-    const bool edge = ry0 < 0 || ry0 + FR > nf1 || cx0 < 0 || cx0 + PITCH > nf2;
-    const int j0 = 2 * Is + a.off[0] - (K - 1);
-    const int j1 = 2 * (Ie - 1) + a.off[0] + K;   // exclusive
-
-    auto src_plane = [&](int j, double& pr, double& pi) -> int {
-      pr = 1.0; pi = 0.0;
-      if (j >= 0 && j < nf0) return j;
-      if (!a.pbc[0]) return -1;
-      const int sd = j < 0;
-      pr = PH[0][sd][0]; pi = PH[0][sd][1];
-      return tr_mod(j, nf0);
-    };
-    auto issue = [&](int j) {
-      double pr, pi;
-      const int sp = src_plane(j, pr, pi);
-      if (sp < 0) return;
-      stage_plane<T, FR, PITCH, PITCH, NT>(ring + ((j - j0) % NS) * PLANE, src + (int64_t)sp * nf12,
-                                           ry0, cx0, nf1, nf2, a.pbc[1], a.pbc[2], tid);
-    };
-
-    T q[NQ];
-#pragma unroll
-    for (int m = 0; m < NQ; ++m) q[m] = zero<T>();
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (j0 + d < j1) issue(j0 + d);
-      cp_async_commit();
-    }
-    for (int j = j0; j < j1; ++j) {
-      cp_async_wait<D - 1>();
-      __syncthreads();
-      double pr, pi;
-      const int sp = src_plane(j, pr, pi);
-      T* P = ring + ((j - j0) % NS) * PLANE;
-      T u = zero<T>();
-      if (sp >= 0) {
-        if (CPLX && a.phs.any && edge) {
-          phase_fixup<T, FR, PITCH, PITCH, NT>(P, ry0, cx0, nf1, nf2, a, PH, tid);
-          __syncthreads();
-        }
-        if constexpr (K == 2) {
-          // k = 2: the 3 x 3 in-plane stencil straight from the staged plane
-          // (the same operations, in the same order, as the two separable
-          // passes below; no intermediate buffer, no barrier)
-          const T* f = P + (2 * ty + 1) * PITCH + sh + 2 * tz + 1;
-          T g[3];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const T* fr = f + (d - 1) * PITCH;
-            g[d] = scale(half, fmadd(fr[0], w[0], add(fr[1], fr[-1])));
-          }
-          u = scale(half, fmadd(g[1], w[0], add(g[2], g[0])));
-          if (CPLX) u = phase_mul(u, pr, pi);
-        } else {
-          // pass A: along axis 2 for every staged row
-          for (int e = tid; e < FR * CZ; e += NT) {
-            const int r = e / CZ, jz = e % CZ;
-            const T* f = P + r * PITCH + sh + 2 * jz + (K - 1);
-            T x = f[0];
-#pragma unroll
-            for (int m = 0; m < K / 2; ++m) x = fmadd(x, w[m], add(f[2 * m + 1], f[-(2 * m + 1)]));
-            tbuf[r * CZ + jz] = scale(half, x);
-          }
-          __syncthreads();
-          // pass B: along axis 1 for the own coarse point
-          const T* tcol = tbuf + (2 * ty + (K - 1)) * CZ + tz;
-          T x = tcol[0];
-#pragma unroll
-          for (int m = 0; m < K / 2; ++m)
-            x = fmadd(x, w[m], add(tcol[(2 * m + 1) * CZ], tcol[-(2 * m + 1) * CZ]));
-          u = scale(half, x);
-          if (CPLX) u = phase_mul(u, pr, pi);
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < NQ - 1; ++m) q[m] = q[m + 1];
-      q[NQ - 1] = u;
-      // axis 0: coarse plane whose last fine contribution just arrived
-      const int tI = j - a.off[0] - (K - 1);
-      if (tI >= 2 * Is && (tI & 1) == 0) {
-        const int I = tI >> 1;
-        T x = q[K - 1];
-#pragma unroll
-        for (int m = 0; m < K / 2; ++m) x = fmadd(x, w[m], add(q[K - 1 + 2 * m + 1], q[K - 1 - (2 * m + 1)]));
-        x = scale(half, x);
-        const int yi = Y0 + ty, zi = Z0 + tz;
-        if (yi < nc1 && zi < nc2) dst[(int64_t)I * nc12 + (int64_t)yi * nc2 + zi] = scale(alpha, x);
-      }
-      // the separable passes reuse tbuf next step; the k = 2 path needs no
-      // barrier here: the slot refilled below was last read in step j - 1,
-      // which every thread finished before the barrier at the top of step j
-      if constexpr (K != 2) __syncthreads();
-      if (j + D < j1) issue(j + D);
-      cp_async_commit();
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------- interpolation
-template <typename T_, int K_, int FY_, int FZ_, int RY_, int RZ_, int D_>
-struct ICfg {
-  using T = T_;
-  static constexpr int K = K_, FY = FY_, FZ = FZ_, RY = RY_, RZ = RZ_, D = D_;
-  static constexpr int TY = FY / RY, TZ = FZ / RZ, NT = TY * TZ;
-  static constexpr int VEC = 16 / (int)sizeof(T);
-  static constexpr int CR = FY / 2 + K + 1;                     // coarse rows staged
-  static constexpr int CC = FZ / 2 + K + 1;                     // coarse cols needed
-  static constexpr int PITCH = ((CC + VEC - 1 + VEC - 1) / VEC) * VEC;
-  static constexpr int PLANE = CR * PITCH;
-  static constexpr int NS = D + 1;
-  static constexpr int TB = CR * FZ;
-  static constexpr size_t SMEM = ((size_t)NS * PLANE + TB) * sizeof(T);
-};
-
-template <class C>
-__global__ void __launch_bounds__(C::NT) interpolate_kernel(const TrArgs a) {
-  using T = typename C::T;
-  using R = typename Elem<T>::R;
-  constexpr int K = C::K, FY = C::FY, FZ = C::FZ, RY = C::RY, RZ = C::RZ, D = C::D;
-  constexpr int TZ = C::TZ, NT = C::NT, VEC = C::VEC, CR = C::CR, PITCH = C::PITCH;
-  constexpr int PLANE = C::PLANE, NS = C::NS, KH = K / 2;
-  constexpr bool CPLX = Elem<T>::cplx;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);
-  T* tbuf = ring + NS * PLANE;
-
-  const int tid = threadIdx.x, ty = tid / TZ, tz = tid % TZ;
-  const int nc0 = a.ni[0], nc1 = a.ni[1], nc2 = a.ni[2];
-  const int nf0 = a.no[0], nf1 = a.no[1], nf2 = a.no[2];
-  const int64_t nc12 = (int64_t)nc1 * nc2, nf12 = (int64_t)nf1 * nf2;
-  const int64_t ntiles = (int64_t)a.tiles1 * a.tiles2;
-  // output pairs along axis 0: global coarse C from cmin to cmin + nsteps
-  const int cmin = floor_div(a.skip0[0], 2);
-  const int64_t total = a.nbatch * ntiles * a.nsteps;
-  int64_t s = total * blockIdx.x / gridDim.x;
-  const int64_t s_end = total * (blockIdx.x + 1) / gridDim.x;
+  unsigned t = blockIdx.x;
+  const int K0 = (int)(t % a.tiles2) * T2;
+  t /= a.tiles2;
+  const int J0 = (int)(t % a.tiles1) * T1;
+  t /= a.tiles1;
+  const int I0 = (int)(t % a.nsteps) * IB;
+  const int64_t band = t / a.nsteps;
+  const T* __restrict__ src = reinterpret_cast<const T*>(a.in) + band * nf12 * nf0;
+  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + band * nc12 * nc0;
+  const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
+  const bool phased = CPLX && a.phs.any;
   R w[KH];
 #pragma unroll
   for (int m = 0; m < KH; ++m) w[m] = (R)a.w[m];
-  const R alpha = (R)a.alpha, gamma = (R)a.gamma;
+  const R half = (R)0.5;
+  const int j0 = 2 * I0 + a.off[0];                    // centre plane of coarse plane I0
+  const int r0 = 2 * J0 + a.off[1] - (K - 1), c0 = 2 * K0 + a.off[2] - (K - 1);
 
-  while (s < s_end) {
-    const int64_t col = s / a.nsteps;
-    const int Ps = (int)(s % a.nsteps);
-    const int Pe = (int)((s_end - s) < (int64_t)(a.nsteps - Ps) ? Ps + (s_end - s) : a.nsteps);
-    s += Pe - Ps;
-    const int64_t band = col / ntiles;
-    const int t = (int)(col % ntiles);
-    const int Y0 = (t / a.tiles2) * FY, Z0 = (t % a.tiles2) * FZ;
-    const T* src = reinterpret_cast<const T*>(a.in) + band * nc12 * nc0;
-    T* dst = reinterpret_cast<T*>(a.out) + band * nf12 * nf0;
-    const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
-    const T* ysrc = a.y ? reinterpret_cast<const T*>(a.y) + band * nf12 * nf0 : nullptr;
-    // coarse rows / cols staged: global coarse index base, local = global - cbeg
-    const int crow0 = floor_div(Y0 + a.skip0[1], 2) - (KH - 1);          // global coarse row of staged row 0
-    const int ry0 = crow0 - a.cbeg[1];                                    // local
-    const int ccol0 = floor_div(Z0 + a.skip0[2], 2) - (KH - 1);
-    const int cl = ccol0 - a.cbeg[2];
-    const int cx0 = floor_div(cl, VEC) * VEC;
-    const int sh = cl - cx0;
-    const bool edge = ry0 < 0 || ry0 + CR > nc1 || cx0 < 0 || cx0 + PITCH > nc2;
-    // coarse planes (global) needed for output pairs [cmin+Ps, cmin+Pe)
-    const int g0 = cmin + Ps - (KH - 1), g1 = cmin + Pe + KH;   // [g0, g1)
-
-    auto src_plane = [&](int g, double& pr, double& pi) -> int {
-      pr = 1.0; pi = 0.0;
-      const int l = g - a.cbeg[0];
-      if (l >= 0 && l < nc0) return l;
-      if (!a.pbc[0]) return -1;
-      const int sd = l < 0;
-      pr = PH[0][sd][0]; pi = PH[0][sd][1];
-      return tr_mod(l, nc0);
-    };
-    auto issue = [&](int g) {
-      double pr, pi;
-      const int sp = src_plane(g, pr, pi);
-      if (sp < 0) return;
-      stage_plane<T, CR, PITCH, PITCH, NT>(ring + ((g - g0) % NS) * PLANE, src + (int64_t)sp * nc12,
-                                           ry0, cx0, nc1, nc2, a.pbc[1], a.pbc[2], tid);
-    };
-
-    T q[K][RY][RZ];
+  // fine plane j0 + d at an in-plane offset
+  auto plane = [&](int d, int64_t off) -> T {
+    int side;
+    const int j = tr_index(j0 + d, nf0, a.pbc[0], side);
+    T v = zero<T>();
+    if (j >= 0) v = __ldg(src + j * nf12 + off);
+    if (phased && side >= 0) v = phase_mul(v, PH[0][side][0], PH[0][side][1]);
+    return v;
+  };
+  for (int e = threadIdx.x; e < FR * FC; e += C::NT) {
+    const int r = e / FC, c = e - r * FC;
+    int sy, sz;
+    const int y = tr_index(r0 + r, nf1, a.pbc[1], sy), z = tr_index(c0 + c, nf2, a.pbc[2], sz);
+    T x[IB];
 #pragma unroll
-    for (int m = 0; m < K; ++m)
+    for (int i = 0; i < IB; ++i) x[i] = zero<T>();
+    if (y >= 0 && z >= 0) {
+      const int64_t off = (int64_t)y * nf2 + z;
+      T ev[IB], od[NO];
 #pragma unroll
-      for (int r = 0; r < RY; ++r)
+      for (int i = 0; i < IB; ++i) ev[i] = plane(2 * i, off);
 #pragma unroll
-        for (int c = 0; c < RZ; ++c) q[m][r][c] = zero<T>();
+      for (int i = 0; i < NO; ++i) od[i] = plane(2 * i - (K - 1), off);
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (g0 + d < g1) issue(g0 + d);
-      cp_async_commit();
+      for (int i = 0; i < IB; ++i) {
+        T v = ev[i];
+        // offsets +-(2m + 1) of plane 2i are odd planes i + KH + m and i + KH - 1 - m
+#pragma unroll
+        for (int m = 0; m < KH; ++m) v = fmadd(v, w[m], add(od[i + KH + m], od[i + KH - 1 - m]));
+        x[i] = scale(half, v);
+      }
+      if (phased) {
+        if (sy >= 0)
+#pragma unroll
+          for (int i = 0; i < IB; ++i) x[i] = phase_mul(x[i], PH[1][sy][0], PH[1][sy][1]);
+        if (sz >= 0)
+#pragma unroll
+          for (int i = 0; i < IB; ++i) x[i] = phase_mul(x[i], PH[2][sz][0], PH[2][sz][1]);
+      }
     }
-    for (int g = g0; g < g1; ++g) {
-      cp_async_wait<D - 1>();
-      __syncthreads();
-      double pr, pi;
-      const int sp = src_plane(g, pr, pi);
-      T* P = ring + ((g - g0) % NS) * PLANE;
-      T u[RY][RZ];
-      if (sp >= 0) {
-        if (CPLX && a.phs.any && edge) {
-          phase_fixup<T, CR, PITCH, PITCH, NT>(P, ry0, cx0, nc1, nc2, a, PH, tid);
-          __syncthreads();
-        }
-        // pass A: along axis 2, every staged coarse row -> FZ fine columns
-        for (int e = tid; e < CR * FZ; e += NT) {
-          const int r = e / FZ, fc = e % FZ;
-          const int F = Z0 + fc + a.skip0[2];
-          const T* row = P + r * PITCH + sh;
-          T x;
-          if ((F & 1) == 0) {
-            x = row[(F >> 1) - ccol0];
-          } else {
-            const int cc = ((F - 1) >> 1) - ccol0;
-            x = scale(w[0], add(row[cc], row[cc + 1]));
 #pragma unroll
-            for (int m = 1; m < KH; ++m) x = fmadd(x, w[m], add(row[cc - m], row[cc + 1 + m]));
-          }
-          tbuf[r * FZ + fc] = x;
-        }
-        __syncthreads();
-        // pass B: along axis 1 for the own fine points
+    for (int i = 0; i < IB; ++i) X[i * FR * FC + e] = x[i];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < IB * FR * T2; e += C::NT) {
+    const int r = e / T2, k = e - r * T2;              // r counts the rows of all IB planes
+    const T* f = X + r * FC + 2 * k + (K - 1);
+    T v = f[0];
 #pragma unroll
-        for (int r = 0; r < RY; ++r) {
-          const int F = Y0 + ty * RY + r + a.skip0[1];
+    for (int m = 0; m < KH; ++m) v = fmadd(v, w[m], add(f[2 * m + 1], f[-(2 * m + 1)]));
+    Z[e] = scale(half, v);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < IB * T1 * T2; e += C::NT) {
+    const int k = e % T2, r = (e / T2) % T1, i = e / (T1 * T2);
+    const int I = I0 + i, J = J0 + r, kk = K0 + k;
+    if (I >= nc0 || J >= nc1 || kk >= nc2) continue;
+    const T* f = Z + (i * FR + 2 * r + (K - 1)) * T2 + k;
+    T v = f[0];
 #pragma unroll
-          for (int c = 0; c < RZ; ++c) {
-            const T* tc = tbuf + tz * RZ + c;
-            T x;
-            if ((F & 1) == 0) {
-              x = tc[((F >> 1) - crow0) * FZ];
-            } else {
-              const int cr = ((F - 1) >> 1) - crow0;
-              x = scale(w[0], add(tc[cr * FZ], tc[(cr + 1) * FZ]));
+    for (int m = 0; m < KH; ++m) v = fmadd(v, w[m], add(f[(2 * m + 1) * T2], f[-(2 * m + 1) * T2]));
+    dst[I * nc12 + (int64_t)J * nc2 + kk] = scale((R)a.alpha, scale(half, v));
+  }
+}
+
+// Interpolation, likewise: a CTA owns T1 x T2 fine points of the 2 IB fine
+// planes of IB coarse planes; axis 0 from global loads, axes 2 and 1 in
+// shared memory.
+template <typename T_, int K_, int IB_, int T1_, int T2_>
+struct IXCfg {
+  using T = T_;
+  static constexpr int K = K_, IB = IB_, T1 = T1_, T2 = T2_, NT = 256;
+  static constexpr int CR = T1 / 2 + K, CC = T2 / 2 + K;
+  static constexpr size_t SMEM = (size_t)2 * IB * CR * (CC + T2) * sizeof(T);
+};
+
+template <class C>
+__global__ void __launch_bounds__(C::NT) interpolate_x_kernel(const __grid_constant__ TrArgs a) {
+  using T = typename C::T;
+  using R = typename Elem<T>::R;
+  constexpr int K = C::K, IB = C::IB, T1 = C::T1, T2 = C::T2, CR = C::CR, CC = C::CC, KH = K / 2;
+  constexpr int NP = IB + K - 1;                       // coarse planes read
+  constexpr bool CPLX = Elem<T>::cplx;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* X = reinterpret_cast<T*>(smem_raw);               // [2 IB][CR][CC]
+  T* Z = X + 2 * IB * CR * CC;                         // [2 IB][CR][T2]
+  const int nc0 = a.ni[0], nc1 = a.ni[1], nc2 = a.ni[2];
+  const int nf0 = a.no[0], nf1 = a.no[1], nf2 = a.no[2];
+  const int64_t nc12 = (int64_t)nc1 * nc2, nf12 = (int64_t)nf1 * nf2;
+  unsigned t = blockIdx.x;
+  const int Z0 = (int)(t % a.tiles2) * T2;
+  t /= a.tiles2;
+  const int Y0 = (int)(t % a.tiles1) * T1;
+  t /= a.tiles1;
+  const int cells = (a.nsteps + IB - 1) / IB;
+  const int C0 = floor_div(a.skip0[0], 2) + (int)(t % cells) * IB;   // first global coarse plane
+  const int64_t band = t / cells;
+  const T* __restrict__ src = reinterpret_cast<const T*>(a.in) + band * nc12 * nc0;
+  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + band * nf12 * nf0;
+  const T* __restrict__ ysrc = a.y ? reinterpret_cast<const T*>(a.y) + band * nf12 * nf0 : nullptr;
+  const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
+  const bool phased = CPLX && a.phs.any;
+  R w[KH];
 #pragma unroll
-              for (int m = 1; m < KH; ++m) x = fmadd(x, w[m], add(tc[(cr - m) * FZ], tc[(cr + 1 + m) * FZ]));
-            }
-            u[r][c] = CPLX ? phase_mul(x, pr, pi) : x;
-          }
-        }
-      } else {
+  for (int m = 0; m < KH; ++m) w[m] = (R)a.w[m];
+  // global coarse row / column of staged row / column 0
+  const int crow0 = floor_div(Y0 + a.skip0[1], 2) - (KH - 1);
+  const int ccol0 = floor_div(Z0 + a.skip0[2], 2) - (KH - 1);
+
+  for (int e = threadIdx.x; e < CR * CC; e += C::NT) {
+    const int r = e / CC, c = e - r * CC;
+    int sy, sz;
+    const int y = tr_index(crow0 + r - a.cbeg[1], nc1, a.pbc[1], sy);
+    const int z = tr_index(ccol0 + c - a.cbeg[2], nc2, a.pbc[2], sz);
+    T x[2 * IB];
 #pragma unroll
-        for (int r = 0; r < RY; ++r)
+    for (int i = 0; i < 2 * IB; ++i) x[i] = zero<T>();
+    if (y >= 0 && z >= 0) {
+      const int64_t off = (int64_t)y * nc2 + z;
+      T p[NP];
 #pragma unroll
-          for (int c = 0; c < RZ; ++c) u[r][c] = zero<T>();
+      for (int i = 0; i < NP; ++i) {
+        int side;
+        const int g = tr_index(C0 - (KH - 1) + i - a.cbeg[0], nc0, a.pbc[0], side);
+        p[i] = zero<T>();
+        if (g >= 0) p[i] = __ldg(src + g * nc12 + off);
+        if (phased && side >= 0) p[i] = phase_mul(p[i], PH[0][side][0], PH[0][side][1]);
       }
 #pragma unroll
-      for (int m = 0; m < K - 1; ++m)
+      for (int i = 0; i < IB; ++i) {
+        x[2 * i] = p[KH - 1 + i];
+        T v = scale(w[0], add(p[KH - 1 + i], p[KH + i]));
 #pragma unroll
-        for (int r = 0; r < RY; ++r)
+        for (int m = 1; m < KH; ++m) v = fmadd(v, w[m], add(p[KH - 1 + i - m], p[KH + i + m]));
+        x[2 * i + 1] = v;
+      }
+      if (phased) {
+        if (sy >= 0)
 #pragma unroll
-          for (int c = 0; c < RZ; ++c) q[m][r][c] = q[m + 1][r][c];
+          for (int i = 0; i < 2 * IB; ++i) x[i] = phase_mul(x[i], PH[1][sy][0], PH[1][sy][1]);
+        if (sz >= 0)
 #pragma unroll
-      for (int r = 0; r < RY; ++r)
+          for (int i = 0; i < 2 * IB; ++i) x[i] = phase_mul(x[i], PH[2][sz][0], PH[2][sz][1]);
+      }
+    }
 #pragma unroll
-        for (int c = 0; c < RZ; ++c) q[K - 1][r][c] = u[r][c];
-      // output fine planes 2C and 2C+1 for C = g - KH once coarse C+KH is in
-      const int Cg = g - KH;
-      if (Cg >= cmin + Ps) {
+    for (int i = 0; i < 2 * IB; ++i) X[i * CR * CC + e] = x[i];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 2 * IB * CR * T2; e += C::NT) {
+    const int r = e / T2, fc = e - r * T2;
+    const int F = Z0 + fc + a.skip0[2];
+    const T* f = X + r * CC + (floor_div(F, 2) - ccol0);
+    T v = f[0];
+    if (F & 1) {
+      v = scale(w[0], add(f[0], f[1]));
 #pragma unroll
-        for (int par = 0; par < 2; ++par) {
-          const int f = 2 * Cg + par - a.skip0[0];
-          if (f < 0 || f >= nf0) continue;
-          T* op = dst + (int64_t)f * nf12;
-          const T* yp = ysrc ? ysrc + (int64_t)f * nf12 : nullptr;
+      for (int m = 1; m < KH; ++m) v = fmadd(v, w[m], add(f[-m], f[1 + m]));
+    }
+    Z[e] = v;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 2 * IB * T1 * T2; e += C::NT) {
+    const int c = e % T2, r = (e / T2) % T1, i = e / (T1 * T2);
+    const int f0 = 2 * C0 + i - a.skip0[0], y = Y0 + r, z = Z0 + c;
+    if (f0 < 0 || f0 >= nf0 || y >= nf1 || z >= nf2) continue;
+    const int F = y + a.skip0[1];
+    const T* f = Z + (i * CR + floor_div(F, 2) - crow0) * T2 + c;
+    T v = f[0];
+    if (F & 1) {
+      v = scale(w[0], add(f[0], f[T2]));
 #pragma unroll
-          for (int r = 0; r < RY; ++r) {
-            const int yi = Y0 + ty * RY + r;
-            if (yi >= nf1) continue;
+      for (int m = 1; m < KH; ++m) v = fmadd(v, w[m], add(f[-m * T2], f[(1 + m) * T2]));
+    }
+    const int64_t o = f0 * nf12 + (int64_t)y * nf2 + z;
+    v = scale((R)a.alpha, v);
+    if (ysrc) v = fmadd(v, (R)a.gamma, __ldcs(ysrc + o));
+    dst[o] = v;
+  }
+}
+
+// ---------------------------------------------------------------- k = 2
+// The preconditioner's transfers on grids whose axes each have the usual
+// geometry (periodic: 2 n fine for n coarse points; zero boundary: 2 n + 1),
+// whatever the row length, boundary mix, element type and phases.  One thread
+// per coarse (axis 1, axis 2) column marches over a few coarse planes; its
+// 3 x 3 (restriction) or 2 x 2 (interpolation) in-plane values come straight
+// from global memory through L1, so there is no staging and no barrier.
+// phase of a cell wrapped over two axes
+__device__ __forceinline__ double2 corner_phase(const double (&p)[2], const double (&q)[2]) {
+  return make_double2(__fma_rn(p[0], q[0], -__dmul_rn(p[1], q[1])), __fma_rn(p[0], q[1], __dmul_rn(p[1], q[0])));
+}
+
+template <typename T, bool PER>
+__global__ void __launch_bounds__(256) restrict2_direct_kernel(const __grid_constant__ TrArgs a) {
+  using R = typename Elem<T>::R;
+  constexpr bool CPLX = Elem<T>::cplx;
+  const int nf0 = a.ni[0], nf1 = a.ni[1], nf2 = a.ni[2];
+  const int nc0 = a.no[0], nc1 = a.no[1], nc2 = a.no[2];
+  const int64_t nf12 = (int64_t)nf1 * nf2, nc12 = (int64_t)nc1 * nc2;
+  unsigned t = blockIdx.x;
+  const int64_t f = (int64_t)(t % a.tiles1) * 256 + threadIdx.x;
+  t /= a.tiles1;
+  const int chunk = (int)(t % a.nsteps);
+  const int64_t band = t / a.nsteps;
+  int K;
+  const int J = (int)div_mod(f, nc2, K);
+  if (J >= nc1) return;
+  const int I_beg = (int)((int64_t)nc0 * chunk / a.nsteps), I_end = (int)((int64_t)nc0 * (chunk + 1) / a.nsteps);
+  const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
+  const bool phased = CPLX && PER && a.phs.any;
+  const R w0 = (R)a.w[0], half = (R)0.5;
+  // fine neighbours of the centre (2J + off, 2K + off): only index -1 of a
+  // periodic axis is outside the grid
+  const bool wy = PER && a.pbc[1] && J == 0, wz = PER && a.pbc[2] && K == 0;
+  const int oz = wz ? nf2 - 1 : -1;
+  const int64_t oy = wy ? (int64_t)(nf1 - 1) * nf2 : -nf2;
+  const T* __restrict__ p = reinterpret_cast<const T*>(a.in) + band * nf12 * nf0 +
+                            (int64_t)(2 * J + a.off[1]) * nf2 + 2 * K + a.off[2];
+  auto plane = [&](int j) -> T {
+    const bool wx = PER && j < 0;
+    const T* c = p + (int64_t)(wx ? j + nf0 : j) * nf12;
+    T v[3][3];
 #pragma unroll
-            for (int c = 0; c < RZ; ++c) {
-              const int zi = Z0 + tz * RZ + c;
-              if (zi >= nf2) continue;
-              T x;
-              if (par == 0) {
-                x = q[KH - 1][r][c];
-              } else {
-                x = scale(w[0], add(q[KH - 1][r][c], q[KH][r][c]));
+    for (int d = 0; d < 3; ++d) {
+      const T* row = c + (d == 0 ? oy : d == 1 ? 0 : (int64_t)nf2);
+      v[d][0] = __ldg(row + oz);
+      v[d][1] = __ldg(row);
+      v[d][2] = __ldg(row + 1);
+    }
+    if (phased) {
+      // each wrapped cell by its own phase, the corner by the product
+      if (wz) {
+        v[1][0] = phase_mul(v[1][0], PH[2][1][0], PH[2][1][1]);
+        v[2][0] = phase_mul(v[2][0], PH[2][1][0], PH[2][1][1]);
+        if (!wy) v[0][0] = phase_mul(v[0][0], PH[2][1][0], PH[2][1][1]);
+      }
+      if (wy) {
+        const double2 c = wz ? corner_phase(PH[1][1], PH[2][1]) : make_double2(PH[1][1][0], PH[1][1][1]);
+        v[0][0] = phase_mul(v[0][0], c.x, c.y);
+        v[0][1] = phase_mul(v[0][1], PH[1][1][0], PH[1][1][1]);
+        v[0][2] = phase_mul(v[0][2], PH[1][1][0], PH[1][1][1]);
+      }
+    }
+    T g[3];
 #pragma unroll
-                for (int m = 1; m < KH; ++m) x = fmadd(x, w[m], add(q[KH - 1 - m][r][c], q[KH + m][r][c]));
-              }
-              x = scale(alpha, x);
-              const int64_t o = (int64_t)yi * nf2 + zi;
-              if (yp) x = fmadd(x, gamma, yp[o]);
-              op[o] = x;
-            }
-          }
+    for (int d = 0; d < 3; ++d) g[d] = scale(half, fmadd(v[d][1], w0, add(v[d][2], v[d][0])));
+    T u = scale(half, fmadd(g[1], w0, add(g[2], g[0])));
+    if (phased && wx) u = phase_mul(u, PH[0][1][0], PH[0][1][1]);
+    return u;
+  };
+  T* __restrict__ o = reinterpret_cast<T*>(a.out) + band * nc12 * nc0 + I_beg * nc12 + (int64_t)J * nc2 + K;
+  int j = 2 * I_beg + a.off[0];
+  T um = plane(j - 1);
+  for (int I = I_beg; I < I_end; ++I, j += 2, o += nc12) {
+    const T uc = plane(j), up = plane(j + 1);
+    *o = scale((R)a.alpha, scale(half, fmadd(uc, w0, add(up, um))));
+    um = up;
+  }
+}
+
+// One thread per (coarse row cell, fine column): its lanes write consecutive
+// fine points (a thread per coarse cell wrote every other one, and took 1.4
+// times as long on partial sectors).
+template <typename T, bool PER>
+__global__ void __launch_bounds__(256) interp2_direct_kernel(const __grid_constant__ TrArgs a) {
+  using R = typename Elem<T>::R;
+  constexpr bool CPLX = Elem<T>::cplx;
+  const int nc0 = a.ni[0], nc1 = a.ni[1], nc2 = a.ni[2];
+  const int nf0 = a.no[0], nf1 = a.no[1], nf2 = a.no[2];
+  const int64_t nc12 = (int64_t)nc1 * nc2, nf12 = (int64_t)nf1 * nf2;
+  // cells C (between coarse points C and C + 1, global numbering): one per
+  // coarse point of a periodic axis, one more on a zero-boundary one
+  const int m0 = nc0 + a.cbeg[0], m1 = nc1 + a.cbeg[1];
+  unsigned t = blockIdx.x;
+  const int64_t f = (int64_t)(t % a.tiles1) * 256 + threadIdx.x;
+  t /= a.tiles1;
+  const int chunk = (int)(t % a.nsteps);
+  const int64_t band = t / a.nsteps;
+  int zf;
+  const int Cy = (int)div_mod(f, nf2, zf);
+  if (Cy >= m1) return;
+  const int C_beg = (int)((int64_t)m0 * chunk / a.nsteps), C_end = (int)((int64_t)m0 * (chunk + 1) / a.nsteps);
+  const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
+  const bool phased = CPLX && PER && a.phs.any;
+  const R w0 = (R)a.w[0], alpha = (R)a.alpha, gamma = (R)a.gamma;
+  // local coarse row and column of the cell's lower points; an even fine
+  // column takes the lower column alone
+  const int Fz = zf + a.skip0[2];
+  const bool odd = Fz & 1;
+  const int y0 = Cy - a.cbeg[1], z0 = (Fz >> 1) - a.cbeg[2];
+  const bool wy = PER && a.pbc[1] && y0 + 1 == nc1, wz = PER && a.pbc[2] && z0 + 1 == nc2;
+  const bool by0 = y0 >= 0, bz0 = z0 >= 0, by1 = y0 + 1 < nc1 || wy, bz1 = odd && (z0 + 1 < nc2 || wz);
+  const int64_t oy = wy ? -(int64_t)(nc1 - 1) * nc2 : nc2;
+  const int oz = wz ? -(nc2 - 1) : 1;
+  const T* __restrict__ p = reinterpret_cast<const T*>(a.in) + band * nc12 * nc0 + (int64_t)y0 * nc2 + z0;
+  // the two fine rows of coarse plane C at this column
+  auto plane = [&](int C, T (&u)[2]) {
+    int l = C - a.cbeg[0];
+    const bool wx = PER && a.pbc[0] && l == nc0;
+    if (wx) l = 0;
+    const bool in = l >= 0 && l < nc0;
+    const T* c = p + (int64_t)l * nc12;
+    T A[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool row = in && (h ? by1 : by0);
+      T v0 = zero<T>(), v1 = zero<T>();
+      if (row && bz0) v0 = __ldg(c + (h ? oy : 0));
+      if (row && bz1) v1 = __ldg(c + (h ? oy : 0) + oz);
+      if (phased) {
+        const bool y = wy && h == 1;
+        if (y) v0 = phase_mul(v0, PH[1][0][0], PH[1][0][1]);
+        if (y || wz) {
+          const double2 c = y && wz ? corner_phase(PH[1][0], PH[2][0])
+                                    : y ? make_double2(PH[1][0][0], PH[1][0][1])
+                                        : make_double2(PH[2][0][0], PH[2][0][1]);
+          v1 = phase_mul(v1, c.x, c.y);
         }
       }
-      __syncthreads();
-      if (g + D < g1) issue(g + D);
-      cp_async_commit();
+      A[h] = odd ? scale(w0, add(v0, v1)) : v0;
     }
-    cp_async_wait<0>();
-    __syncthreads();
+    u[0] = A[0];
+    u[1] = scale(w0, add(A[0], A[1]));
+    if (phased && wx) {
+      u[0] = phase_mul(u[0], PH[0][0][0], PH[0][0][1]);
+      u[1] = phase_mul(u[1], PH[0][0][0], PH[0][0][1]);
+    }
+  };
+  // fine local rows and planes are 2 C + parity - skip
+  const int fy = 2 * Cy - a.skip0[1];
+  const bool sy[2] = {fy >= 0, fy + 1 < nf1};
+  const int64_t base = band * nf12 * nf0 + (int64_t)fy * nf2 + zf;
+  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + base;
+  const T* __restrict__ ysrc = a.y ? reinterpret_cast<const T*>(a.y) + base : nullptr;
+  T q[2];
+  plane(C_beg, q);
+  for (int C = C_beg; C < C_end; ++C) {
+    T u[2];
+    plane(C + 1, u);
+#pragma unroll
+    for (int par = 0; par < 2; ++par) {
+      const int fp = 2 * C + par - a.skip0[0];
+      if (fp < 0 || fp >= nf0) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (!sy[h]) continue;
+        const int64_t o = fp * nf12 + h * (int64_t)nf2;
+        T v = scale(alpha, par ? scale(w0, add(q[h], u[h])) : q[h]);
+        if (ysrc) v = fmadd(v, gamma, __ldcs(ysrc + o));
+        dst[o] = v;
+      }
+    }
+    q[0] = u[0];
+    q[1] = u[1];
   }
 }
 
@@ -500,35 +496,53 @@ static void fill_common(const gb_transformer* t, TrArgs& a, const double* ph, in
   fill_phase_sets(a.phs, ph, nk, nbatch);
 }
 
-template <class C, typename KernelT>
-static int launch_persistent(KernelT kernel, const TrArgs& a, int64_t total, cudaStream_t st, int min_steps) {
-  static int occ = -1;
-  if (occ < 0) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, C::NT, C::SMEM);
-    if (occ < 1) occ = 1;
+// every axis periodic with 2 n fine points, or zero-boundary with 2 n + 1
+static bool usual_geometry(const gb_transformer* t) {
+  for (int c = 0; c < 3; ++c) {
+    const int64_t nf = t->interpolate ? t->nout_c[c] : t->nin_c[c], nc = t->interpolate ? t->nin_c[c] : t->nout_c[c];
+    const int z = t->pbc[c] ? 0 : 1;
+    if (nf != 2 * nc + z) return false;
+    if (t->interpolate ? (t->skip0[c] != z || t->cbeg[c] != z) : t->off[c] != z) return false;
   }
-  int64_t blocks = (int64_t)sm_count() * occ;
-  // at least min_steps planes per CTA amortise its (2K-1)-plane prologue --
-  // unless that would leave SMs idle (one small grid, e.g. the density's
-  // 112^3 -> 56^3): then the prologue's L2 re-reads cost less than idle SMs
-  const int64_t by_steps = total / min_steps;
-  blocks = std::min<int64_t>(blocks, by_steps >= sm_count() ? by_steps : std::max<int64_t>(1, total));
+  return true;
+}
+
+template <class C, typename KernelT>
+static int launch_x(KernelT kernel, const TrArgs& a, int64_t blocks, cudaStream_t st) {
+  static bool set = false;
+  if (!set && C::SMEM > 48 * 1024) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    set = true;
+  }
   kernel<<<(unsigned)blocks, C::NT, C::SMEM, st>>>(a);
   return check_launch("transformer kernel");
 }
 
-template <typename T, int K, int CY, int CZ>
-static int restrict_cfg(const gb_transformer* t, const void* in, void* out, int64_t nin,
-                        const double* ph, cudaStream_t st, double alpha, int nk) {
-  using C = RCfg<T, K, CY, CZ, 2>;
+// planes per thread of the k = 2 kernels: chunks of at most 12, more of them
+// while the grid would not fill the GPU
+static int direct_chunks(int64_t cols, int n0) {
+  return (int)std::max<int64_t>(ceil_div(n0, 12), std::min<int64_t>(n0, ceil_div((int64_t)sm_count() * 8, cols)));
+}
+
+template <typename T, int K>
+static int restrict_x(const gb_transformer* t, const void* in, void* out, int64_t nin, const double* ph,
+                      cudaStream_t st, double alpha, int nk) {
   TrArgs a;
   fill_common(t, a, ph, nk, nin);
   a.in = in; a.out = out; a.nbatch = nin; a.alpha = alpha;
-  a.tiles1 = ceil_div(a.no[1], C::CY);
-  a.tiles2 = ceil_div(a.no[2], C::CZ);
-  const int64_t total = nin * (int64_t)a.tiles1 * a.tiles2 * a.no[0];
-  return launch_persistent<C>(restrict_kernel<C>, a, total, st, 4 + K);
+  if (K == 2 && usual_geometry(t)) {
+    a.tiles1 = ceil_div((int64_t)a.no[1] * a.no[2], 256);
+    a.nsteps = direct_chunks(nin * a.tiles1, a.no[0]);
+    const unsigned blocks = (unsigned)(nin * a.tiles1 * a.nsteps);
+    if (a.pbc[0] || a.pbc[1] || a.pbc[2]) restrict2_direct_kernel<T, true><<<blocks, 256, 0, st>>>(a);
+    else restrict2_direct_kernel<T, false><<<blocks, 256, 0, st>>>(a);
+    return check_launch("restrict2_direct_kernel");
+  }
+  using C = RXCfg<T, K, 2, 8, sizeof(T) == 16 ? 16 : 32>;
+  a.tiles1 = ceil_div(a.no[1], C::T1);
+  a.tiles2 = ceil_div(a.no[2], C::T2);
+  a.nsteps = ceil_div(a.no[0], C::IB);
+  return launch_x<C>(restrict_x_kernel<C>, a, nin * (int64_t)a.tiles1 * a.tiles2 * a.nsteps, st);
 }
 
 // k = 2 restriction of real data on a grid periodic on every axis (the
@@ -840,200 +854,13 @@ static int interp2_march_launch(const gb_transformer* t, const void* in, void* o
   return check_launch("interp2_march_kernel");
 }
 
-// coarse rows of at most 16 points (the coarse levels of small grids) use a
-// 16 x 16 tile, wider ones 8 x 32: no more than half a warp idles on a row
-// k = 6 restriction of real data on a grid periodic on every axis (the
-// density / potential transfers between the coarse and the fine grid),
-// marching along axis 0 like restrict2_march_kernel: a CTA owns TYC coarse
-// rows of one band over a chunk of coarse planes and stages every fine
-// plane it needs once (rows 2 J0 + off - 5 .. 2 (J0 + TYC - 1) + off + 5,
-// five wrap-around columns on each side) with cp.async into a two-slot
-// ring.  A thread restricts the plane in-plane for two neighbouring coarse
-// points -- axis 2 on each of its seven fine rows, then axis 1 -- and the
-// axis-0 step takes the last eleven fine planes from a register queue; the
-// arithmetic of the general kernel (x = f0, x += w_m (f_{2m+1} + f_{-2m-1}),
-// m = 0, 1, 2, then x / 2, axis by axis), in its order.  Rows must be
-// 16-byte aligned.
-template <typename T, int TYC>
-__global__ void __launch_bounds__(256) restrict6_march_kernel(const TrArgs a, int nch) {
-  extern __shared__ __align__(16) unsigned char r6m_smem[];
-  T* slot = reinterpret_cast<T*>(r6m_smem);
-  constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int CO = ((5 + VEC - 1) / VEC) * VEC;        // fine column c at CO + c
-  const int nf0 = a.ni[0], nf1 = a.ni[1], nf2 = a.ni[2];
-  const int nc0 = a.no[0], nc1 = a.no[1], nc2 = a.no[2];
-  const int FR = 2 * TYC + 9, FP = nf2 + 2 * CO + 2 * VEC;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int ngx = (nc2 + 1) >> 1;
-  const int gx = tid % ngx, ty = tid / ngx;
-  const int J0 = blockIdx.y * TYC, J = J0 + ty, K0 = 2 * gx;
-  const int64_t b = blockIdx.z;
-  const int I_beg = (int)((int64_t)blockIdx.x * nc0 / nch), I_end = (int)((int64_t)(blockIdx.x + 1) * nc0 / nch);
-  const T* src = reinterpret_cast<const T*>(a.in) + b * (int64_t)nf0 * nf1 * nf2;
-  T* dst = reinterpret_cast<T*>(a.out) + b * (int64_t)nc0 * nc1 * nc2;
-  const T w0 = (T)a.w[0], w1 = (T)a.w[1], w2 = (T)a.w[2], half = (T)0.5, alpha = (T)a.alpha;
-  const int r0 = 2 * J0 + a.off[1] - 5;                 // first staged fine row
-  auto wrap = [](int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); };
-  // element e = (row r, piece c): 16-byte chunks c < chunks, then the five
-  // columns -5 .. -1 and the five columns nf2 .. nf2 + 4
-  const int chunks = nf2 / VEC, per = chunks + 10, ne = FR * per;
-  constexpr int MAXU = 8;
-  int s_off[MAXU], d_off[MAXU];
-  unsigned wide = 0u;
-#pragma unroll
-  for (int u = 0; u < MAXU; ++u) {
-    const int e = tid + u * nt;
-    s_off[u] = 0;
-    d_off[u] = -1;
-    if (e < ne) {
-      const int r = e / per, c = e % per;
-      const int row = wrap(r0 + r, nf1) * nf2;
-      if (c < chunks) {
-        s_off[u] = row + c * VEC;
-        d_off[u] = r * FP + CO + c * VEC;
-        wide |= 1u << u;
-      } else if (c < chunks + 5) {
-        const int h = c - chunks;                   // column h - 5
-        s_off[u] = row + nf2 - 5 + h;
-        d_off[u] = r * FP + CO - 5 + h;
-      } else {
-        const int h = c - chunks - 5;               // column nf2 + h
-        s_off[u] = row + h;
-        d_off[u] = r * FP + CO + nf2 + h;
-      }
-    }
-  }
-  auto stage = [&](int p, T* d) {
-    const T* pl = src + (int64_t)wrap(p, nf0) * nf1 * nf2;
-#pragma unroll
-    for (int u = 0; u < MAXU; ++u) {
-      if (d_off[u] < 0) continue;
-      if (wide & (1u << u)) cp_async16(d + d_off[u], pl + s_off[u]);
-      else cp_async_elem(d + d_off[u], pl + s_off[u]);
-    }
-    for (int e = tid + MAXU * nt; e < ne; e += nt) {
-      const int r = e / per, c = e % per;
-      const T* row = pl + (int64_t)wrap(r0 + r, nf1) * nf2;
-      T* dr = d + r * FP + CO;
-      if (c < chunks) cp_async16(dr + c * VEC, row + c * VEC);
-      else if (c < chunks + 5) cp_async_elem(dr - 5 + (c - chunks), row + nf2 - 5 + (c - chunks));
-      else cp_async_elem(dr + nf2 + (c - chunks - 5), row + (c - chunks - 5));
-    }
-  };
-  // one axis: x = f0; x += w_m (f_{2m+1} + f_{-(2m+1)}); x / 2
-  auto axis = [&](T c0, T p1, T m1, T p3, T m3, T p5, T m5) {
-    T x = c0;
-    x = fmadd(x, w0, add(p1, m1));
-    x = fmadd(x, w1, add(p3, m3));
-    x = fmadd(x, w2, add(p5, m5));
-    return half * x;
-  };
-  const int p_beg = 2 * I_beg + a.off[0] - 5, p_end = 2 * (I_end - 1) + a.off[0] + 5;
-  stage(p_beg, slot);
-  cp_async_commit();
-  T q[2][11];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int m = 0; m < 11; ++m) q[h][m] = (T)0;
-  const bool act = ty < TYC && J < nc1;
-  for (int p = p_beg; p <= p_end; ++p) {
-    const int s = (p - p_beg) & 1;
-    if (p + 1 <= p_end) stage(p + 1, slot + (s ^ 1) * FR * FP);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    if (act) {
-      // centre fine row 2J + off of this thread: staged row 2 ty + 5
-      const T* P = slot + s * FR * FP + (2 * ty + 5) * FP + CO + 2 * K0 + a.off[2];
-      T g[2][11];                                      // [h][fine row offset + 5]
-#pragma unroll
-      for (int dy = -5; dy <= 5; ++dy) {
-        if (dy != 0 && (dy & 1) == 0) continue;        // even offsets carry no weight
-        const T* f = P + dy * FP;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const T* c = f + 2 * h;
-          g[h][dy + 5] = axis(c[0], c[1], c[-1], c[3], c[-3], c[5], c[-5]);
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int m = 0; m < 10; ++m) q[h][m] = q[h][m + 1];
-        q[h][10] = axis(g[h][5], g[h][6], g[h][4], g[h][8], g[h][2], g[h][10], g[h][0]);
-      }
-      const int tI = p - a.off[0] - 5;                  // fine plane 2I + off + 5 just arrived
-      if (tI >= 2 * I_beg && (tI & 1) == 0) {
-        const int I = tI >> 1;
-        T* o = dst + ((int64_t)I * nc1 + J) * nc2 + K0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (K0 + h < nc2) o[h] = alpha * axis(q[h][5], q[h][6], q[h][4], q[h][8], q[h][2], q[h][10], q[h][0]);
-      }
-    }
-    __syncthreads();
-  }
-  cp_async_wait<0>();
-}
-
-template <typename T>
-static bool restrict6_march_ok(const gb_transformer* t, int64_t nin, const double* ph) {
-  if (!t->pbc[0] || !t->pbc[1] || !t->pbc[2] || nin > 65535 || nin < 1) return false;
-  if (ph)
-    for (int i = 0; i < 12; ++i)
-      if (ph[i] != ((i % 2) ? 0.0 : 1.0)) return false;
-  const int64_t nf2 = t->nin_c[2];
-  const int64_t ngx = (t->nout_c[2] + 1) / 2;
-  const int64_t tyc = ngx * 8 <= 256 ? 8 : (ngx * 4 <= 256 ? 4 : 2);
-  // single-wrap periodic indices: at least 6 fine planes and columns, and
-  // rows enough that the last tile's staged rows (up to nf1 + 2 TYC + 2)
-  // stay below 2 nf1
-  return (nf2 * (int64_t)sizeof(T)) % 16 == 0 && ngx * 2 <= 256 && t->nin_c[0] >= 6 &&
-         t->nin_c[1] >= 2 * tyc + 3 && nf2 >= 6 && t->nout_c[1] >= 1 && t->nout_c[0] >= 1;
-}
-
-template <typename T>
-static int restrict6_march_launch(const gb_transformer* t, const void* in, void* out, int64_t nin,
-                                  cudaStream_t st, double alpha) {
-  constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int CO = ((5 + VEC - 1) / VEC) * VEC;
-  TrArgs a;
-  fill_common(t, a, nullptr, 1, nin);
-  a.in = in; a.out = out; a.nbatch = nin; a.alpha = alpha;
-  const int ngx = (a.no[2] + 1) / 2;
-  const int TYC = ngx * 8 <= 256 ? 8 : (ngx * 4 <= 256 ? 4 : 2);
-  // plane chunks: enough CTAs for every SM (a single grid is cut into
-  // short chunks, each re-staging its ten halo planes from L2)
-  const int64_t tiles = (int64_t)((a.no[1] + TYC - 1) / TYC) * nin;
-  const int nch = (int)std::max<int64_t>(1, std::min<int64_t>(a.no[0], (sm_count() + tiles - 1) / tiles));
-  const size_t smem = (size_t)2 * (2 * TYC + 9) * (a.ni[2] + 2 * CO + 2 * VEC) * sizeof(T);
-  static size_t attr = 0;
-  if (smem > 48 * 1024 && smem > attr) {
-    cudaFuncSetAttribute(restrict6_march_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(restrict6_march_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(restrict6_march_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = smem;
-  }
-  const dim3 grid((unsigned)nch, (unsigned)((a.no[1] + TYC - 1) / TYC), (unsigned)nin);
-  const unsigned threads = (unsigned)(ngx * TYC);
-  if (TYC == 8) restrict6_march_kernel<T, 8><<<grid, threads, smem, st>>>(a, nch);
-  else if (TYC == 4) restrict6_march_kernel<T, 4><<<grid, threads, smem, st>>>(a, nch);
-  else restrict6_march_kernel<T, 2><<<grid, threads, smem, st>>>(a, nch);
-  return check_launch("restrict6_march_kernel");
-}
-
 template <typename T, int K>
 static int restrict_k(const gb_transformer* t, const void* in, void* out, int64_t nin,
                       const double* ph, cudaStream_t st, double alpha, int nk) {
   if constexpr (K == 2 && !Elem<T>::cplx) {
     if (restrict2_march_ok<T>(t, nin, ph)) return restrict2_march_launch<T>(t, in, out, nin, st, alpha);
   }
-  if constexpr (K == 6 && !Elem<T>::cplx) {
-    if (restrict6_march_ok<T>(t, nin, ph)) return restrict6_march_launch<T>(t, in, out, nin, st, alpha);
-  }
-  if (t->nout_c[2] <= 16) return restrict_cfg<T, K, 16, 16>(t, in, out, nin, ph, st, alpha, nk);
-  return restrict_cfg<T, K, 8, 32>(t, in, out, nin, ph, st, alpha, nk);
+  return restrict_x<T, K>(t, in, out, nin, ph, st, alpha, nk);
 }
 
 template <typename T, int K>
@@ -1043,19 +870,26 @@ static int interpolate_k(const gb_transformer* t, const void* in, void* out, int
   if constexpr (K == 2 && !Elem<T>::cplx) {
     if (interp2_march_ok<T>(t, nin, ph, y)) return interp2_march_launch<T>(t, in, out, nin, st, alpha, y, gamma);
   }
-  constexpr int RZ = sizeof(T) == 4 ? 4 : (sizeof(T) == 8 ? 2 : 1);
-  using C = ICfg<T, K, 16, 32, 2, RZ, 2>;
   TrArgs a;
   fill_common(t, a, ph, nk, nin);
   a.in = in; a.out = out; a.nbatch = nin; a.alpha = alpha; a.y = y; a.gamma = gamma;
-  a.tiles1 = ceil_div(a.no[1], C::FY);
-  a.tiles2 = ceil_div(a.no[2], C::FZ);
-  // output pairs C with 2C - skip0 or 2C + 1 - skip0 in [0, nf0)
+  if (K == 2 && usual_geometry(t)) {
+    a.tiles1 = ceil_div((int64_t)(a.ni[1] + a.cbeg[1]) * a.no[2], 256);
+    a.nsteps = direct_chunks(nin * a.tiles1, a.ni[0] + a.cbeg[0]);
+    const unsigned blocks = (unsigned)(nin * a.tiles1 * a.nsteps);
+    if (a.pbc[0] || a.pbc[1] || a.pbc[2]) interp2_direct_kernel<T, true><<<blocks, 256, 0, st>>>(a);
+    else interp2_direct_kernel<T, false><<<blocks, 256, 0, st>>>(a);
+    return check_launch("interp2_direct_kernel");
+  }
+  using C = IXCfg<T, K, 1, 16, sizeof(T) == 16 ? 16 : 32>;
+  a.tiles1 = ceil_div(a.no[1], C::T1);
+  a.tiles2 = ceil_div(a.no[2], C::T2);
+  // coarse planes C with 2C - skip0 or 2C + 1 - skip0 in [0, nf0)
   const int cmin = a.skip0[0] >= 0 ? a.skip0[0] / 2 : -((-a.skip0[0] + 1) / 2);
   const int cmax = (a.no[0] - 1 + a.skip0[0]) / 2;
   a.nsteps = cmax - cmin + 1;
-  const int64_t total = nin * (int64_t)a.tiles1 * a.tiles2 * a.nsteps;
-  return launch_persistent<C>(interpolate_kernel<C>, a, total, st, 4 + K);
+  return launch_x<C>(interpolate_x_kernel<C>, a,
+                     nin * (int64_t)a.tiles1 * a.tiles2 * ceil_div(a.nsteps, C::IB), st);
 }
 
 template <typename T>
