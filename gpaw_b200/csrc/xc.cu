@@ -153,21 +153,61 @@ __device__ __forceinline__ double correlation(const Par& p, double n, double rs,
   return e;
 }
 
+// One point, spin-paired: e, the increment of v, and dedsigma (GGA).
+__device__ __forceinline__ void point_unpolarized(const Par& p, double n, double a2, double& e, double& dv,
+                                                  double& ds) {
+  if (n < NMIN) n = NMIN;
+  const double rs = cbrt(p.C0I / n);
+  double dexdrs, dexda2 = 0.0, decdrs, decda2 = 0.0, dz;
+  const double ex = exchange(p, n, rs, a2, &dexdrs, &dexda2);
+  const double ec = correlation(p, n, rs, 0.0, a2, false, &decdrs, &dz, &decda2);
+  ds = n * (dexda2 + decda2);
+  e = n * (ex + ec);
+  dv = ex + ec - rs * (dexdrs + decdrs) / 3.0;
+}
+
+// One point, spin-polarised: sigma and dedsigma are (up up, up down, down down).
+__device__ __forceinline__ void point_polarized(const Par& p, double nu, double nd, const double (&sg)[3], double& e,
+                                                double (&dv)[2], double (&ds)[3]) {
+  double na = 2.0 * nu;
+  if (na < NMIN) na = NMIN;
+  const double rsa = cbrt(p.C0I / na);
+  double nb = 2.0 * nd;
+  if (nb < NMIN) nb = NMIN;
+  const double rsb = cbrt(p.C0I / nb);
+  const double n = 0.5 * (na + nb);
+  const double rs = cbrt(p.C0I / n);
+  const double zeta = 0.5 * (na - nb) / n;
+  double dexadrs, dexada2 = 0.0, dexbdrs, dexbda2 = 0.0, decdrs, decdzeta, decda2 = 0.0;
+  double exa, exb, ec;
+  if (p.gga) {
+    exa = exchange(p, na, rsa, 4.0 * sg[0], &dexadrs, &dexada2);
+    exb = exchange(p, nb, rsb, 4.0 * sg[2], &dexbdrs, &dexbda2);
+    const double a2 = sg[0] + 2.0 * sg[1] + sg[2];
+    ec = correlation(p, n, rs, zeta, a2, true, &decdrs, &decdzeta, &decda2);
+    ds[0] = 2.0 * na * dexada2 + n * decda2;
+    ds[1] = 2.0 * n * decda2;
+    ds[2] = 2.0 * nb * dexbda2 + n * decda2;
+  } else {
+    exa = exchange(p, na, rsa, 0.0, &dexadrs, &dexada2);
+    exb = exchange(p, nb, rsb, 0.0, &dexbdrs, &dexbda2);
+    ec = correlation(p, n, rs, zeta, 0.0, true, &decdrs, &decdzeta, &decda2);
+  }
+  e = 0.5 * (na * exa + nb * exb) + n * ec;
+  dv[0] = exa + ec - (rsa * dexadrs + rs * decdrs) / 3.0 - (zeta - 1.0) * decdzeta;
+  dv[1] = exb + ec - (rsb * dexbdrs + rs * decdrs) / 3.0 - (zeta + 1.0) * decdzeta;
+}
+
 __global__ void xc_unpolarized(const Par p, int64_t ng, double* __restrict__ e_g,
                                const double* __restrict__ n_g, double* __restrict__ v_g,
                                const double* __restrict__ sigma_g, double* __restrict__ dedsigma_g) {
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng;
        g += (int64_t)gridDim.x * blockDim.x) {
-    double n = n_g[g];
-    if (n < NMIN) n = NMIN;
-    const double rs = cbrt(p.C0I / n);
-    double dexdrs, dexda2 = 0.0, decdrs, decda2 = 0.0, dz;
-    const double a2 = p.gga ? sigma_g[g] : 0.0;
-    const double ex = exchange(p, n, rs, a2, &dexdrs, &dexda2);
-    const double ec = correlation(p, n, rs, 0.0, a2, false, &decdrs, &dz, &decda2);
-    if (p.gga) dedsigma_g[g] = n * (dexda2 + decda2);
-    e_g[g] = n * (ex + ec);
-    v_g[g] += ex + ec - rs * (dexdrs + decdrs) / 3.0;
+    double e, dv, ds;
+    point_unpolarized(p, n_g[g], p.gga ? sigma_g[g] : 0.0, e, dv, ds);
+    if (p.gga) dedsigma_g[g] = ds;
+    e_g[g] = e;
+    v_g[g] += dv;
   }
 }
 
@@ -176,35 +216,111 @@ __global__ void xc_polarized(const Par p, int64_t ng, double* __restrict__ e_g,
                              const double* __restrict__ sigma_xg, double* __restrict__ dedsigma_xg) {
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng;
        g += (int64_t)gridDim.x * blockDim.x) {
-    double na = 2.0 * n_sg[g];
-    if (na < NMIN) na = NMIN;
-    const double rsa = cbrt(p.C0I / na);
-    double nb = 2.0 * n_sg[ng + g];
-    if (nb < NMIN) nb = NMIN;
-    const double rsb = cbrt(p.C0I / nb);
-    const double n = 0.5 * (na + nb);
-    const double rs = cbrt(p.C0I / n);
-    const double zeta = 0.5 * (na - nb) / n;
-    double dexadrs, dexada2 = 0.0, dexbdrs, dexbda2 = 0.0, decdrs, decdzeta, decda2 = 0.0;
-    double exa, exb, ec;
-    if (p.gga) {
-      const double s0 = sigma_xg[g], s1 = sigma_xg[ng + g], s2 = sigma_xg[2 * ng + g];
-      exa = exchange(p, na, rsa, 4.0 * s0, &dexadrs, &dexada2);
-      exb = exchange(p, nb, rsb, 4.0 * s2, &dexbdrs, &dexbda2);
-      const double a2 = s0 + 2.0 * s1 + s2;
-      ec = correlation(p, n, rs, zeta, a2, true, &decdrs, &decdzeta, &decda2);
-      dedsigma_xg[g] = 2.0 * na * dexada2 + n * decda2;
-      dedsigma_xg[ng + g] = 2.0 * n * decda2;
-      dedsigma_xg[2 * ng + g] = 2.0 * nb * dexbda2 + n * decda2;
-    } else {
-      exa = exchange(p, na, rsa, 0.0, &dexadrs, &dexada2);
-      exb = exchange(p, nb, rsb, 0.0, &dexbdrs, &dexbda2);
-      ec = correlation(p, n, rs, zeta, 0.0, true, &decdrs, &decdzeta, &decda2);
-    }
-    e_g[g] = 0.5 * (na * exa + nb * exb) + n * ec;
-    v_sg[g] += exa + ec - (rsa * dexadrs + rs * decdrs) / 3.0 - (zeta - 1.0) * decdzeta;
-    v_sg[ng + g] += exb + ec - (rsb * dexbdrs + rs * decdrs) / 3.0 - (zeta + 1.0) * decdzeta;
+    double e, dv[2], ds[3], sg[3] = {0.0, 0.0, 0.0};
+    if (p.gga)
+#pragma unroll
+      for (int x = 0; x < 3; ++x) sg[x] = sigma_xg[x * ng + g];
+    point_polarized(p, n_sg[g], n_sg[ng + g], sg, e, dv, ds);
+    if (p.gga)
+#pragma unroll
+      for (int x = 0; x < 3; ++x) dedsigma_xg[x * ng + g] = ds[x];
+    e_g[g] = e;
+    v_sg[g] += dv[0];
+    v_sg[ng + g] += dv[1];
   }
+}
+
+// GGA on the grid in two launches.  The first evaluates, per point, grad n
+// (central differences along the axes, neighbours through L1), sigma, the
+// functional, and stores the flux 2 (de/dsigma_ss) grad n_s + (de/dsigma_ud)
+// grad n_s'; the second subtracts its divergence from v.  Separate gradients,
+// sums, products and divergences took 27 launches, each through memory: 594
+// us for PBE on 151^3 points against 201 us for the two.  The first (146 us)
+// is bound by the functional's FP64 arithmetic, the second (54 us) by the
+// flux, whose three arrays no longer fit L2 beside the others at that size
+// (marching along axis 0 to read one of them once measured the same).
+constexpr int GH = 4;                      // largest stencil radius
+struct GradArgs {
+  int n[3], pbc[3], H;
+  double c0[3], a[3][2 * GH + 1];          // centre and offset coefficients of d/dx_v along axis v
+};
+
+// sum_m a_v[m] f[. + m along axis v] (f: this point; i: its index on the axis);
+// the loads are issued together
+template <int H>
+__device__ __forceinline__ double axis_derivative(const GradArgs& ga, const double* __restrict__ f, int v, int i,
+                                                  int64_t stride) {
+  double w[2 * H + 1];
+#pragma unroll
+  for (int m = -H; m <= H; ++m) {
+    int j = i + m;
+    bool ok = true;
+    if (j < 0 || j >= ga.n[v]) {
+      ok = ga.pbc[v];
+      j += j < 0 ? ga.n[v] : -ga.n[v];
+    }
+    w[m + H] = ok ? __ldg(f + (j - i) * stride) : 0.0;
+  }
+  double x = ga.c0[v] * w[H];
+#pragma unroll
+  for (int m = -H; m <= H; ++m)
+    if (m) x = fma(ga.a[v][m + GH], w[m + H], x);
+  return x;
+}
+
+template <int NS, int H>
+__global__ void __launch_bounds__(256) gga_flux_kernel(const Par p, const __grid_constant__ GradArgs ga, int64_t ng,
+                                                       double* __restrict__ e_g, const double* __restrict__ n_sg,
+                                                       double* __restrict__ v_sg, double* __restrict__ flux) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (g >= ng) return;
+  const int64_t st[3] = {(int64_t)ga.n[1] * ga.n[2], ga.n[2], 1};
+  int i[3];
+  i[0] = (int)div_mod(div_mod(g, ga.n[2], i[2]), ga.n[1], i[1]);
+  double d[3][NS];
+#pragma unroll
+  for (int v = 0; v < 3; ++v)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) d[v][s] = axis_derivative<H>(ga, n_sg + s * ng + g, v, i[v], st[v]);
+  double e;
+  if constexpr (NS == 1) {
+    const double sg = d[0][0] * d[0][0] + d[1][0] * d[1][0] + d[2][0] * d[2][0];
+    double dv, ds;
+    point_unpolarized(p, n_sg[g], sg, e, dv, ds);
+    v_sg[g] += dv;
+#pragma unroll
+    for (int v = 0; v < 3; ++v) flux[v * ng + g] = 2.0 * ds * d[v][0];
+  } else {
+    double dv[2], ds[3];
+    const double sg[3] = {d[0][0] * d[0][0] + d[1][0] * d[1][0] + d[2][0] * d[2][0],
+                          d[0][0] * d[0][1] + d[1][0] * d[1][1] + d[2][0] * d[2][1],
+                          d[0][1] * d[0][1] + d[1][1] * d[1][1] + d[2][1] * d[2][1]};
+    point_polarized(p, n_sg[g], n_sg[ng + g], sg, e, dv, ds);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      v_sg[s * ng + g] += dv[s];
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+        flux[(v * 2 + s) * ng + g] = 2.0 * ds[2 * s] * d[v][s] + ds[1] * d[v][1 - s];
+    }
+  }
+  e_g[g] = e;
+}
+
+template <int H>
+__global__ void __launch_bounds__(256) gga_divergence_kernel(const __grid_constant__ GradArgs ga, int64_t ng, int ns,
+                                                             double* __restrict__ v_sg,
+                                                             const double* __restrict__ flux) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (g >= ng) return;
+  const int s = blockIdx.y;
+  const int64_t st[3] = {(int64_t)ga.n[1] * ga.n[2], ga.n[2], 1};
+  int i[3];
+  i[0] = (int)div_mod(div_mod(g, ga.n[2], i[2]), ga.n[1], i[1]);
+  double v = v_sg[s * ng + g];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v -= axis_derivative<H>(ga, flux + (c * ns + s) * ng + g, c, i[c], st[c]);
+  v_sg[s * ng + g] = v;
 }
 
 static Par make_par(int code) {
@@ -249,4 +365,48 @@ extern "C" int gb_xc_calculate(int code, int nspins, int64_t ng, double* e_g, co
     xc::xc_polarized<<<(unsigned)blocks, threads, 0, (cudaStream_t)stream>>>(p, ng, e_g, n_sg, v_sg, sigma_xg,
                                                                             dedsigma_xg);
   return check_launch("xc kernel");
+}
+
+extern "C" int gb_gga_calculate(int code, int nspins, const gb_operator* grad0, const gb_operator* grad1,
+                                const gb_operator* grad2, double* e_g, const double* n_sg, double* v_sg,
+                                double* flux, void* stream) {
+  GB_REQUIRE(code == 0 || code == 1 || code == 2, "gb_gga_calculate: code must be 0 (PBE), 1 (revPBE) or 2 (RPBE)");
+  GB_REQUIRE(nspins == 1 || nspins == 2, "gb_gga_calculate: nspins must be 1 or 2");
+  GB_REQUIRE(grad0 && grad1 && grad2 && e_g && n_sg && v_sg && flux, "gb_gga_calculate: null pointer");
+  const gb_operator* op[3] = {grad0, grad1, grad2};
+  xc::GradArgs ga{};
+  for (int c = 0; c < 3; ++c) {
+    GB_REQUIRE(op[c]->real && op[c]->cfd && op[c]->H <= xc::GH, "gb_gga_calculate: gradients must be real, on the "
+                                                               "axes and of radius at most 4");
+    ga.H = std::max(ga.H, op[c]->H);
+    ga.c0[c] = op[c]->center;
+    for (int d = 0; d < 3; ++d) {
+      GB_REQUIRE(op[c]->n[d] == op[0]->n[d] && op[c]->pbc[d] == op[0]->pbc[d],
+                 "gb_gga_calculate: the gradients are on different grids");
+      for (int m = 0; m < 2 * HMAX + 1; ++m)
+        GB_REQUIRE(d == c || op[c]->a[d][m] == 0.0, "gb_gga_calculate: gradient c must lie along axis c");
+    }
+    ga.n[c] = (int)op[0]->n[c];
+    ga.pbc[c] = op[0]->pbc[c];
+    for (int m = -xc::GH; m <= xc::GH; ++m) ga.a[c][m + xc::GH] = op[c]->a[c][m + HMAX];
+  }
+  for (int c = 0; c < 3; ++c) GB_REQUIRE(ga.H <= ga.n[c], "gb_gga_calculate: stencil longer than domain");
+  const int64_t ng = op[0]->n[0] * op[0]->n[1] * op[0]->n[2];
+  const xc::Par p = xc::make_par(code);
+  const unsigned blocks = (unsigned)((ng + 255) / 256);
+  cudaStream_t st = (cudaStream_t)stream;
+#define GB_GGA(HH)                                                                                              \
+  case HH:                                                                                                      \
+    if (nspins == 1) xc::gga_flux_kernel<1, HH><<<blocks, 256, 0, st>>>(p, ga, ng, e_g, n_sg, v_sg, flux);     \
+    else xc::gga_flux_kernel<2, HH><<<blocks, 256, 0, st>>>(p, ga, ng, e_g, n_sg, v_sg, flux);                 \
+    xc::gga_divergence_kernel<HH><<<dim3(blocks, (unsigned)nspins), 256, 0, st>>>(ga, ng, nspins, v_sg, flux); \
+    break
+  switch (ga.H) {
+    GB_GGA(1);
+    GB_GGA(2);
+    GB_GGA(3);
+    GB_GGA(4);
+  }
+#undef GB_GGA
+  return check_launch("gga_flux_kernel / gga_divergence_kernel");
 }

@@ -91,9 +91,14 @@ class GGA(XCFunctional):
         from gpaw_b200.fd_operators import Gradient
         XCFunctional.set_grid_descriptor(self, gd)
         self.grad_v = [Gradient(gd, v, n=self.stencil_range) for v in range(3)]
+        # every gradient along its own axis: the two-launch form applies
+        self.on_axes = all(not op.offset_pc[:, [c for c in range(3) if c != v]].any()
+                           for v, op in enumerate(self.grad_v))
 
     def calculate_impl(self, gd, n_sg, v_sg, e_g):
         nspins = n_sg.shape[0]
+        if self.on_axes:
+            return self._calculate_on_axes(nspins, n_sg, v_sg, e_g)
         # sigma and grad n (gpaw/xc/gga.py:106-133): one stencil launch per
         # Cartesian direction covers both spins
         gradn_vsg = torch.empty((3,) + tuple(n_sg.shape), dtype=n_sg.dtype,
@@ -118,6 +123,24 @@ class GGA(XCFunctional):
                     flux[s] += dedsigma_xg[1] * gradn_vsg[v, 1 - s]
             self.grad_v[v].apply(flux, out)
             v_sg -= out
+
+
+    def _calculate_on_axes(self, nspins, n_sg, v_sg, e_g):
+        """Gradients, functional and divergence in two launches
+        (gb_gga_calculate)."""
+        assert 1 <= nspins <= 2
+        G = self.grad_v[0].shape
+        if tuple(n_sg.shape[1:]) != G:
+            raise ValueError(f'shape mismatch: {tuple(n_sg.shape)} for grid {G}')
+        assert tuple(e_g.shape) == G and tuple(v_sg.shape) == (nspins,) + G
+        for a in (e_g, n_sg, v_sg):
+            if a.dtype != torch.float64:
+                raise ValueError('XC arrays are float64')
+        nat.require_cuda(e_g, n_sg, v_sg)
+        flux = torch.empty((3,) + tuple(n_sg.shape), dtype=n_sg.dtype, device=n_sg.device)
+        nat.check(nat.lib().gb_gga_calculate(
+            self.kernel.code, nspins, *[op.handle for op in self.grad_v], nat.ptr(e_g),
+            nat.ptr(n_sg), nat.ptr(v_sg), nat.ptr(flux), nat.stream_of(e_g)), 'gb_gga_calculate')
 
 
 def XC(name, **kwargs):

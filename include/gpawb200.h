@@ -289,6 +289,15 @@ int gb_lfc_derivative(const gb_lfc* lfc, const void* a_xG, void* c_xMv,
 int gb_xc_calculate(int code, int nspins, int64_t ng, double* e_g,
                     const double* n_sg, double* v_sg, const double* sigma_xg,
                     double* dedsigma_xg, void* stream);
+/* GGA on the grid in two launches (replaces the gradient, sum, functional and
+ * divergence passes of gpaw/xc/gga.py:106-200): grad0..2 are the operators of
+ * d/dx, d/dy, d/dz, each along its own axis (radius <= 4, one grid); e_g is
+ * overwritten, v_sg (nspins grids) is added to, flux is a work space of
+ * 3 nspins grids.  code: 0 PBE, 1 revPBE, 2 RPBE.  FP64. */
+int gb_gga_calculate(int code, int nspins, const gb_operator* grad0,
+                     const gb_operator* grad1, const gb_operator* grad2,
+                     double* e_g, const double* n_sg, double* v_sg,
+                     double* flux, void* stream);
 
 /* ======================================================================
  * Density accumulation  -- replaces _gpaw.add_to_density
