@@ -18,8 +18,8 @@
 // channels' weights come in one 16-byte broadcast load; every thread keeps
 // 4 (8 for one output channel) consecutive points x all output channels in
 // registers.  Backward-weight: CTAs
-// over (co, ci) pairs x chunks of the points; each reduces its chunk's 27
-// sums and adds them to dw with FP32 atomics (dw accumulates, as before).
+// over (co, ci) pairs x chunks of the points, each writing its 27 partial
+// sums; a second kernel adds them in a fixed order (dw accumulates).
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <mutex>
@@ -345,63 +345,110 @@ static int conv16_launch(const ConvArgs& a, size_t smem, cudaStream_t st) {
 }
 
 // dw[co][ci][k] += sum_b sum_p dy[b][co][p] x[b][ci][p + o_k]   (FP32)
-// grid: (cin * cout channel pairs) x (chunks of the band x point range);
-// each CTA reduces its chunk in a fixed order and writes its 27 sums to
-// part[pair][chunk]; conv3d_bwd_w_reduce_kernel adds them to dw in chunk
-// order, so the gradient does not depend on scheduling
-__global__ void __launch_bounds__(256) conv3d_bwd_w_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                                                           float* __restrict__ part, int64_t nb, int cin, int cout,
-                                                           int n0, int n1, int n2, int pbc0, int pbc1, int pbc2) {
-  const int co = blockIdx.x / cin, ci = blockIdx.x % cin;
-  const int64_t n012 = (int64_t)n0 * n1 * n2;
-  const int64_t total = nb * n012;
-  const int64_t e0 = total * blockIdx.y / gridDim.y, e1 = total * (blockIdx.y + 1) / gridDim.y;
-  float acc[27];
+// grid: (input channel, block of COB output channels) x (splits of the work
+// items).  An item is a column (axis 1, axis 2) of one band over a chunk of
+// planes: a thread marches along axis 0 with the 3 x 3 x 3 window of x in
+// registers, so a point costs 9 loads of x and COB of dy for 27 COB FMAs
+// (the per-point form, 27 loads with their boundary tests for 27 FMAs, was
+// bound by its address arithmetic: 2770 us for the five gradients of a
+// 16 x 56^3 training step).  Each CTA reduces its items in a fixed order and
+// writes its sums to part[pair][split]; conv3d_bwd_w_reduce_kernel adds them
+// to dw in a fixed order, so the gradient does not depend on scheduling.
+constexpr int BW_NT = 128;
+template <int COB>
+__global__ void __launch_bounds__(BW_NT, 4) conv3d_bwd_w_kernel(const float* __restrict__ x, const float* __restrict__ dy,
+                                                             float* __restrict__ part, int cin, int cout, int n0,
+                                                             int n1, int n2, int pbc0, int pbc1, int pbc2, int npc,
+                                                             int64_t items) {
+  const int co0 = (int)(blockIdx.x / cin) * COB, ci = blockIdx.x % cin;
+  const int64_t n12 = (int64_t)n1 * n2, n012 = n12 * n0;
+  const int64_t i0 = items * blockIdx.y / gridDim.y, i1 = items * (blockIdx.y + 1) / gridDim.y;
+  float acc[COB][27];
 #pragma unroll
-  for (int k = 0; k < 27; ++k) acc[k] = 0.f;
-  for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const int64_t b = e / n012, p = e % n012;
-    const int g2 = (int)(p % n2), g1 = (int)((p / n2) % n1), g0 = (int)(p / ((int64_t)n1 * n2));
-    const float d = dy[(b * cout + co) * n012 + p];
-    if (d == 0.f) continue;
+  for (int c = 0; c < COB; ++c)
+#pragma unroll
+    for (int k = 0; k < 27; ++k) acc[c][k] = 0.f;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += BW_NT) {
+    int y, z, pc;
+    int64_t b = div_mod(i, n2, z);
+    b = div_mod(div_mod(b, n1, y), npc, pc);
+    const int64_t col = (int64_t)y * n2 + z;
+    const int p_beg = (int)((int64_t)n0 * pc / npc), p_end = (int)((int64_t)n0 * (pc + 1) / npc);
+    // the nine in-plane neighbours: offset from the column, or outside
+    int off[9];
+    bool ok[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      int h1 = y + j / 3 - 1, h2 = z + j % 3 - 1;
+      ok[j] = true;
+      if (h1 < 0 || h1 >= n1) { if (pbc1) h1 = cwrap(h1, n1); else ok[j] = false; }
+      if (h2 < 0 || h2 >= n2) { if (pbc2) h2 = cwrap(h2, n2); else ok[j] = false; }
+      off[j] = h1 * n2 + h2;
+    }
     const float* xb = x + (b * cin + ci) * n012;
+    const float* db = dy + (b * cout + co0) * n012 + col;
+    auto plane = [&](int p, float (&w)[9]) {
+      bool in = true;
+      if (p < 0 || p >= n0) { if (pbc0) p = cwrap(p, n0); else in = false; }
+      const float* xp = xb + (in ? p : 0) * n12;
 #pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      int h0 = g0 + k / 9 - 1, h1 = g1 + (k / 3) % 3 - 1, h2 = g2 + k % 3 - 1;
-      bool ok = true;
-      if (h0 < 0 || h0 >= n0) { if (pbc0) h0 = cwrap(h0, n0); else ok = false; }
-      if (h1 < 0 || h1 >= n1) { if (pbc1) h1 = cwrap(h1, n1); else ok = false; }
-      if (h2 < 0 || h2 >= n2) { if (pbc2) h2 = cwrap(h2, n2); else ok = false; }
-      if (ok) acc[k] = fmaf(d, xb[((int64_t)h0 * n1 + h1) * n2 + h2], acc[k]);
+      for (int j = 0; j < 9; ++j) w[j] = in && ok[j] ? __ldg(xp + off[j]) : 0.f;
+    };
+    float w[3][9];
+    plane(p_beg - 1, w[0]);
+    plane(p_beg, w[1]);
+    for (int pb = p_beg; pb < p_end; pb += 3) {
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int p = pb + u;
+        if (p >= p_end) break;
+        float d[COB];
+#pragma unroll
+        for (int c = 0; c < COB; ++c) d[c] = __ldg(db + c * n012 + p * n12);
+        plane(p + 1, w[(u + 2) % 3]);
+#pragma unroll
+        for (int c = 0; c < COB; ++c) {
+          if (d[c] == 0.f) continue;
+#pragma unroll
+          for (int k = 0; k < 27; ++k) acc[c][k] = fmaf(d[c], w[(u + k / 9) % 3][k % 9], acc[c][k]);
+        }
+      }
     }
   }
-  __shared__ float red[8][27];
+  __shared__ float red[BW_NT / 32][COB * 27];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < 27; ++k) {
-    float v = acc[k];
+  for (int c = 0; c < COB; ++c)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][k] = v;
-  }
+    for (int k = 0; k < 27; ++k) {
+      float v = acc[c][k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) red[warp][c * 27 + k] = v;
+    }
   __syncthreads();
-  if (threadIdx.x < 27) {
+  for (int e = threadIdx.x; e < COB * 27; e += BW_NT) {
     float v = 0.f;
-    for (int w = 0; w < (int)(blockDim.x / 32); ++w) v += red[w][threadIdx.x];
-    part[((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * 27 + threadIdx.x] = v;
+#pragma unroll
+    for (int w = 0; w < BW_NT / 32; ++w) v += red[w][e];
+    const int64_t pair = (int64_t)(co0 + e / 27) * cin + ci;
+    part[(pair * gridDim.y + blockIdx.y) * 27 + e % 27] = v;
   }
 }
 
-// dw[pair][k] += sum over chunks c (in order) of part[pair][c][k]
-__global__ void conv3d_bwd_w_reduce_kernel(const float* __restrict__ part, int nchunk, int n,
+// dw[pair][k] += sum over splits of part[pair][split][k]: one warp per weight,
+// lane l adds splits l, l + 32, ... and the lanes are added as a tree
+__global__ void conv3d_bwd_w_reduce_kernel(const float* __restrict__ part, int nsplit, int n,
                                            float* __restrict__ dw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= n) return;
   const int pair = i / 27, k = i - pair * 27;
-  const float* p = part + (int64_t)pair * nchunk * 27 + k;
+  const float* p = part + (int64_t)pair * nsplit * 27 + k;
   float s = 0.f;
-  for (int c = 0; c < nchunk; ++c) s += p[(int64_t)c * 27];
-  dw[i] += s;
+  for (int c = lane; c < nsplit; c += 32) s += p[(int64_t)c * 27];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) dw[i] += s;
 }
 
 template <int CIN, int COUT, int CZT>
@@ -494,12 +541,15 @@ int gb_conv3d_backward_weight(const float* x, const float* dy, float* dw, int64_
   GB_REQUIRE(x && dy && dw && n_c && pbc_c && nb >= 0 && cin > 0 && cout > 0,
              "gb_conv3d_backward_weight: bad arguments");
   if (nb == 0) return GB_OK;
-  // enough chunks to fill the GPU about four times over, each >= 4096 points
-  const int64_t total = nb * n_c[0] * n_c[1] * n_c[2];
-  const int64_t want = std::max<int64_t>(1, (int64_t)sm_count() * 8 / (cin * cout));
-  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(want, total / 4096));
-  const int nchunk = (int)std::min<int64_t>(chunks, 65535);
-  dim3 grid((unsigned)(cin * cout), (unsigned)nchunk);
+  // plane chunks of at most 14; splits enough for four CTAs per SM, each with
+  // at least one item per thread
+  const int cob = cout % 2 == 0 ? 2 : 1;
+  const int64_t groups = (int64_t)cin * (cout / cob);
+  const int npc = (int)((n_c[0] + 13) / 14);
+  const int64_t items = nb * npc * n_c[1] * n_c[2];
+  const int64_t want = std::max<int64_t>(1, (int64_t)sm_count() * 4 / groups);
+  const int nchunk = (int)std::min<int64_t>(std::max<int64_t>(1, std::min<int64_t>(want, items / BW_NT)), 65535);
+  dim3 grid((unsigned)groups, (unsigned)nchunk);
   // per-CTA partial sums in stream-ordered memory (freed on the stream
   // after the reduction), so concurrent calls on different streams do not
   // share them; from a pool of this library that keeps freed memory, so
@@ -510,12 +560,13 @@ int gb_conv3d_backward_weight(const float* x, const float* dy, float* dw, int64_
   if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&part),
                                        (size_t)cin * cout * nchunk * 27 * sizeof(float), pool, st) != cudaSuccess)
     return fail(GB_E_NOMEM, "gb_conv3d_backward_weight: partial-sum allocation failed");
-  conv3d_bwd_w_kernel<<<grid, 256, 0, st>>>(x, dy, part, nb, cin, cout, (int)n_c[0], (int)n_c[1], (int)n_c[2],
-                                            pbc_c[0], pbc_c[1], pbc_c[2]);
+  auto kern = cob == 2 ? conv3d_bwd_w_kernel<2> : conv3d_bwd_w_kernel<1>;
+  kern<<<grid, BW_NT, 0, st>>>(x, dy, part, cin, cout, (int)n_c[0], (int)n_c[1], (int)n_c[2], pbc_c[0], pbc_c[1],
+                               pbc_c[2], npc, items);
   int rc = check_launch("conv3d_bwd_w_kernel");
   if (rc == GB_OK) {
     const int n = cin * cout * 27;
-    conv3d_bwd_w_reduce_kernel<<<(n + 255) / 256, 256, 0, st>>>(part, nchunk, n, dw);
+    conv3d_bwd_w_reduce_kernel<<<(n + 7) / 8, 256, 0, st>>>(part, nchunk, n, dw);
     rc = check_launch("conv3d_bwd_w_reduce_kernel");
   }
   cudaFreeAsync(part, st);
