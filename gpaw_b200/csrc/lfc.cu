@@ -25,6 +25,7 @@
 #include <map>
 #include <type_traits>
 #include <vector>
+#include <cooperative_groups.h>
 #include "internal.cuh"
 #include "spline.cuh"
 
@@ -58,13 +59,17 @@ struct gb_lfc {
   int* row_G = nullptr;       // [rows] grid point of every global row
   int64_t* vol_aoff = nullptr;  // [nW] offset (doubles) of row0 in A
   std::vector<int> h_gr_nm;
-  // all-band add for real data (every volume has <= 16 functions): A rows
-  // zero-padded to fast_nmax, in contribution order
-  int fast_nmax = 0;          // 8 or 16; 0 = not built
-  bool full32 = false;        // every contribution: nm == fast_nmax, M and nM multiples of 4
-  bool full64 = false;        // the same with multiples of 2 (16-byte FP64 loads)
-  float* Ac32 = nullptr;      // [C][fast_nmax]
-  double* Ac64 = nullptr;
+  // FP64 tensor-core add / integrate for real data (every volume has <= 16
+  // functions): one entry per (volume, 8-point sub-tile of the flattened grid
+  // it touches) with its values there as nf dense [m][p] 8 x 8 blocks
+  int nf = 0;                 // 1 or 2 blocks per entry; 0 = not built
+  int ns = 0;                 // sub-tiles with entries
+  int2* st_sub = nullptr;     // [ns] sub-tile | mask of its covered points
+  int* st_eoff = nullptr;     // [ns + 1] entries of each
+  int2* st_M = nullptr;       // [ne] first function and function count of an entry
+  double* st_A = nullptr;     // [ne][nf][8][8]
+  int* sg_off = nullptr;      // [ngroups + 1] entries of each function group:
+  int2* sg_e = nullptr;       //   entry | sub-tile, in the order of the sub-tiles
   // brick-tiled FP32 add / integrate for real data (every volume has <= 8
   // functions, nG a multiple of 4): 32-point chunks of four 8-point
   // sub-tiles; one entry per (volume, sub-tile it touches) with the volume's
@@ -361,146 +366,243 @@ __global__ void __launch_bounds__(NT) lfc_integrate_kernel(const LfcView l, cons
   }
 }
 
-// ------------------------------------------------ real data, all bands
+// ------------------------------------------------ real data, FP64 tensor cores
 // For real data (Gamma point: every periodic image has phase 1) and at most
-// 16 functions per volume, the add runs every band in one pass: one thread
-// per covered point holds the zero-padded A rows of its first KREG
-// contributions in registers (a copy of A in contribution order, so a warp's
-// row loads are contiguous) and loops over the bands XU at a time, issuing
-// the XU read-modify-write loads of a[x][G] before the coefficient loads and
-// FMAs of those bands.  Per band it sums the contributions in point order,
-// m within each, as lfc_add_kernel does, so the two give identical results.
-// (The same all-band treatment of the integrate, with row tiles of A staged in
-// shared memory per (group, 16-band) CTA, measured no faster than
-// lfc_integrate_kernel on the Si64 shape and slower in FP64, so the integrate
-// keeps the kernel above.)
-template <typename T, int NMAX, bool FULL>
-__device__ __forceinline__ void load_coef(const T* __restrict__ cx, int nm, T (&v)[NMAX]) {
-  if constexpr (FULL) {
-    // every contribution has NMAX functions at a 16-byte aligned offset
-    if constexpr (sizeof(T) == 4) {
+// 16 functions per volume both products run as m16n8k8 FP64 MMAs on 16 bands
+// x 8 grid points x 8 functions, the three operands exactly as they lie in
+// memory: bands x points (a), points x functions (an entry's dense block) and
+// bands x functions (c).  FP32 data are widened on the way in and rounded
+// once on the way out.
+//   integrate: a cluster of four CTAs takes one function group and 16 NB
+//     bands; its 32 warps split the group's entries evenly, and the 32 sums
+//     are added in warp order (shared, then distributed shared memory).
+//   add: a warp takes one sub-tile and 16 NB bands, sums its entries and adds
+//     the sum to the covered points.
+// The split depends on the object alone and every sum has one order, so the
+// results depend neither on scheduling nor on how the bands are blocked.
+// A non-finite value at an uncovered point (integrate) or in the coefficients
+// of another volume (add) can reach the sums of its own sub-tile.
+//
+// Bound by L1 requests (a fragment load touches eight rows).  71^3 grid, 24
+// atoms x 9 functions of radius 2.5 A, 96 FP64 bands: integrate 189 -> 84 us,
+// add 196 -> 140 us against the point-major kernels (gathered rows, one point
+// per thread).  FP32 with at most eight functions keeps the brick tiling
+// below, which is as fast there (an FP32 form of this add with coefficients
+// and blocks read through L1 took 140 us against 133 us).
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+constexpr int LM_CLUSTER = 4;              // CTAs per (function group, band block)
+constexpr int LM_WARPS = 8;
+
+template <typename T, int NB, int NF>
+__global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WARPS)
+    lfc_integrate_mma_kernel(const int* __restrict__ sg_off, const int2* __restrict__ sg_e,
+                             const double* __restrict__ st_A, const int* __restrict__ gr_M,
+                             const int* __restrict__ gr_nm, const T* __restrict__ a_xG, T* __restrict__ c_xM,
+                             int64_t nx, int64_t nG, int nM, double dv) {
+  extern __shared__ __align__(16) double lm_red[];   // [LM_WARPS][NB * NF * 4][32]
+  constexpr int NE = NB * NF * 128;
+  const int rank = blockIdx.x % LM_CLUSTER, gi = blockIdx.x / LM_CLUSTER;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t x0 = (int64_t)blockIdx.y * 16 * NB;
+  const int M = gr_M[gi], nm = gr_nm[gi];
+  const int e0 = sg_off[gi], ne = sg_off[gi + 1] - e0, w = rank * LM_WARPS + warp;
+  const int i0 = e0 + (int)((int64_t)ne * w / (LM_CLUSTER * LM_WARPS));
+  const int i1 = e0 + (int)((int64_t)ne * (w + 1) / (LM_CLUSTER * LM_WARPS));
+  const T* row[NB][2];
+  bool on[NB][2];
 #pragma unroll
-      for (int h = 0; h < NMAX / 4; ++h) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(cx) + h);
-        v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t x = x0 + 16 * i + 8 * h + g;
+      on[i][h] = x < nx;
+      row[i][h] = a_xG + (on[i][h] ? x : 0) * nG;
+    }
+  double acc[NB][NF][4];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[i][f][k] = 0.0;
+#pragma unroll 2
+  for (int q = i0; q < i1; ++q) {
+    const int2 es = sg_e[q];
+    const int64_t p = (int64_t)es.y * 8 + t;
+    const bool in0 = p < nG, in1 = p + 4 < nG;
+    const double* blk = st_A + (int64_t)es.x * (NF * 64) + g * 8 + t;
+    double b[NF][2];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      b[f][0] = __ldg(blk + f * 64);
+      b[f][1] = __ldg(blk + f * 64 + 4);
+    }
+    double av[NB][4];
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        av[i][h] = on[i][h] && in0 ? (double)__ldg(row[i][h] + p) : 0.0;
+        av[i][2 + h] = on[i][h] && in1 ? (double)__ldg(row[i][h] + p + 4) : 0.0;
       }
-    } else {
 #pragma unroll
-      for (int h = 0; h < NMAX / 2; ++h) {
-        const double2 a = __ldg(reinterpret_cast<const double2*>(cx) + h);
-        v[2 * h] = a.x; v[2 * h + 1] = a.y;
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int f = 0; f < NF; ++f) mma_f64(acc[i][f], av[i], b[f][0], b[f][1]);
+  }
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) lm_red[warp * NE + ((i * NF + f) * 4 + k) * 32 + lane] = acc[i][f][k];
+  __syncthreads();
+  for (int e = threadIdx.x; e < NE; e += 32 * LM_WARPS) {
+    double v = lm_red[e];
+#pragma unroll
+    for (int ww = 1; ww < LM_WARPS; ++ww) v += lm_red[ww * NE + e];
+    lm_red[e] = v;
+  }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int e = rank * 32 * LM_WARPS + threadIdx.x; e < NE; e += LM_CLUSTER * 32 * LM_WARPS) {
+    double v = 0.0;
+#pragma unroll
+    for (int r = 0; r < LM_CLUSTER; ++r) v += cluster.map_shared_rank(lm_red, r)[e];
+    const int l = e & 31, k = (e >> 5) & 3, f = (e >> 7) % NF, i = (e >> 7) / NF;
+    const int64_t x = x0 + 16 * i + 8 * (k >> 1) + (l >> 2);
+    const int m = f * 8 + 2 * (l & 3) + (k & 1);
+    if (x < nx && m < nm) {
+      T* cp = c_xM + x * nM + M + m;
+      *cp = (T)fma(dv, v, (double)*cp);
+    }
+  }
+  cluster.sync();        // the other CTAs may still be reading this one's sums
+}
+
+template <typename T, int NB, int NF>
+__global__ void __launch_bounds__(32 * LM_WARPS)
+    lfc_add_mma_kernel(int ns, const int2* __restrict__ st_sub, const int* __restrict__ st_eoff,
+                       const int2* __restrict__ st_M, const double* __restrict__ st_A, const T* __restrict__ c_xM,
+                       T* __restrict__ a_xG, int64_t nx, int64_t nG, int nM) {
+  const int s = blockIdx.x * LM_WARPS + (threadIdx.x >> 5);
+  if (s >= ns) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t x0 = (int64_t)blockIdx.y * 16 * NB;
+  const int2 sub = st_sub[s];
+  const int e0 = st_eoff[s], e1 = st_eoff[s + 1];
+  const T* row[NB][2];
+  bool on[NB][2];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t x = x0 + 16 * i + 8 * h + g;
+      on[i][h] = x < nx;
+      row[i][h] = c_xM + (on[i][h] ? x : 0) * nM;
+    }
+  double acc[NB][4];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[i][k] = 0.0;
+  for (int e = e0; e < e1; ++e) {
+    const int2 mn = st_M[e];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      if (f * 8 >= mn.y) break;
+      const double* blk = st_A + ((int64_t)e * NF + f) * 64 + t * 8 + g;
+      const double b0 = __ldg(blk), b1 = __ldg(blk + 32);
+      const int m = f * 8 + t;
+      const bool in0 = m < mn.y, in1 = m + 4 < mn.y;
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        double cv[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const T* c = row[i][h] + mn.x + m;
+          cv[h] = on[i][h] && in0 ? (double)__ldg(c) : 0.0;
+          cv[2 + h] = on[i][h] && in1 ? (double)__ldg(c + 4) : 0.0;
+        }
+        mma_f64(acc[i], cv, b0, b1);
       }
     }
-  } else {
-#pragma unroll
-    for (int m = 0; m < NMAX; ++m) v[m] = m < nm ? __ldg(cx + m) : (T)0;
   }
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int pt = 2 * t + (k & 1);
+      const int64_t x = x0 + 16 * i + 8 * (k >> 1) + g;
+      if (x < nx && (sub.y >> pt & 1)) {
+        T* ap = a_xG + x * nG + (int64_t)sub.x * 8 + pt;
+        *ap = (T)((double)*ap + acc[i][k]);
+      }
+    }
 }
 
-template <typename T, int NMAX>
-__device__ __forceinline__ void load_padded_row(const T* __restrict__ src, T (&v)[NMAX]) {
-  if constexpr (sizeof(T) == 4) {
-#pragma unroll
-    for (int h = 0; h < NMAX / 4; ++h) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(src) + h);
-      v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
-    }
-  } else {
-#pragma unroll
-    for (int h = 0; h < NMAX / 2; ++h) {
-      const double2 a = __ldg(reinterpret_cast<const double2*>(src) + h);
-      v[2 * h] = a.x; v[2 * h + 1] = a.y;
-    }
-  }
+// A single grid (a density or potential, not a block of bands) would fill one
+// row of sixteen of every tile and keeps the point-major kernels; the launch
+// grid's second dimension bounds the bands.
+static bool mma_usable(const gb_lfc* l, int64_t nx) { return l->nf && nx > 1 && nx < 65535 * 16; }
+
+// 16-band tiles per warp: at most 5, the blocks of a call as even as possible
+static int mma_tiles(int64_t nx) {
+  const int64_t tiles = (nx + 15) / 16, blocks = (tiles + 4) / 5;
+  return (int)((tiles + blocks - 1) / blocks);
 }
 
-// acc[u] += sum_m A[m] c[x0 + u][M + m], u < NU, cx = &c[x0][M] (the
-// contribution's sum is formed first, then added, as in lfc_add_kernel)
-template <typename T, int NMAX, bool FULL, int NU>
-__device__ __forceinline__ void add_contribution(const T (&A)[NMAX], const T* __restrict__ cx, int nM, int nm,
-                                                 T (&acc)[NU]) {
-#pragma unroll
-  for (int u = 0; u < NU; ++u) {
-    T cv[NMAX];
-    load_coef<T, NMAX, FULL>(cx, nm, cv);
-    T t = (T)0;
-#pragma unroll
-    for (int m = 0; m < NMAX; ++m) t = fmadd(t, A[m], cv[m]);
-    acc[u] += t;
-    cx += nM;
+template <typename T, int NB, int NF>
+static int integrate_mma_nb(const gb_lfc* l, const void* a, void* c, int64_t nx, cudaStream_t st) {
+  constexpr int smem = LM_WARPS * NB * NF * 128 * (int)sizeof(double);
+  auto kern = lfc_integrate_mma_kernel<T, NB, NF>;
+  static bool set = false;
+  if (!set && smem > 48 * 1024) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return check_launch("lfc shared memory");
+    set = true;
   }
+  const dim3 grid((unsigned)(l->ngroups * LM_CLUSTER), (unsigned)((nx + 16 * NB - 1) / (16 * NB)));
+  kern<<<grid, 32 * LM_WARPS, smem, st>>>(l->sg_off, l->sg_e, l->st_A, l->gr_M, l->gr_nm, (const T*)a, (T*)c, nx,
+                                          l->nG, l->nM, l->dv);
+  return check_launch("lfc_integrate_mma_kernel");
 }
 
-// bands x0 .. x0+NU-1 of one point: a[x][G] += sum_k sum_m A_k[m] c[x][M_k + m]
-template <typename T, int NMAX, int KREG, bool FULL, int NU>
-__device__ __forceinline__ void add_point_bands(const T (&A)[KREG][NMAX], const T* const (&cb)[KREG],
-                                                const int (&nmk)[KREG], int K, int k0,
-                                                const int* __restrict__ ct_M, const int* __restrict__ ct_nm,
-                                                const T* __restrict__ Ac, const T* __restrict__ c_xM, int nM,
-                                                int64_t x0, T* __restrict__ ax, int64_t nG) {
-  // the read-modify-write loads first: their latency overlaps the FMAs
-  T av[NU], acc[NU];
-  {
-    const T* q = ax;
-#pragma unroll
-    for (int u = 0; u < NU; ++u) {
-      av[u] = *q;
-      acc[u] = (T)0;
-      q += nG;
-    }
-  }
-  const int64_t xo = x0 * nM;
-#pragma unroll
-  for (int k = 0; k < KREG; ++k)
-    if (k < K) add_contribution<T, NMAX, FULL, NU>(A[k], cb[k] + xo, nM, nmk[k], acc);
-  for (int k = KREG; k < K; ++k) {
-    T Ak[NMAX];
-    load_padded_row<T, NMAX>(Ac + (int64_t)(k0 + k) * NMAX, Ak);
-    add_contribution<T, NMAX, FULL, NU>(Ak, c_xM + ct_M[k0 + k] + xo, nM, ct_nm[k0 + k], acc);
-  }
-  T* q = ax;
-#pragma unroll
-  for (int u = 0; u < NU; ++u) {
-    *q = av[u] + acc[u];
-    q += nG;
-  }
+template <typename T, int NB, int NF>
+static int add_mma_nb(const gb_lfc* l, const void* c, void* a, int64_t nx, cudaStream_t st) {
+  const dim3 grid((unsigned)((l->ns + LM_WARPS - 1) / LM_WARPS), (unsigned)((nx + 16 * NB - 1) / (16 * NB)));
+  lfc_add_mma_kernel<T, NB, NF><<<grid, 32 * LM_WARPS, 0, st>>>(l->ns, l->st_sub, l->st_eoff, l->st_M, l->st_A,
+                                                                (const T*)c, (T*)a, nx, l->nG, l->nM);
+  return check_launch("lfc_add_mma_kernel");
 }
 
-template <typename T, int NMAX, int KREG, bool FULL, int XU>
-__global__ void __launch_bounds__(256) lfc_add_bands_kernel(const int* __restrict__ pt_G,
-                                                            const int* __restrict__ pt_off,
-                                                            const int* __restrict__ ct_M,
-                                                            const int* __restrict__ ct_nm,
-                                                            const T* __restrict__ Ac, int64_t P,
-                                                            const T* __restrict__ c_xM, int nM,
-                                                            T* __restrict__ a_xG, int64_t nG, int64_t nx) {
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const int G = pt_G[p];
-  const int k0 = pt_off[p], K = pt_off[p + 1] - k0;
-  T A[KREG][NMAX];
-  const T* cb[KREG];
-  int nmk[KREG];
-#pragma unroll
-  for (int k = 0; k < KREG; ++k) {
-    if (k < K) {
-      load_padded_row<T, NMAX>(Ac + (int64_t)(k0 + k) * NMAX, A[k]);
-      cb[k] = c_xM + ct_M[k0 + k];
-      nmk[k] = ct_nm[k0 + k];
-    } else {
-#pragma unroll
-      for (int m = 0; m < NMAX; ++m) A[k][m] = (T)0;
-      cb[k] = c_xM;
-      nmk[k] = 0;
-    }
+#define GB_LFC_NB(FN, ...)                                                    \
+  switch (mma_tiles(nx)) {                                                    \
+    case 1: return l->nf == 1 ? FN<T, 1, 1>(__VA_ARGS__) : FN<T, 1, 2>(__VA_ARGS__); \
+    case 2: return l->nf == 1 ? FN<T, 2, 1>(__VA_ARGS__) : FN<T, 2, 2>(__VA_ARGS__); \
+    case 3: return l->nf == 1 ? FN<T, 3, 1>(__VA_ARGS__) : FN<T, 3, 2>(__VA_ARGS__); \
+    case 4: return l->nf == 1 ? FN<T, 4, 1>(__VA_ARGS__) : FN<T, 4, 2>(__VA_ARGS__); \
+    default: return l->nf == 1 ? FN<T, 5, 1>(__VA_ARGS__) : FN<T, 5, 2>(__VA_ARGS__); \
   }
-  const int64_t nfull = nx / XU * XU;
-  T* ax = a_xG + G;
-  for (int64_t x0 = 0; x0 < nfull; x0 += XU, ax += XU * nG)
-    add_point_bands<T, NMAX, KREG, FULL, XU>(A, cb, nmk, K, k0, ct_M, ct_nm, Ac, c_xM, nM, x0, ax, nG);
-  for (int64_t x0 = nfull; x0 < nx; ++x0, ax += nG)
-    add_point_bands<T, NMAX, KREG, FULL, 1>(A, cb, nmk, K, k0, ct_M, ct_nm, Ac, c_xM, nM, x0, ax, nG);
+template <typename T>
+static int integrate_mma(const gb_lfc* l, const void* a, void* c, int64_t nx, cudaStream_t st) {
+  if (l->ngroups == 0) return GB_OK;
+  GB_LFC_NB(integrate_mma_nb, l, a, c, nx, st)
 }
+template <typename T>
+static int add_mma(const gb_lfc* l, const void* c, void* a, int64_t nx, cudaStream_t st) {
+  if (l->ns == 0) return GB_OK;
+  GB_LFC_NB(add_mma_nb, l, c, a, nx, st)
+}
+#undef GB_LFC_NB
 
 template <typename T, int NM>
 static int integrate_nm(const gb_lfc* l, int gbeg, int gcount, const void* a, void* c, int64_t nx, int q,
@@ -524,28 +626,6 @@ static int nm_class(int nm) {
   return 0;
 }
 
-template <typename T>
-static int add_fast(const gb_lfc* l, const void* c, void* a, int64_t nx, cudaStream_t st) {
-  const T* Ac;
-  if constexpr (sizeof(T) == 4) Ac = l->Ac32; else Ac = l->Ac64;
-  const bool full = (sizeof(T) == 4 ? l->full32 : l->full64) && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
-  constexpr int NT = 256, XU = 8;
-  const unsigned grid = (unsigned)((l->P + NT - 1) / NT);
-  const T* cc = (const T*)c;
-  T* aa = (T*)a;
-#define GB_ADD_BANDS(NMAX, KREG, FULL)                                                                        \
-  lfc_add_bands_kernel<T, NMAX, KREG, FULL, XU><<<grid, NT, 0, st>>>(l->pt_G, l->pt_off, l->ct_M, l->ct_nm, Ac, \
-                                                                      l->P, cc, l->nM, aa, l->nG, nx)
-  constexpr int K8 = sizeof(T) == 4 ? 4 : 2, K16 = sizeof(T) == 4 ? 2 : 1;
-  if (l->fast_nmax == 8) {
-    if (full) GB_ADD_BANDS(8, K8, true); else GB_ADD_BANDS(8, K8, false);
-  } else {
-    if (full) GB_ADD_BANDS(16, K16, true); else GB_ADD_BANDS(16, K16, false);
-  }
-#undef GB_ADD_BANDS
-  return check_launch("lfc_add_bands_kernel");
-}
-
 static bool tiles_usable(const gb_lfc* l, const void* a);
 static int integrate_tiles(const gb_lfc* l, const float* a, float* c, int64_t nx, cudaStream_t st);
 
@@ -555,6 +635,9 @@ static int integrate_t(const gb_lfc* l, const void* a, void* c, int64_t nx, int 
   if constexpr (std::is_same<T, float>::value) {
     if (tiles_usable(l, a))
       return integrate_tiles(l, static_cast<const float*>(a), static_cast<float*>(c), nx, st);
+  }
+  if constexpr (!Elem<T>::cplx) {
+    if (mma_usable(l, nx)) return integrate_mma<T>(l, a, c, nx, st);
   }
   // groups are sorted by nm on the host; one launch per padded class
   int g = 0;
@@ -927,7 +1010,7 @@ static int add_t(const gb_lfc* l, const void* c, void* a, int64_t nx, int q, cud
     if (tiles_usable(l, a)) return add_tiles(l, static_cast<const float*>(c), static_cast<float*>(a), nx, st);
   }
   if constexpr (!Elem<T>::cplx) {
-    if (l->fast_nmax) return add_fast<T>(l, c, a, nx, st);
+    if (mma_usable(l, nx)) return add_mma<T>(l, c, a, nx, st);
   }
   switch (nm_class(l->maxnm)) {
     case 1: return add_nm<T, 8, 1>(l, c, a, nx, q, st, per_q);
@@ -1176,20 +1259,52 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     for (int W : kv.second) gv_W.push_back(W);
     gr_voff.push_back((int)gv_W.size());
   }
-  // zero-padded A rows in contribution order for the all-band real add
-  std::vector<double> hAc;
-  if (l->maxnm <= 16) {
-    const int F = l->maxnm <= 8 ? 8 : 16;
-    l->fast_nmax = F;
-    bool full32 = nM % 4 == 0, full64 = nM % 2 == 0;
-    hAc.assign(ct_aoff.size() * F, 0.0);
-    for (size_t c = 0; c < ct_aoff.size(); ++c) {
-      for (int m = 0; m < ct_nm[c]; ++m) hAc[c * F + m] = A_all[ct_aoff[c] + m];
-      full32 = full32 && ct_nm[c] == F && ct_M[c] % 4 == 0;
-      full64 = full64 && ct_nm[c] == F && ct_M[c] % 2 == 0;
+  // entries of the tensor-core path, in the order of their sub-tiles
+  std::vector<int2> st_sub, st_M, sg_e;
+  std::vector<int> st_eoff, sg_off;
+  std::vector<double> st_A;
+  if (l->maxnm <= 16 && nW > 0) {
+    l->nf = l->maxnm <= 8 ? 1 : 2;
+    const int nblk = l->nf * 64, ngr = (int)gr_M.size();
+    std::vector<int> vol_group(nW);
+    for (int gi = 0; gi < ngr; ++gi)
+      for (int v = gr_voff[gi]; v < gr_voff[gi + 1]; ++v) vol_group[gv_W[v]] = gi;
+    struct Ent { int sub, W; int64_t r0, r1; };          // rows of W in the sub-tile
+    std::vector<Ent> ents;
+    for (int W = 0; W < nW; ++W)
+      for (int64_t r = row0[W]; r < row0[W + 1]; ++r) {
+        const int sub = row_G[r] / 8;
+        if (r == row0[W] || sub != ents.back().sub) ents.push_back({sub, W, r, r});
+        ents.back().r1 = r + 1;
+      }
+    std::sort(ents.begin(), ents.end(),
+              [](const Ent& x, const Ent& y) { return x.sub != y.sub ? x.sub < y.sub : x.W < y.W; });
+    st_A.assign(ents.size() * (size_t)nblk, 0.0);
+    std::vector<std::vector<int2>> by_group(ngr);
+    for (size_t e = 0; e < ents.size(); ++e) {
+      const Ent& n = ents[e];
+      if (st_sub.empty() || st_sub.back().x != n.sub) {
+        st_sub.push_back(make_int2(n.sub, 0));
+        st_eoff.push_back((int)e);
+      }
+      const int nm = nm_W[n.W];
+      st_M.push_back(make_int2(M_W[n.W], nm));
+      by_group[vol_group[n.W]].push_back(make_int2((int)e, n.sub));
+      double* blk = st_A.data() + e * (size_t)nblk;
+      for (int64_t r = n.r0; r < n.r1; ++r) {
+        const int p = row_G[r] % 8;
+        st_sub.back().y |= 1 << p;
+        const double* Ar = A_all + aoff[n.W] + (r - row0[n.W]) * nm;
+        for (int m = 0; m < nm; ++m) blk[m * 8 + p] = Ar[m];
+      }
     }
-    l->full32 = full32;
-    l->full64 = full64;
+    st_eoff.push_back((int)ents.size());
+    sg_off.push_back(0);
+    for (int gi = 0; gi < ngr; ++gi) {
+      sg_e.insert(sg_e.end(), by_group[gi].begin(), by_group[gi].end());
+      sg_off.push_back((int)sg_e.size());
+    }
+    l->ns = (int)st_sub.size();
   }
   // brick tiling for the FP32 real path
   std::vector<int> tch_c, tch_eoff, te_nm, te_slot, te_lst, te_info, tbr_ch0, tbr_pbase, tps_M, tps_nm, tps_eoff,
@@ -1330,18 +1445,9 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
       ok = cudaDeviceSynchronize() == cudaSuccess;
     }
   }
-  if (ok && l->fast_nmax) {
-    ok = upload(l, &l->Ac64, hAc);
-    if (ok) {
-      l->Ac32 = dalloc<float>(l, hAc.size());
-      ok = l->Ac32 != nullptr;
-    }
-    if (ok && !hAc.empty()) {
-      to_float<<<std::min<int64_t>(((int64_t)hAc.size() + 255) / 256, 4096), 256>>>(l->Ac64, l->Ac32,
-                                                                                      (int64_t)hAc.size());
-      ok = cudaDeviceSynchronize() == cudaSuccess;
-    }
-  }
+  if (ok && l->nf)
+    ok = upload(l, &l->st_sub, st_sub) && upload(l, &l->st_eoff, st_eoff) && upload(l, &l->st_M, st_M) &&
+         upload(l, &l->st_A, st_A) && upload(l, &l->sg_off, sg_off) && upload(l, &l->sg_e, sg_e);
   if (ok && tiled) {
     ok = upload(l, &l->tch_c, tch_c) && upload(l, &l->tch_eoff, tch_eoff) && upload(l, &l->te_info, te_info) &&
          upload(l, &l->te_A, te_A) && upload(l, &l->tbr_ch0, tbr_ch0) && upload(l, &l->tbr_pbase, tbr_pbase) &&
