@@ -436,7 +436,7 @@ static int launch_box(const gb_operator* op, const void* in, void* out, int64_t 
                       const double* phase_cd, cudaStream_t stream, const Epilogue& ep, int nk) {
   BoxArgs a;
   fill_box_args(op, a, phase_cd, nk, nin);
-  a.alpha = ep.alpha; a.beta = ep.beta; a.gamma = ep.gamma; a.y = ep.y;
+  a.alpha = ep.alpha; a.beta = ep.beta; a.gamma = ep.gamma; a.y = ep.y; a.vpot = ep.vpot;
   a.in = in; a.out = out; a.nbatch = nin;
   a.b0 = 4; a.b1 = 8; a.b2 = 32;
   const int M = a.M;

@@ -175,3 +175,21 @@ def test_lfc_tensor_cores(nx, ls, dtype):
     one = a[k:].clone()
     lfc.add_M(one, c[k:].contiguous())
     assert torch.equal(one, b[k:])
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+def test_potential_of_a_skew_cell(dtype):
+    """The potential joins stencils with points off the axes as it does the others."""
+    from gpaw_b200.fd_operators import Laplace
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor((12, 10, 14), [[4.0, 0, 0], [1.5, 4.0, 0], [0.5, 0.7, 4.5]], True)
+    lap = Laplace(gd, -0.5, 2)
+    assert not lap.cfd
+    g = torch.Generator(device='cuda').manual_seed(7)
+    x = torch.randn((3,) + tuple(gd.n_c), generator=g, device='cuda', dtype=dtype)
+    v = torch.randn(tuple(gd.n_c), generator=g, device='cuda', dtype=dtype)
+    y = torch.empty_like(x)
+    lap.apply_potential(x, y, v)
+    h = x.cpu().numpy().astype(np.float64)
+    ref = fd.fd_apply(lap.coef_p, lap.offset_pc, h, (1, 1, 1)) + v.cpu().numpy().astype(np.float64) * h
+    assert relerr(y.cpu().numpy(), ref) < TOL[dtype]
