@@ -83,6 +83,7 @@ struct gb_lfc {
   int tbr_n = 0;              // bricks
   int tbr_smax = 1;           // most slots in a brick
   int tbr_emax = 0;           // most entries in a brick
+  int tnm = 0;                // functions of every group, 0: they differ
   int* tbr_ch0 = nullptr;     // [tbr_n + 1] chunk range of each brick
   int* tbr_pbase = nullptr;   // [tbr_n + 1] first (brick, slot) pair
   int64_t tpart_n = 0;        // (brick, slot) pairs
@@ -680,27 +681,37 @@ static int add_nm(const gb_lfc* l, const void* c, void* a, int64_t nx, int q, cu
 // there as a dense [m][p] 8 x 8 block.  A brick is a run of at most TBRICK
 // consecutive chunks with entries that meets at most TSLOTS function groups
 // (its slots) and holds at most TBENT entries.  One CTA takes one (brick,
-// group of 32 bands) and first copies into shared memory, with coalesced
-// 16-byte cp.async copies, the brick's rows of a (a band row pitch of
-// 32 TBRICK + 4 floats, so that lanes reading one band each do not collide
-// on banks), its entries' blocks and, for the add, the coefficients of its
-// slots as [slot][m][band] (rows of cT, c transposed by a first kernel).
-// Every operand of the FMAs then comes from shared memory.
-//  add:        warp w updates sub-tiles w, w + 8, ... in place (one owner per
-//              sub-tile): a[x][p] += sum_e sum_m A_e[m][p] c[x][M_e + m];
+// group of bands: 32 for the add, 64 for the integral) and first copies into
+// shared memory, with coalesced 16-byte cp.async copies, the brick's rows of
+// a (a band row pitch of 32 TBRICK + 4 floats, free of bank conflicts), its
+// entries' blocks and, for the add, the coefficients of its slots as
+// [slot][m][band] (rows of cT, c transposed by a first kernel).  A warp works
+// on 8 points x 32 bands: lane (q, b) holds points 4 q .. 4 q + 3 of bands b
+// and b + 16, so that one 16-byte read of a block's row -- two addresses in
+// the warp -- feeds both, and cT holds such pairs side by side.
+//  add:        warp w updates sub-tiles w, w + 16, ... in place (one owner
+//              per sub-tile): a[x][p] += sum_e sum_m A_e[m][p] c[x][M_e + m];
 //              the brick's rows are then written back.
-//  integrate:  warp s sums slot s over its entries (lists made on the host)
-//              and writes one partial sum per (brick, slot, band); a second
-//              kernel adds dv times each group's partials, in brick order,
-//              to c.
+//  integrate:  a warp sums one slot and 32 bands over its entries (lists made
+//              on the host) and writes one partial sum per (brick, slot,
+//              band); a second kernel adds dv times each group's partials, in
+//              brick order, to c.
 // No atomics: the results do not depend on scheduling.
+// Bound by shared-memory wavefronts and the wait for the copies: (160, 56^3),
+// 64 atoms with 5 functions: add 133 -> 109 us, integrate 117 -> 95 us against
+// lanes owning one band and all 8 points (three wavefronts per block row and
+// 32 bands instead of two in the add, 18 instead of 13 per entry in the
+// integral, and twice the instructions).  Adding to a directly in global
+// memory, 64 bands per CTA, took 122 us: 16 rows per store instruction.  Half
+// as long bricks, 8-warp CTAs: add 118, integrate 102 us.
 constexpr int TCH = 32;                    // points per chunk
 constexpr int TSLOTS = 16;                 // function groups per brick
 constexpr int TBRICK = 8;                  // chunks per brick
-constexpr int TBENT = 192;                 // entries per brick
-constexpr int TBAND = 32;                  // bands per CTA
+constexpr int TBENT = 176;                 // entries per brick (two integrate CTAs per SM)
+constexpr int TADD_BAND = 32;              // bands per CTA, add
+constexpr int TINT_BAND = 64;              // and integrate
 constexpr int TPITCH = TBRICK * TCH + 4;   // floats per band row in shared memory
-constexpr int TADD_WARPS = 16;
+constexpr int TILE_WARPS = 16;
 
 struct TileView {
   const int* ch_c;      // [nch] chunk index (first point 32 c) of every used chunk
@@ -720,40 +731,30 @@ static TileView tile_view(const gb_lfc* l) {
                   l->tps_M, l->tps_nm, l->tps_eoff, l->tps_info};
 }
 
-// shared-memory copy of brick b for bands x0 .. x0 + nb - 1 (of the rows at a)
-__device__ __forceinline__ void brick_stage(const TileView& t, int b, const float* __restrict__ a, int64_t nG,
-                                            int x0, int nb, float* sa, float* sA, float* sc,
-                                            const float* __restrict__ cT, int ldT) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int k0 = t.br_ch0[b], nk = t.br_ch0[b + 1] - k0;
-  for (int x = warp; x < nb; x += nw) {
-    const float* src = a + (int64_t)(x0 + x) * nG;
-    for (int i = lane; i < nk * 8; i += 32) {
-      const int kk = i >> 3, q = i & 7;
-      const int64_t G = (int64_t)t.ch_c[k0 + kk] * TCH + 4 * q;
-      float* d = sa + x * TPITCH + kk * TCH + 4 * q;
-      if (G < nG) cp_async16(d, src + G);
-      else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  const int E0 = t.ch_eoff[4 * k0], E1 = t.ch_eoff[4 * (k0 + nk)];
+// the blocks of entries E0 .. E1 - 1
+__device__ __forceinline__ void stage_blocks(const TileView& t, int E0, int E1, float* sA) {
   for (int i = threadIdx.x; i < (E1 - E0) * 16; i += blockDim.x) cp_async16(sA + 4 * i, t.e_A + (int64_t)E0 * 64 + 4 * i);
-  if (sc) {
-    const int pbase = t.br_pbase[b], S = t.br_pbase[b + 1] - pbase;
-    for (int r = warp; r < S * 8; r += nw) {
-      const int s = r >> 3, m = r & 7;
-      if (lane < 8) {
-        float* d = sc + r * TBAND + 4 * lane;
-        if (m < t.ps_nm[pbase + s]) cp_async16(d, cT + (int64_t)(t.ps_M[pbase + s] + m) * ldT + x0 + 4 * lane);
-        else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
 }
 
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// f(integral_constant<int, nm>) for 1 <= nm <= 8, uniform in a warp
+template <class F>
+__device__ __forceinline__ void for_functions(int nm, F&& f) {
+  switch (nm) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+  }
+}
+
+// cT[M][x0 + 2 b + i] = c[x0 + b + 16 i][M]
 __global__ void lfc_coef_transpose_kernel(const float* __restrict__ c, int nM, int R, int ldT, float* __restrict__ cT) {
   __shared__ float tile[32][33];
   const int M0 = blockIdx.x * 32, x0 = blockIdx.y * 32;
@@ -764,116 +765,167 @@ __global__ void lfc_coef_transpose_kernel(const float* __restrict__ c, int nM, i
   __syncthreads();
   for (int i = threadIdx.y; i < 32; i += 8) {
     const int M = M0 + i;
-    if (M < nM) cT[(int64_t)M * ldT + x0 + threadIdx.x] = tile[threadIdx.x][i];
+    if (M < nM) cT[(int64_t)M * ldT + x0 + threadIdx.x] = tile[16 * (threadIdx.x & 1) + (threadIdx.x >> 1)][i];
   }
 }
 
-// acc (points 2k, 2k+1 in acc[k]) += A row m (4 float2) * cv
-__device__ __forceinline__ void add_row(float2 (&acc)[4], const float4* __restrict__ Ab, int m, float cv) {
-  const float4 A0 = Ab[2 * m], A1 = Ab[2 * m + 1];
-  const float2 c2 = make_float2(cv, cv);
-  acc[0] = __ffma2_rn(make_float2(A0.x, A0.y), c2, acc[0]);
-  acc[1] = __ffma2_rn(make_float2(A0.z, A0.w), c2, acc[1]);
-  acc[2] = __ffma2_rn(make_float2(A1.x, A1.y), c2, acc[2]);
-  acc[3] = __ffma2_rn(make_float2(A1.z, A1.w), c2, acc[3]);
+// rows x0 .. x0 + nb - 1 of a brick's chunks
+__device__ __forceinline__ void stage_rows(const TileView& t, int k0, int nk, const float* __restrict__ a, int64_t nG,
+                                           int x0, int nb, float* sa) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int x = warp; x < nb; x += TILE_WARPS) {
+    const float* src = a + (int64_t)(x0 + x) * nG;
+    for (int i = lane; i < nk * 8; i += 32) {
+      const int64_t G = (int64_t)t.ch_c[k0 + (i >> 3)] * TCH + 4 * (i & 7);
+      float* d = sa + x * TPITCH + 4 * i;
+      if (G < nG) cp_async16(d, src + G);
+      else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
 }
 
-__global__ void __launch_bounds__(32 * TADD_WARPS) lfc_add_tiles_kernel(const TileView t, const float* __restrict__ cT,
-                                                                       int ldT, float* __restrict__ a, int64_t nG,
-                                                                       int R, int sA_floats) {
-  extern __shared__ __align__(16) float tsm[];
-  float* sa = tsm;
-  float* sA = sa + TBAND * TPITCH;
-  float* sc = sA + sA_floats;
-  const int b = blockIdx.x, x0 = blockIdx.y * TBAND;
-  const int nb = min(TBAND, R - x0);
-  brick_stage(t, b, a, nG, x0, nb, sa, sA, sc, cT, ldT);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k0 = t.br_ch0[b], nk = t.br_ch0[b + 1] - k0;
+// acc (points 2 k, 2 k + 1 of band i in acc[i][k]) += nm rows of a block
+template <int NM>
+__device__ __forceinline__ void add_entry(float2 (&acc)[2][2], const float4* __restrict__ Ab,
+                                          const float* __restrict__ cs) {
+#pragma unroll
+  for (int m = 0; m < NM; ++m) {
+    const float4 A = Ab[2 * m];
+    const float2 c = *reinterpret_cast<const float2*>(cs + m * TADD_BAND);
+    const float2 c0 = make_float2(c.x, c.x), c1 = make_float2(c.y, c.y);
+    acc[0][0] = __ffma2_rn(lo2(A), c0, acc[0][0]);
+    acc[0][1] = __ffma2_rn(hi2(A), c0, acc[0][1]);
+    acc[1][0] = __ffma2_rn(lo2(A), c1, acc[1][0]);
+    acc[1][1] = __ffma2_rn(hi2(A), c1, acc[1][1]);
+  }
+}
+
+// the sub-tiles of a brick; NM: functions of every entry, 0: each entry's own
+template <int NM>
+__device__ __forceinline__ void add_sub_tiles(const TileView& t, int k0, int nk, const float* sA, const float* sc,
+                                              float* sa) {
+  const int warp = threadIdx.x >> 5, q = (threadIdx.x >> 4) & 1, b = threadIdx.x & 15;
   const int E0 = t.ch_eoff[4 * k0];
-  for (int st = warp; st < 4 * nk; st += TADD_WARPS) {
+  for (int st = warp; st < 4 * nk; st += TILE_WARPS) {
     const int e0 = t.ch_eoff[4 * k0 + st], e1 = t.ch_eoff[4 * k0 + st + 1];
     if (e0 == e1) continue;
-    float* row = sa + lane * TPITCH + 8 * st;
-    const float4 u = *reinterpret_cast<const float4*>(row), v = *reinterpret_cast<const float4*>(row + 4);
-    float2 acc[4] = {make_float2(u.x, u.y), make_float2(u.z, u.w), make_float2(v.x, v.y), make_float2(v.z, v.w)};
+    float4* row = reinterpret_cast<float4*>(sa + b * TPITCH + 8 * st + 4 * q);
+    float2 acc[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 u = row[4 * TPITCH * i];
+      acc[i][0] = lo2(u);
+      acc[i][1] = hi2(u);
+    }
     int info = t.e_info[e0];
     for (int e = e0; e < e1; ++e) {
+      const float4* Ab = reinterpret_cast<const float4*>(sA + (e - E0) * 64) + q;
+      const float* cs = sc + (info & 255) * 8 * TADD_BAND + 2 * b;
       const int nm = info >> 8;
-      const float4* Ab = reinterpret_cast<const float4*>(sA + (e - E0) * 64);
-      const float* cs = sc + (info & 255) * 8 * TBAND + lane;
       if (e + 1 < e1) info = t.e_info[e + 1];
-      if (nm == 8) {
+      if constexpr (NM > 0) add_entry<NM>(acc, Ab, cs);
+      else for_functions(nm, [&](auto n) { add_entry<n.value>(acc, Ab, cs); });
+    }
 #pragma unroll
-        for (int m = 0; m < 8; ++m) add_row(acc, Ab, m, cs[m * TBAND]);
-      } else {
-        for (int m = 0; m < nm; ++m) add_row(acc, Ab, m, cs[m * TBAND]);
-      }
-    }
-    *reinterpret_cast<float4*>(row) = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
-    *reinterpret_cast<float4*>(row + 4) = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
-  }
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  for (int x = warp; x < nb; x += nw) {
-    float* dst = a + (int64_t)(x0 + x) * nG;
-    for (int i = lane; i < nk * 8; i += 32) {
-      const int kk = i >> 3, q = i & 7;
-      const int64_t G = (int64_t)t.ch_c[k0 + kk] * TCH + 4 * q;
-      if (G < nG)
-        *reinterpret_cast<float4*>(dst + G) = *reinterpret_cast<const float4*>(sa + x * TPITCH + kk * TCH + 4 * q);
-    }
+    for (int i = 0; i < 2; ++i) row[4 * TPITCH * i] = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
   }
 }
 
-// acc[m] (even / odd point sums) += A row m . av
-__device__ __forceinline__ void int_row(float2 (&acc)[8], const float4* __restrict__ Ab, int m, const float2 (&av)[4]) {
-  const float4 A0 = Ab[2 * m], A1 = Ab[2 * m + 1];
-  float2 s = acc[m];
-  s = __ffma2_rn(make_float2(A0.x, A0.y), av[0], s);
-  s = __ffma2_rn(make_float2(A0.z, A0.w), av[1], s);
-  s = __ffma2_rn(make_float2(A1.x, A1.y), av[2], s);
-  s = __ffma2_rn(make_float2(A1.z, A1.w), av[3], s);
-  acc[m] = s;
-}
-
-__global__ void __launch_bounds__(32 * TSLOTS) lfc_integrate_tiles_kernel(const TileView t,
-                                                                         const float* __restrict__ a, int64_t nG,
-                                                                         int R, float* __restrict__ part) {
+__global__ void __launch_bounds__(32 * TILE_WARPS, 2) lfc_add_tiles_kernel(const TileView t,
+                                                                         const float* __restrict__ cT, int ldT,
+                                                                         float* __restrict__ a, int64_t nG, int R,
+                                                                         int sA_floats, int nm_all) {
   extern __shared__ __align__(16) float tsm[];
   float* sa = tsm;
-  float* sA = sa + TBAND * TPITCH;
-  const int b = blockIdx.x, x0 = blockIdx.y * TBAND;
-  const int nb = min(TBAND, R - x0);
-  brick_stage(t, b, a, nG, x0, nb, sa, sA, nullptr, nullptr, 0);
+  float* sA = sa + TADD_BAND * TPITCH;
+  float* sc = sA + sA_floats;
+  const int b = blockIdx.x, x0 = blockIdx.y * TADD_BAND;
+  const int nb = min(TADD_BAND, R - x0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k0 = t.br_ch0[b], nk = t.br_ch0[b + 1] - k0;
+  stage_rows(t, k0, nk, a, nG, x0, nb, sa);
+  stage_blocks(t, t.ch_eoff[4 * k0], t.ch_eoff[4 * (k0 + nk)], sA);
   const int pbase = t.br_pbase[b], S = t.br_pbase[b + 1] - pbase;
-  if (warp >= S) return;
-  float2 acc[8];
-#pragma unroll
-  for (int m = 0; m < 8; ++m) acc[m] = make_float2(0.f, 0.f);
-  const int q0 = t.ps_eoff[pbase + warp], q1 = t.ps_eoff[pbase + warp + 1];
-  int info = q0 < q1 ? t.ps_info[q0] : 0;
-  for (int q = q0; q < q1; ++q) {
-    const int el = info & 0xffff, lst = (info >> 16) & 255, nm = info >> 24;
-    if (q + 1 < q1) info = t.ps_info[q + 1];
-    const float* row = sa + lane * TPITCH + 8 * lst;
-    const float4 u = *reinterpret_cast<const float4*>(row), v = *reinterpret_cast<const float4*>(row + 4);
-    const float2 av[4] = {make_float2(u.x, u.y), make_float2(u.z, u.w), make_float2(v.x, v.y), make_float2(v.z, v.w)};
-    const float4* Ab = reinterpret_cast<const float4*>(sA + el * 64);
-    if (nm == 8) {
-#pragma unroll
-      for (int m = 0; m < 8; ++m) int_row(acc, Ab, m, av);
-    } else {
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-        if (m < nm) int_row(acc, Ab, m, av);
+  for (int r = 4 * warp + (lane >> 3); r < S * 8; r += 4 * TILE_WARPS) {
+    const int s = r >> 3, m = r & 7, x = 4 * (lane & 7);
+    if (m < t.ps_nm[pbase + s])
+      cp_async16(sc + r * TADD_BAND + x, cT + (int64_t)(t.ps_M[pbase + s] + m) * ldT + x0 + x);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (nm_all) for_functions(nm_all, [&](auto n) { add_sub_tiles<n.value>(t, k0, nk, sA, sc, sa); });
+  else add_sub_tiles<0>(t, k0, nk, sA, sc, sa);
+  __syncthreads();
+  for (int x = warp; x < nb; x += TILE_WARPS) {
+    float* dst = a + (int64_t)(x0 + x) * nG;
+    for (int i = lane; i < nk * 8; i += 32) {
+      const int64_t G = (int64_t)t.ch_c[k0 + (i >> 3)] * TCH + 4 * (i & 7);
+      if (G < nG) *reinterpret_cast<float4*>(dst + G) = *reinterpret_cast<const float4*>(sa + x * TPITCH + 4 * i);
     }
   }
-  if (lane < nb) {
-    float4* d = reinterpret_cast<float4*>(part + ((int64_t)(pbase + warp) * R + x0 + lane) * 8);
-    d[0] = make_float4(acc[0].x + acc[0].y, acc[1].x + acc[1].y, acc[2].x + acc[2].y, acc[3].x + acc[3].y);
-    d[1] = make_float4(acc[4].x + acc[4].y, acc[5].x + acc[5].y, acc[6].x + acc[6].y, acc[7].x + acc[7].y);
+}
+
+// acc[i][m] (even / odd point sums of band i) over entries q0 .. q1 - 1 of a
+// slot of NM functions
+template <int NM>
+__device__ __forceinline__ void integrate_entries(float2 (&acc)[2][8], const int* __restrict__ ps_info, int q0, int q1,
+                                                  const float* __restrict__ row, const float* __restrict__ sA) {
+  constexpr int U = NM <= 6 ? 2 : 1;       // entries in flight, within 64 registers
+#pragma unroll U
+  for (int e = q0; e < q1; ++e) {
+    const int info = __ldg(ps_info + e);
+    const float* r = row + 8 * ((info >> 16) & 255);
+    const float4 u = *reinterpret_cast<const float4*>(r), v = *reinterpret_cast<const float4*>(r + 16 * TPITCH);
+    const float4* Ab = reinterpret_cast<const float4*>(sA + (info & 0xffff) * 64);
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+      const float4 A = Ab[2 * m];
+      acc[0][m] = __ffma2_rn(hi2(A), hi2(u), __ffma2_rn(lo2(A), lo2(u), acc[0][m]));
+      acc[1][m] = __ffma2_rn(hi2(A), hi2(v), __ffma2_rn(lo2(A), lo2(v), acc[1][m]));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32 * TILE_WARPS, 2) lfc_integrate_tiles_kernel(const TileView t,
+                                                                               const float* __restrict__ a,
+                                                                               int64_t nG, int R,
+                                                                               float* __restrict__ part) {
+  extern __shared__ __align__(16) float tsm[];
+  float* sa = tsm;
+  float* sA = sa + TINT_BAND * TPITCH;
+  const int br = blockIdx.x, x0 = blockIdx.y * TINT_BAND;
+  const int nb = min(TINT_BAND, R - x0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 4, b = lane & 15;
+  const int k0 = t.br_ch0[br], nk = t.br_ch0[br + 1] - k0;
+  stage_rows(t, k0, nk, a, nG, x0, nb, sa);
+  stage_blocks(t, t.ch_eoff[4 * k0], t.ch_eoff[4 * (k0 + nk)], sA);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int pbase = t.br_pbase[br], S = t.br_pbase[br + 1] - pbase, H = nb > 32 ? 2 : 1;
+  for (int it = warp; it < S * H; it += TILE_WARPS) {
+    const int s = it / H, xb = (it - s * H) * 32 + b;      // bands xb and xb + 16 of the group
+    float2 acc[2][8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) acc[0][m] = acc[1][m] = make_float2(0.f, 0.f);
+    const int q0 = t.ps_eoff[pbase + s], q1 = t.ps_eoff[pbase + s + 1];
+    for_functions(t.ps_nm[pbase + s], [&](auto n) {
+      integrate_entries<n.value>(acc, t.ps_info, q0, q1, sa + xb * TPITCH + 4 * q, sA + 4 * q);
+    });
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float r[8];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        r[m] = acc[i][m].x + acc[i][m].y;
+        r[m] += __shfl_xor_sync(0xffffffffu, r[m], 16);
+      }
+      // lane half q writes functions 4 q .. 4 q + 3
+      if (xb + 16 * i < nb)
+        reinterpret_cast<float4*>(part + ((int64_t)(pbase + s) * R + x0 + xb + 16 * i) * 8)[q] =
+            q ? make_float4(r[4], r[5], r[6], r[7]) : make_float4(r[0], r[1], r[2], r[3]);
+    }
   }
 }
 
@@ -937,9 +989,10 @@ static int tile_work(const gb_lfc* l, size_t bytes, cudaStream_t st) {
 static int tile_smem_attr() {
   static int done = 0;
   if (!done) {
-    const int mx = (TBAND * TPITCH + TBENT * 64 + TSLOTS * 8 * TBAND) * (int)sizeof(float);
-    if (cudaFuncSetAttribute(lfc_add_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) != cudaSuccess ||
-        cudaFuncSetAttribute(lfc_integrate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) !=
+    const int mxa = (TADD_BAND * TPITCH + TBENT * 64 + TSLOTS * 8 * TADD_BAND) * (int)sizeof(float);
+    const int mxi = (TINT_BAND * TPITCH + TBENT * 64) * (int)sizeof(float);
+    if (cudaFuncSetAttribute(lfc_add_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mxa) != cudaSuccess ||
+        cudaFuncSetAttribute(lfc_integrate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mxi) !=
             cudaSuccess)
       return check_launch("lfc tiled shared memory");
     done = 1;
@@ -962,15 +1015,15 @@ static int add_tiles(const gb_lfc* l, const float* c, float* a, int64_t nx, cuda
   if (rc) return rc;
   float* cT = static_cast<float*>(l->work);
   const int sA_floats = l->tbr_emax * 64;
-  const int smem = (TBAND * TPITCH + sA_floats + TSLOTS * 8 * TBAND) * (int)sizeof(float);
+  const int smem = (TADD_BAND * TPITCH + sA_floats + l->tbr_smax * 8 * TADD_BAND) * (int)sizeof(float);
   for (int64_t x0 = 0; x0 < nx; x0 += 256) {
     const int R = (int)std::min<int64_t>(nx - x0, 256);
     const int ldT = (R + 31) / 32 * 32;
     dim3 tg((unsigned)((l->nM + 31) / 32), (unsigned)(ldT / 32));
     lfc_coef_transpose_kernel<<<tg, dim3(32, 8), 0, st>>>(c + x0 * l->nM, l->nM, R, ldT, cT);
-    dim3 grid((unsigned)l->tbr_n, (unsigned)(ldT / TBAND));
-    lfc_add_tiles_kernel<<<grid, 32 * TADD_WARPS, smem, st>>>(tile_view(l), cT, ldT, a + x0 * l->nG, l->nG, R,
-                                                              sA_floats);
+    dim3 grid((unsigned)l->tbr_n, (unsigned)(ldT / TADD_BAND));
+    lfc_add_tiles_kernel<<<grid, 32 * TILE_WARPS, smem, st>>>(tile_view(l), cT, ldT, a + x0 * l->nG, l->nG, R,
+                                                              sA_floats, l->tnm);
     rc = check_launch("lfc_add_tiles_kernel");
     if (rc) return rc;
   }
@@ -985,11 +1038,11 @@ static int integrate_tiles(const gb_lfc* l, const float* a, float* c, int64_t nx
   rc = tile_work(l, (size_t)l->tpart_n * Rmax * 8 * sizeof(float), st);
   if (rc) return rc;
   float* part = static_cast<float*>(l->work);
-  const int smem = (TBAND * TPITCH + l->tbr_emax * 64) * (int)sizeof(float);
+  const int smem = (TINT_BAND * TPITCH + l->tbr_emax * 64) * (int)sizeof(float);
   for (int64_t x0 = 0; x0 < nx; x0 += 256) {
     const int R = (int)std::min<int64_t>(nx - x0, 256);
-    dim3 grid((unsigned)l->tbr_n, (unsigned)((R + TBAND - 1) / TBAND));
-    lfc_integrate_tiles_kernel<<<grid, 32 * l->tbr_smax, smem, st>>>(tile_view(l), a + x0 * l->nG, l->nG, R, part);
+    dim3 grid((unsigned)l->tbr_n, (unsigned)((R + TINT_BAND - 1) / TINT_BAND));
+    lfc_integrate_tiles_kernel<<<grid, 32 * TILE_WARPS, smem, st>>>(tile_view(l), a + x0 * l->nG, l->nG, R, part);
     rc = check_launch("lfc_integrate_tiles_kernel");
     if (rc) return rc;
     dim3 rg((unsigned)((R * 8 + 31) / 32), (unsigned)l->ngroups);
@@ -1458,6 +1511,7 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     l->tbr_n = (int)tbr_ch0.size() - 1;
     l->tbr_smax = tbr_smax;
     l->tbr_emax = tbr_emax;
+    l->tnm = std::all_of(gr_nm.begin(), gr_nm.end(), [&](int n) { return n == gr_nm[0]; }) ? gr_nm[0] : 0;
     l->tpart_n = tbr_pbase.back();
   }
   if (!ok) {

@@ -9,8 +9,9 @@
 
 namespace gb {
 
-constexpr int WAIT_HINT_NS = 20000;     // longest time one poll may sleep
-constexpr int WAIT_LIMIT = 1 << 20;     // polls: a tenth of a second if none sleeps, 20 s if all do
+constexpr long long WAIT_LIMIT = 1LL << 25;   // ~ seconds of polling
+constexpr int WAIT_HINT_NS = 20000;           // longest time a poll with a hint may sleep
+constexpr int WAIT_LIMIT_HINT = 1 << 20;      // such polls: 20 s if all sleep that long
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((uint32_t)__cvta_generic_to_shared(bar)),
@@ -52,7 +53,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // marching stencil took 7 of its 94 issue slots per 32 points.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = (uint32_t)__cvta_generic_to_shared(bar);
-  for (int i = 0; i < WAIT_LIMIT; ++i) {
+  for (int i = 0; i < WAIT_LIMIT_HINT; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n"
