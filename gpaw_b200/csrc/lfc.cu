@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(NT) lfc_integrate_kernel(const LfcView l, cons
 // A non-finite value at an uncovered point (integrate) or in the coefficients
 // of another volume (add) can reach the sums of its own sub-tile.
 //
-// Bound by L1 requests (a fragment load touches eight rows).  71^3 grid, 24
+// Bound by the latency of gathered operands; fewer bands per warp is slower
+// all the same (integrate 114 us with 32 bands, 135 with 16).  71^3 grid, 24
 // atoms x 9 functions of radius 2.5 A, 96 FP64 bands: integrate 189 -> 84 us,
 // add 196 -> 140 us against the point-major kernels (gathered rows, one point
 // per thread).  FP32 with at most eight functions keeps the brick tiling
