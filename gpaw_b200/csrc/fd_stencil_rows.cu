@@ -15,11 +15,12 @@
 // the centre plane.  Ring: H + 1 planes in use and two on their way, one
 // barrier per plane (deeper rings measured the same).
 //
-// Bound by issue slots, 107 per 32 points in FP64 (the
-// 32 x 32 tiles it replaces spent most of theirs on addresses, boundaries and
-// the unused part of edge tiles): (160, 75^3) FP64 zero boundary 1080 -> 433 us
-// (2.5 TB/s), with a potential 1680 -> 506 us; FP32 768 -> 305 us;
-// (64, 60^3) complex128 with phases 597 -> 225 us.
+// Bound by issue slots, 107 per 32 points in FP64, and by instruction fetch
+// (the 32 x 32 tiles it replaces spent most of theirs on addresses, boundaries
+// and the unused part of edge tiles): (160, 75^3) FP64 zero boundary 1080 ->
+// 433 us (2.5 TB/s), with a potential 1680 -> 506 us; FP32 768 -> 305 us;
+// (64, 60^3) complex128 with phases 597 -> 225 us, all before the compute part
+// alone was unrolled.
 #include <algorithm>
 #include <cstring>
 #include "star_core.cuh"
@@ -160,55 +161,57 @@ __global__ void __launch_bounds__(ROWS_NT, 2) rows_star_kernel(const __grid_cons
     }
     T q[NQ][R1][R2];
     int slot = 0;
-    for (int jb = j0; jb < j1; jb += NQ) {
-#pragma unroll
-      for (int u = 0; u < NQ; ++u) {
-        const int j = jb + u;
-        if (j < j1) {
-        cp_async_wait<D - 1>();
-        __syncthreads();
-        // the slot refilled here was last read as the centre plane of step j - 1
-        {
-          int ns = slot + D;
-          if (ns >= NS) ns -= NS;
-          if (j + D < j1) issue(j + D, ns);
-          cp_async_commit();
-        }
-        if (phased) {
-          // Bloch phases of the wrapped cells of the plane that just landed:
-          // they are read when it is the centre plane, H barriers from here
-          T* L = slots + slot * slot_elems;
-          const int ncol = a.pbc2 ? 2 * H * a.T1 : 0;
-          const int top = a.pbc1 ? max(0, H - y0) : 0;                    // wrapped rows above the grid
-          const int nrow = a.pbc1 ? top + max(0, rows - (n1 + H - y0)) : 0;
-          for (int e = tid; e < ncol + nrow * n2; e += blockDim.x) {
-            int off, ax, sd;
-            if (e < ncol) {
-              const int r = e / (2 * H), k = e - r * (2 * H);
-              ax = 2;
-              sd = k < H ? 1 : 0;
-              off = (H + r) * pitch + HZ + (k < H ? k - H : n2 + k - H);
-            } else {
-              const int r = (e - ncol) / n2, c = (e - ncol) - r * n2;
-              ax = 1;
-              sd = r < top ? 1 : 0;
-              off = (r < top ? r : n1 + H - y0 + (r - top)) * pitch + HZ + c;
-            }
-            L[off] = phase_mul(L[off], PH[ax][sd][0], PH[ax][sd][1]);
+    int turn = 0;
+    for (int j = j0; j < j1; ++j) {
+      cp_async_wait<D - 1>();
+      __syncthreads();
+      // the slot refilled here was last read as the centre plane of step j - 1
+      {
+        int ns = slot + D;
+        if (ns >= NS) ns -= NS;
+        if (j + D < j1) issue(j + D, ns);
+        cp_async_commit();
+      }
+      if (phased) {
+        // Bloch phases of the wrapped cells of the plane that just landed:
+        // they are read when it is the centre plane, H barriers from here
+        T* L = slots + slot * slot_elems;
+        const int ncol = a.pbc2 ? 2 * H * a.T1 : 0;
+        const int top = a.pbc1 ? max(0, H - y0) : 0;                    // wrapped rows above the grid
+        const int nrow = a.pbc1 ? top + max(0, rows - (n1 + H - y0)) : 0;
+        for (int e = tid; e < ncol + nrow * n2; e += blockDim.x) {
+          int off, ax, sd;
+          if (e < ncol) {
+            const int r = e / (2 * H), k = e - r * (2 * H);
+            ax = 2;
+            sd = k < H ? 1 : 0;
+            off = (H + r) * pitch + HZ + (k < H ? k - H : n2 + k - H);
+          } else {
+            const int r = (e - ncol) / n2, c = (e - ncol) - r * n2;
+            ax = 1;
+            sd = r < top ? 1 : 0;
+            off = (r < top ? r : n1 + H - y0 + (r - top)) * pitch + HZ + c;
           }
+          L[off] = phase_mul(L[off], PH[ax][sd][0], PH[ax][sd][1]);
         }
-        const int cpl = j - H;
-        T yv[R1][R2];
-        R vv[R1][R2];
-        if (EPI && cpl >= p_start) {
+      }
+      const int cpl = j - H;
+      T yv[R1][R2];
+      R vv[R1][R2];
+      if (EPI && cpl >= p_start) {
 #pragma unroll
-          for (int r = 0; r < R1; ++r)
+        for (int r = 0; r < R1; ++r)
 #pragma unroll
-            for (int c = 0; c < R2; ++c) {
-              if (EPI == 2) yv[r][c] = ld_if(yp + (r * n2 + c), a.y && on[r][c]);
-              vv[r][c] = ld_if(vp + (r * n2 + c), a.vpot && on[r][c]);
-            }
-        }
+          for (int c = 0; c < R2; ++c) {
+            if (EPI == 2) yv[r][c] = ld_if(yp + (r * n2 + c), a.y && on[r][c]);
+            vv[r][c] = ld_if(vp + (r * n2 + c), a.vpot && on[r][c]);
+          }
+      }
+      // only this part is unrolled over the turns of the register queue (the
+      // whole step seven times over waited for instructions: 68 -> 59 us for 96
+      // complex128 bands of 28^3, 580 -> 537 us for 160 FP64 bands of 75^3)
+      auto turn_of = [&](auto uc) {
+        constexpr int u = uc.value;
         const T* P = slots + slot * slot_elems + own;
         const bool outside = j < 0 || j >= n0;
         if (outside && !a.pbc0) {
@@ -259,9 +262,20 @@ __global__ void __launch_bounds__(ROWS_NT, 2) rows_star_kernel(const __grid_cons
           if (EPI == 2) yp += yp ? n12 : 0;
           if (EPI) vp += vp ? n12 : 0;
         }
-        if (++slot == NS) slot = 0;
-        }
+      };
+      switch (turn) {
+        case 0: turn_of(std::integral_constant<int, 0>{}); break;
+        case 1: turn_of(std::integral_constant<int, 1 % NQ>{}); break;
+        case 2: turn_of(std::integral_constant<int, 2 % NQ>{}); break;
+        case 3: if constexpr (NQ > 3) turn_of(std::integral_constant<int, 3 % NQ>{}); break;
+        case 4: if constexpr (NQ > 3) turn_of(std::integral_constant<int, 4 % NQ>{}); break;
+        case 5: if constexpr (NQ > 5) turn_of(std::integral_constant<int, 5 % NQ>{}); break;
+        case 6: if constexpr (NQ > 5) turn_of(std::integral_constant<int, 6 % NQ>{}); break;
+        case 7: if constexpr (NQ > 7) turn_of(std::integral_constant<int, 7 % NQ>{}); break;
+        case 8: if constexpr (NQ > 7) turn_of(std::integral_constant<int, 8 % NQ>{}); break;
       }
+      if (++turn == NQ) turn = 0;
+      if (++slot == NS) slot = 0;
     }
     cp_async_wait<0>();
   }
