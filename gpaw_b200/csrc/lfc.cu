@@ -48,6 +48,11 @@ struct gb_lfc {
   int* ct_M = nullptr;        // [C]
   int* ct_nm = nullptr;       // [C]
   int* ct_W = nullptr;        // [C]
+  // zero-padded FP32 rows of A in contribution order (FP32 real add outside
+  // the bricks, at most 16 functions per volume)
+  int pad_nm = 0;             // 8 or 16; 0 = not built
+  bool pad_full = false;      // every contribution has pad_nm functions at a multiple of 4
+  float* A32p = nullptr;      // [C][pad_nm]
   // integrate (group-major)
   int ngroups = 0;
   int* gr_M = nullptr;        // [ngroups]
@@ -59,7 +64,7 @@ struct gb_lfc {
   int* row_G = nullptr;       // [rows] grid point of every global row
   int64_t* vol_aoff = nullptr;  // [nW] offset (doubles) of row0 in A
   std::vector<int> h_gr_nm;
-  // FP64 tensor-core add / integrate for real data (every volume has <= 16
+  // tensor-core add / integrate for FP64 real data (every volume has <= 16
   // functions): one entry per (volume, 8-point sub-tile of the flattened grid
   // it touches) with its values there as nf dense [m][p] 8 x 8 blocks
   int nf = 0;                 // 1 or 2 blocks per entry; 0 = not built
@@ -367,13 +372,132 @@ __global__ void __launch_bounds__(NT) lfc_integrate_kernel(const LfcView l, cons
   }
 }
 
+// -------------------------------------- FP32 real data outside the bricks
+// One thread per covered point holds the zero-padded A rows of its first KREG
+// contributions in registers (a copy of A in contribution order, so a warp's
+// row loads are contiguous) and loops over the bands XU at a time, issuing the
+// XU read-modify-write loads of a[x][G] before the coefficient loads and FMAs
+// of those bands.  Per band it sums the contributions in point order, m within
+// each, as lfc_add_kernel does: the same bits.  (FP32 data widened for the FP64
+// matrix instructions below were slower for most calls: 72^3 zero-boundary
+// grid, 24 atoms with 5 functions, 160 bands: add 111 against 76 us, integrate
+// 163 against 39 us.)
+template <int NMAX, bool FULL>
+__device__ __forceinline__ void load_coef(const float* __restrict__ cx, int nm, float (&v)[NMAX]) {
+  if constexpr (FULL) {
+#pragma unroll
+    for (int h = 0; h < NMAX / 4; ++h) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(cx) + h);
+      v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < NMAX; ++m) v[m] = m < nm ? __ldg(cx + m) : 0.f;
+  }
+}
+
+// acc[u] += sum_m A[m] c[x0 + u][M + m], u < NU, cx = &c[x0][M] (the
+// contribution's sum is formed first, then added)
+template <int NMAX, bool FULL, int NU>
+__device__ __forceinline__ void add_contribution(const float (&A)[NMAX], const float* __restrict__ cx, int nM, int nm,
+                                                 float (&acc)[NU]) {
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    float cv[NMAX];
+    load_coef<NMAX, FULL>(cx, nm, cv);
+    float t = 0.f;
+#pragma unroll
+    for (int m = 0; m < NMAX; ++m) t = fmadd(t, A[m], cv[m]);
+    acc[u] += t;
+    cx += nM;
+  }
+}
+
+// bands x0 .. x0 + NU - 1 of one point: a[x][G] += sum_k sum_m A_k[m] c[x][M_k + m]
+template <int NMAX, int KREG, bool FULL, int NU>
+__device__ __forceinline__ void add_point_bands(const float (&A)[KREG][NMAX], const float* const (&cb)[KREG],
+                                                const int (&nmk)[KREG], int K, int k0, const int* __restrict__ ct_M,
+                                                const int* __restrict__ ct_nm, const float* __restrict__ Ap,
+                                                const float* __restrict__ c_xM, int nM, int64_t x0,
+                                                float* __restrict__ ax, int64_t nG) {
+  float av[NU], acc[NU];
+  float* q = ax;
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    av[u] = *q;
+    acc[u] = 0.f;
+    q += nG;
+  }
+  const int64_t xo = x0 * nM;
+#pragma unroll
+  for (int k = 0; k < KREG; ++k)
+    if (k < K) add_contribution<NMAX, FULL, NU>(A[k], cb[k] + xo, nM, nmk[k], acc);
+  for (int k = KREG; k < K; ++k) {
+    float Ak[NMAX];
+    load_coef<NMAX, true>(Ap + (int64_t)(k0 + k) * NMAX, NMAX, Ak);
+    add_contribution<NMAX, FULL, NU>(Ak, c_xM + ct_M[k0 + k] + xo, nM, ct_nm[k0 + k], acc);
+  }
+  q = ax;
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    *q = av[u] + acc[u];
+    q += nG;
+  }
+}
+
+template <int NMAX, int KREG, bool FULL, int XU>
+__global__ void __launch_bounds__(256) lfc_add_bands_kernel(const int* __restrict__ pt_G, const int* __restrict__ pt_off,
+                                                            const int* __restrict__ ct_M,
+                                                            const int* __restrict__ ct_nm,
+                                                            const float* __restrict__ Ap, int64_t P,
+                                                            const float* __restrict__ c_xM, int nM,
+                                                            float* __restrict__ a_xG, int64_t nG, int64_t nx) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  const int k0 = pt_off[p], K = pt_off[p + 1] - k0;
+  float A[KREG][NMAX];
+  const float* cb[KREG];
+  int nmk[KREG];
+#pragma unroll
+  for (int k = 0; k < KREG; ++k) {
+    const bool on = k < K;
+    if (on) load_coef<NMAX, true>(Ap + (int64_t)(k0 + k) * NMAX, NMAX, A[k]);
+    cb[k] = c_xM + (on ? ct_M[k0 + k] : 0);
+    nmk[k] = on ? ct_nm[k0 + k] : 0;
+  }
+  const int64_t nfull = nx / XU * XU;
+  float* ax = a_xG + pt_G[p];
+  for (int64_t x0 = 0; x0 < nfull; x0 += XU, ax += XU * nG)
+    add_point_bands<NMAX, KREG, FULL, XU>(A, cb, nmk, K, k0, ct_M, ct_nm, Ap, c_xM, nM, x0, ax, nG);
+  for (int64_t x0 = nfull; x0 < nx; ++x0, ax += nG)
+    add_point_bands<NMAX, KREG, FULL, 1>(A, cb, nmk, K, k0, ct_M, ct_nm, Ap, c_xM, nM, x0, ax, nG);
+}
+
+static int add_bands(const gb_lfc* l, const float* c, float* a, int64_t nx, cudaStream_t st) {
+  const bool full = l->pad_full && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
+  const unsigned grid = (unsigned)((l->P + 255) / 256);
+  auto kern = l->pad_nm == 8 ? (full ? lfc_add_bands_kernel<8, 4, true, 8> : lfc_add_bands_kernel<8, 4, false, 8>)
+                             : (full ? lfc_add_bands_kernel<16, 2, true, 8> : lfc_add_bands_kernel<16, 2, false, 8>);
+  kern<<<grid, 256, 0, st>>>(l->pt_G, l->pt_off, l->ct_M, l->ct_nm, l->A32p, l->P, c, l->nM, a, l->nG, nx);
+  return check_launch("lfc_add_bands_kernel");
+}
+
+// A32p[c][m] = A of contribution c, zero for m >= nm
+static __global__ void lfc_pad_rows_kernel(const double* __restrict__ A, const int64_t* __restrict__ ct_aoff,
+                                           const int* __restrict__ ct_nm, int64_t C, int F, float* __restrict__ Ap) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < C * F; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = i / F;
+    const int m = (int)(i - c * F);
+    Ap[i] = m < ct_nm[c] ? (float)A[ct_aoff[c] + m] : 0.f;
+  }
+}
+
 // ------------------------------------------------ real data, FP64 tensor cores
-// For real data (Gamma point: every periodic image has phase 1) and at most
-// 16 functions per volume both products run as m16n8k8 FP64 MMAs on 16 bands
-// x 8 grid points x 8 functions, the three operands exactly as they lie in
-// memory: bands x points (a), points x functions (an entry's dense block) and
-// bands x functions (c).  FP32 data are widened on the way in and rounded
-// once on the way out.
+// For FP64 real data (Gamma point: every periodic image has phase 1) and at
+// most 16 functions per volume both products run as m16n8k8 FP64 MMAs on 16
+// bands x 8 grid points x 8 functions, the three operands exactly as they lie
+// in memory: bands x points (a), points x functions (an entry's dense block)
+// and bands x functions (c).
 //   integrate: a cluster of four CTAs takes one function group and 16 NB
 //     bands; its 32 warps split the group's entries evenly, and the 32 sums
 //     are added in warp order (shared, then distributed shared memory).
@@ -388,9 +512,7 @@ __global__ void __launch_bounds__(NT) lfc_integrate_kernel(const LfcView l, cons
 // all the same (integrate 114 us with 32 bands, 135 with 16).  71^3 grid, 24
 // atoms x 9 functions of radius 2.5 A, 96 FP64 bands: integrate 189 -> 84 us,
 // add 196 -> 140 us against the point-major kernels (gathered rows, one point
-// per thread).  FP32 with at most eight functions keeps the brick tiling
-// below, which is as fast there (an FP32 form of this add with coefficients
-// and blocks read through L1 took 140 us against 133 us).
+// per thread).
 __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
@@ -638,7 +760,7 @@ static int integrate_t(const gb_lfc* l, const void* a, void* c, int64_t nx, int 
     if (tiles_usable(l, a))
       return integrate_tiles(l, static_cast<const float*>(a), static_cast<float*>(c), nx, st);
   }
-  if constexpr (!Elem<T>::cplx) {
+  if constexpr (std::is_same<T, double>::value) {
     if (mma_usable(l, nx)) return integrate_mma<T>(l, a, c, nx, st);
   }
   // groups are sorted by nm on the host; one launch per padded class
@@ -1062,8 +1184,9 @@ static int add_t(const gb_lfc* l, const void* c, void* a, int64_t nx, int q, cud
   if (l->P == 0) return GB_OK;
   if constexpr (std::is_same<T, float>::value) {
     if (tiles_usable(l, a)) return add_tiles(l, static_cast<const float*>(c), static_cast<float*>(a), nx, st);
+    if (l->A32p) return add_bands(l, static_cast<const float*>(c), static_cast<float*>(a), nx, st);
   }
-  if constexpr (!Elem<T>::cplx) {
+  if constexpr (std::is_same<T, double>::value) {
     if (mma_usable(l, nx)) return add_mma<T>(l, c, a, nx, st);
   }
   switch (nm_class(l->maxnm)) {
@@ -1496,6 +1619,18 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     ok = l->A32 != nullptr;
     if (ok && l->nA) {
       to_float<<<std::min<int64_t>((l->nA + 255) / 256, 4096), 256>>>(l->A64, l->A32, l->nA);
+      ok = cudaDeviceSynchronize() == cudaSuccess;
+    }
+  }
+  if (ok && !tiled && l->maxnm <= 16 && l->C) {
+    l->pad_nm = l->maxnm <= 8 ? 8 : 16;
+    l->pad_full = nM % 4 == 0;
+    for (size_t i = 0; i < ct_nm.size() && l->pad_full; ++i) l->pad_full = ct_nm[i] == l->pad_nm && ct_M[i] % 4 == 0;
+    l->A32p = dalloc<float>(l, l->C * l->pad_nm);
+    ok = l->A32p != nullptr;
+    if (ok) {
+      lfc_pad_rows_kernel<<<(unsigned)std::min<int64_t>((l->C * l->pad_nm + 255) / 256, 4096), 256>>>(
+          l->A64, l->ct_aoff, l->ct_nm, l->C, l->pad_nm, l->A32p);
       ok = cudaDeviceSynchronize() == cudaSuccess;
     }
   }

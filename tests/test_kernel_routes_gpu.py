@@ -1,0 +1,57 @@
+"""GPU: which kernel a call takes, for the forms whose rule was drawn by
+measuring both sides, and what a rule must not change: a band's result must
+not depend on how many bands come with it."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def kernels(f):
+    """Names of the kernels f() launches."""
+    f()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+def lfc_on(N, pbc, natoms, ls, seed=3):
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    from gpaw_b200.lfc import LFC
+    from gpaw_b200.spline import Spline
+    rc = 3.4
+    r = np.linspace(0, rc, 41)
+    spl = [Spline.from_data(l, rc, np.exp(-(r / 1.5)**2) * (1 + 0.3 * j)) for j, l in enumerate(ls)]
+    gd = GridDescriptor((N, N, N), (0.38 * N,) * 3, pbc)
+    lfc = LFC(gd, [spl] * natoms, cut=True)
+    lfc.set_positions(0.2 + 0.6 * np.random.default_rng(seed).random((natoms, 3)))
+    return gd, lfc
+
+
+@pytest.mark.parametrize('N,pbc,ls', [(24, 0, (0, 0, 1)),       # 23^3 points: no multiple of 4
+                                      (24, 1, (0, 1, 2)),       # 9 functions
+                                      (24, 0, (0, 1, 0, 1, 0, 2))])
+@pytest.mark.parametrize('nx', [1, 2, 40])
+def test_fp32_lfc_outside_the_bricks(N, pbc, ls, nx):
+    """FP32 data that the bricks do not take: FP32 sums, point by point and
+    group by group (widened for the FP64 matrix instructions they took up to
+    four times as long), one kernel each whatever the number of bands."""
+    gd, lfc = lfc_on(N, pbc, 5, ls)
+    g = torch.Generator(device='cuda').manual_seed(nx)
+    a = torch.randn((nx,) + tuple(gd.n_c), generator=g, device='cuda', dtype=torch.float32)
+    c = torch.randn((nx, lfc.Mmax), generator=g, device='cuda', dtype=torch.float32)
+    names = kernels(lambda: lfc.integrate(a, {}))
+    assert any('lfc_integrate_kernel' in k for k in names) and not any('mma' in k for k in names)
+    b = a.clone()
+    names = kernels(lambda: lfc.add_M(b, c))
+    assert any('lfc_add_bands_kernel' in k for k in names) and not any('mma' in k for k in names)
+    b = a.clone()
+    lfc.add_M(b, c)
+    P = lfc.integrate(a, {})
+    one = a[nx - 1:].clone()
+    lfc.add_M(one, c[nx - 1:].contiguous())
+    assert torch.equal(one, b[nx - 1:])
+    assert torch.equal(lfc.integrate(a[nx - 1:].contiguous(), {}), P[nx - 1:])
