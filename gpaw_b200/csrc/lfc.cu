@@ -71,10 +71,10 @@ struct gb_lfc {
   int ns = 0;                 // sub-tiles with entries
   int2* st_sub = nullptr;     // [ns] sub-tile | mask of its covered points
   int* st_eoff = nullptr;     // [ns + 1] entries of each
-  int2* st_M = nullptr;       // [ne] first function and function count of an entry
+  int2* st_M = nullptr;       // [ne] first function | function count + covered points << 8 of an entry
   double* st_A = nullptr;     // [ne][nf][8][8]
   int* sg_off = nullptr;      // [ngroups + 1] entries of each function group:
-  int2* sg_e = nullptr;       //   entry | sub-tile, in the order of the sub-tiles
+  int4* sg_e = nullptr;       //   entry | sub-tile | covered points, in the order of the sub-tiles
   // brick-tiled FP32 add / integrate for real data (every volume has <= 8
   // functions, nG a multiple of 4): 32-point chunks of four 8-point
   // sub-tiles; one entry per (volume, sub-tile it touches) with the volume's
@@ -505,8 +505,9 @@ static __global__ void lfc_pad_rows_kernel(const double* __restrict__ A, const i
 //     the sum to the covered points.
 // The split depends on the object alone and every sum has one order, so the
 // results depend neither on scheduling nor on how the bands are blocked.
-// A non-finite value at an uncovered point (integrate) or in the coefficients
-// of another volume (add) can reach the sums of its own sub-tile.
+// A sub-tile holds points that a volume does not cover: integrate reads them
+// as zeros and add drops what an entry gives there, so that a non-finite
+// value reaches the sums it belongs to and no others.
 //
 // Bound by the latency of gathered operands; fewer bands per warp is slower
 // all the same (integrate 114 us with 32 bands, 135 with 16).  71^3 grid, 24
@@ -526,7 +527,7 @@ constexpr int LM_WARPS = 8;
 
 template <typename T, int NB, int NF>
 __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WARPS)
-    lfc_integrate_mma_kernel(const int* __restrict__ sg_off, const int2* __restrict__ sg_e,
+    lfc_integrate_mma_kernel(const int* __restrict__ sg_off, const int4* __restrict__ sg_e,
                              const double* __restrict__ st_A, const int* __restrict__ gr_M,
                              const int* __restrict__ gr_nm, const T* __restrict__ a_xG, T* __restrict__ c_xM,
                              int64_t nx, int64_t nG, int nM, double dv) {
@@ -558,9 +559,9 @@ __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WAR
       for (int k = 0; k < 4; ++k) acc[i][f][k] = 0.0;
 #pragma unroll 2
   for (int q = i0; q < i1; ++q) {
-    const int2 es = sg_e[q];
+    const int4 es = __ldg(sg_e + q);
     const int64_t p = (int64_t)es.y * 8 + t;
-    const bool in0 = p < nG, in1 = p + 4 < nG;
+    const bool in0 = es.z >> t & 1, in1 = es.z >> t & 16;
     const double* blk = st_A + (int64_t)es.x * (NF * 64) + g * 8 + t;
     double b[NF][2];
 #pragma unroll
@@ -640,15 +641,22 @@ __global__ void __launch_bounds__(32 * LM_WARPS)
     for (int k = 0; k < 4; ++k) acc[i][k] = 0.0;
   for (int e = e0; e < e1; ++e) {
     const int2 mn = st_M[e];
+    const int nm = mn.y & 255;
+    const bool cov[2] = {(mn.y >> (8 + 2 * t) & 1) != 0, (mn.y >> (9 + 2 * t) & 1) != 0};
+    double b[NF][2];
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-      if (f * 8 >= mn.y) break;
       const double* blk = st_A + ((int64_t)e * NF + f) * 64 + t * 8 + g;
-      const double b0 = __ldg(blk), b1 = __ldg(blk + 32);
-      const int m = f * 8 + t;
-      const bool in0 = m < mn.y, in1 = m + 4 < mn.y;
+      b[f][0] = __ldg(blk);
+      b[f][1] = __ldg(blk + 32);
+    }
 #pragma unroll
-      for (int i = 0; i < NB; ++i) {
+    for (int i = 0; i < NB; ++i) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const int m = f * 8 + t;
+        const bool in0 = m < nm, in1 = m + 4 < nm;
         double cv[4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -656,8 +664,11 @@ __global__ void __launch_bounds__(32 * LM_WARPS)
           cv[h] = on[i][h] && in0 ? (double)__ldg(c) : 0.0;
           cv[2 + h] = on[i][h] && in1 ? (double)__ldg(c + 4) : 0.0;
         }
-        mma_f64(acc[i], cv, b0, b1);
+        mma_f64(d, cv, b[f][0], b[f][1]);
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (cov[k & 1]) acc[i][k] += d[k];
     }
   }
 #pragma unroll
@@ -1437,7 +1448,8 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     gr_voff.push_back((int)gv_W.size());
   }
   // entries of the tensor-core path, in the order of their sub-tiles
-  std::vector<int2> st_sub, st_M, sg_e;
+  std::vector<int2> st_sub, st_M;
+  std::vector<int4> sg_e;
   std::vector<int> st_eoff, sg_off;
   std::vector<double> st_A;
   if (l->maxnm <= 16 && nW > 0) {
@@ -1457,7 +1469,7 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     std::sort(ents.begin(), ents.end(),
               [](const Ent& x, const Ent& y) { return x.sub != y.sub ? x.sub < y.sub : x.W < y.W; });
     st_A.assign(ents.size() * (size_t)nblk, 0.0);
-    std::vector<std::vector<int2>> by_group(ngr);
+    std::vector<std::vector<int4>> by_group(ngr);
     for (size_t e = 0; e < ents.size(); ++e) {
       const Ent& n = ents[e];
       if (st_sub.empty() || st_sub.back().x != n.sub) {
@@ -1465,15 +1477,17 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
         st_eoff.push_back((int)e);
       }
       const int nm = nm_W[n.W];
-      st_M.push_back(make_int2(M_W[n.W], nm));
-      by_group[vol_group[n.W]].push_back(make_int2((int)e, n.sub));
+      int cov = 0;
       double* blk = st_A.data() + e * (size_t)nblk;
       for (int64_t r = n.r0; r < n.r1; ++r) {
         const int p = row_G[r] % 8;
-        st_sub.back().y |= 1 << p;
+        cov |= 1 << p;
         const double* Ar = A_all + aoff[n.W] + (r - row0[n.W]) * nm;
         for (int m = 0; m < nm; ++m) blk[m * 8 + p] = Ar[m];
       }
+      st_sub.back().y |= cov;
+      st_M.push_back(make_int2(M_W[n.W], nm | cov << 8));
+      by_group[vol_group[n.W]].push_back(make_int4((int)e, n.sub, cov, 0));
     }
     st_eoff.push_back((int)ents.size());
     sg_off.push_back(0);

@@ -348,3 +348,43 @@ def test_fp32_tiled_fallback_when_a_chunk_meets_too_many_groups():
     b = torch.from_numpy(a0).cuda().float()
     lfc.add_M(b, torch.from_numpy(c).cuda().float())
     assert rel(b.double().cpu().numpy(), ol.add(a0.copy(), c, Phi)) < 1e-5
+
+
+@pytest.mark.parametrize('n_c,dtype', [((21, 22, 23), torch.float64), ((21, 22, 23), torch.float32),
+                                       ((20, 22, 24), torch.float64)])
+@pytest.mark.parametrize('nfun', [4, 12])
+def test_non_finite_values_stay_with_their_own_sums(n_c, dtype, nfun):
+    """Infinities and NaNs of the grids at points outside every sphere reach
+    no projection; those of one atom's coefficients reach the points of its
+    spheres and no others.  Everything else keeps its bits."""
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    from gpaw_b200.lfc import LFC
+    from gpaw_b200.spline import Spline
+    rc = 2.9
+    r = np.linspace(0, rc, 41)
+    ls = {4: (0, 1), 12: (0, 1, 0, 1, 0, 1)}[nfun]
+    spl = [(l, rc, np.exp(-r**2 / 2) * (1 + 0.3 * j)) for j, l in enumerate(ls)]
+    gd = GridDescriptor(n_c, 0.4 * np.array(n_c), True)
+    spos = np.array([[0.3, 0.3, 0.3], [0.45, 0.4, 0.5]])
+    lfc = LFC(gd, [[Spline.from_data(*s) for s in spl]] * 2)
+    lfc.set_positions(spos)
+    Phi = ol.dense_functions(gd.N_c, gd.cell_cv, gd.pbc_c, spos, [spl] * 2).reshape(2, nfun, -1)
+    cover = torch.from_numpy((Phi != 0).any(axis=1)).cuda()          # [atom][G]
+    g = torch.Generator(device='cuda').manual_seed(1)
+    nx = 18
+    a = torch.randn((nx,) + tuple(gd.n_c), generator=g, device='cuda', dtype=dtype)
+    c = torch.randn((nx, lfc.Mmax), generator=g, device='cuda', dtype=dtype)
+    bare = ~cover.any(0)
+    assert bare.any() and (cover[1] & ~cover[0]).any()
+    bad = a.clone()
+    bad.flatten(1)[:, bare] = torch.tensor([float('nan'), float('inf'), float('-inf')], device='cuda',
+                                           dtype=dtype)[torch.arange(int(bare.sum()), device='cuda') % 3]
+    assert torch.equal(lfc.integrate(bad, {}), lfc.integrate(a, {}))
+    good, out = a.clone(), a.clone()
+    lfc.add_M(good, c)
+    c[:, 0] = float('nan')
+    c[::2, 1] = float('inf')
+    lfc.add_M(out, c)
+    own = cover[0]
+    assert torch.equal(out.flatten(1)[:, ~own], good.flatten(1)[:, ~own])
+    assert not torch.isfinite(out.flatten(1)[:, own]).any()
