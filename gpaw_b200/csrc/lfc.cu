@@ -460,10 +460,16 @@ __global__ void __launch_bounds__(256) lfc_add_bands_kernel(const int* __restric
   int nmk[KREG];
 #pragma unroll
   for (int k = 0; k < KREG; ++k) {
-    const bool on = k < K;
-    if (on) load_coef<NMAX, true>(Ap + (int64_t)(k0 + k) * NMAX, NMAX, A[k]);
-    cb[k] = c_xM + (on ? ct_M[k0 + k] : 0);
-    nmk[k] = on ? ct_nm[k0 + k] : 0;
+    if (k < K) {
+      load_coef<NMAX, true>(Ap + (int64_t)(k0 + k) * NMAX, NMAX, A[k]);
+      cb[k] = c_xM + ct_M[k0 + k];
+      nmk[k] = ct_nm[k0 + k];
+    } else {
+#pragma unroll
+      for (int m = 0; m < NMAX; ++m) A[k][m] = 0.f;
+      cb[k] = c_xM;
+      nmk[k] = 0;
+    }
   }
   const int64_t nfull = nx / XU * XU;
   float* ax = a_xG + pt_G[p];
