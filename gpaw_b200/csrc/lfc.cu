@@ -69,8 +69,8 @@ struct gb_lfc {
   // it touches) with its values there as nf dense [m][p] 8 x 8 blocks
   int nf = 0;                 // 1 or 2 blocks per entry; 0 = not built
   int ns = 0;                 // sub-tiles with entries
-  int2* st_sub = nullptr;     // [ns] sub-tile | mask of its covered points
-  int* st_eoff = nullptr;     // [ns + 1] entries of each
+  int4* st_sub = nullptr;     // [ns][2] sub-tile | mask of its covered points | its entries' range,
+                              //   then the first entry's st_M
   int2* st_M = nullptr;       // [ne] first function | function count + covered points << 8 of an entry
   double* st_A = nullptr;     // [ne][nf][8][8]
   int* sg_off = nullptr;      // [ngroups + 1] entries of each function group:
@@ -504,22 +504,31 @@ static __global__ void lfc_pad_rows_kernel(const double* __restrict__ A, const i
 // bands x 8 grid points x 8 functions, the three operands exactly as they lie
 // in memory: bands x points (a), points x functions (an entry's dense block)
 // and bands x functions (c).
-//   integrate: a cluster of four CTAs takes one function group and 16 NB
-//     bands; its 32 warps split the group's entries evenly, and the 32 sums
-//     are added in warp order (shared, then distributed shared memory).
-//   add: a warp takes one sub-tile and 16 NB bands, sums its entries and adds
+//   integrate: a cluster of four CTAs takes one function group and 16 bands;
+//     its 32 warps split the group's entries evenly, and the 32 sums are added
+//     in warp order (shared, then distributed shared memory).
+//   add: a warp takes one sub-tile and 16 bands, sums its entries and adds
 //     the sum to the covered points.
 // The split depends on the object alone and every sum has one order, so the
-// results depend neither on scheduling nor on how the bands are blocked.
+// results depend neither on scheduling nor on how the bands are blocked.  (The
+// add of one grid alone takes lfc_add_kernel, whose sums may differ from those
+// of a block in the last bits.)
 // A sub-tile holds points that a volume does not cover: integrate reads them
 // as zeros and add drops what an entry gives there, so that a non-finite
 // value reaches the sums it belongs to and no others.
 //
-// Bound by the latency of gathered operands; fewer bands per warp is slower
-// all the same (integrate 114 us with 32 bands, 135 with 16).  71^3 grid, 24
-// atoms x 9 functions of radius 2.5 A, 96 FP64 bands: integrate 189 -> 84 us,
-// add 196 -> 140 us against the point-major kernels (gathered rows, one point
-// per thread).
+// Bound by the latency of gathered operands, so by the warps in flight: one
+// 16-band tile per warp.  (Up to five, one read of a block for 80 bands at up
+// to 190 registers, took 1.6 times as long for the projections of 160 bands on
+// 1 to 64 atoms, in the geometric mean, and 1.3 times for the add; three were
+// faster only where they make the last wave, 90 against 108 us for 96 bands of
+// 9 functions on 24 atoms.)  The add reads the grid points it updates before
+// its sums; in the loop over the stores each load waited for the store before
+// it.  Inputs from HBM, 71^3 points, radius 2.1 A, point-major kernels (gathered
+// rows, one point per thread) against these:
+//   24 atoms x 9 functions, 96 bands:  integrate 127 ->  75 us, add 174 ->  76 us
+//   24 atoms x 5 functions, 160 bands: integrate 120 ->  77 us, add 169 ->  89 us
+//    4 atoms x 9 functions, 32 bands:  integrate  64 ->  36 us, add  22 ->  13 us
 __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
@@ -531,75 +540,59 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], do
 constexpr int LM_CLUSTER = 4;              // CTAs per (function group, band block)
 constexpr int LM_WARPS = 8;
 
-template <typename T, int NB, int NF>
+template <int NF>
 __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WARPS)
     lfc_integrate_mma_kernel(const int* __restrict__ sg_off, const int4* __restrict__ sg_e,
                              const double* __restrict__ st_A, const int* __restrict__ gr_M,
-                             const int* __restrict__ gr_nm, const T* __restrict__ a_xG, T* __restrict__ c_xM,
-                             int64_t nx, int64_t nG, int nM, double dv) {
-  extern __shared__ __align__(16) double lm_red[];   // [LM_WARPS][NB * NF * 4][32]
-  constexpr int NE = NB * NF * 128;
+                             const int* __restrict__ gr_nm, const double* __restrict__ a_xG,
+                             double* __restrict__ c_xM, int64_t nx, int64_t nG, int nM, double dv) {
+  constexpr int NE = NF * 128;
+  __shared__ double red[LM_WARPS * NE];        // [warp][function block][k][lane]
   const int rank = blockIdx.x % LM_CLUSTER, gi = blockIdx.x / LM_CLUSTER;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int64_t x0 = (int64_t)blockIdx.y * 16 * NB;
+  const int64_t x0 = (int64_t)blockIdx.y * 16;
   const int M = gr_M[gi], nm = gr_nm[gi];
   const int e0 = sg_off[gi], ne = sg_off[gi + 1] - e0, w = rank * LM_WARPS + warp;
   const int i0 = e0 + (int)((int64_t)ne * w / (LM_CLUSTER * LM_WARPS));
   const int i1 = e0 + (int)((int64_t)ne * (w + 1) / (LM_CLUSTER * LM_WARPS));
-  const T* row[NB][2];
-  bool on[NB][2];
+  const double* row[2];
+  bool on[2];
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
+  for (int h = 0; h < 2; ++h) {
+    const int64_t x = x0 + 8 * h + g;
+    on[h] = x < nx;
+    row[h] = a_xG + (on[h] ? x : 0) * nG + t;
+  }
+  double acc[NF][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t x = x0 + 16 * i + 8 * h + g;
-      on[i][h] = x < nx;
-      row[i][h] = a_xG + (on[i][h] ? x : 0) * nG;
-    }
-  double acc[NB][NF][4];
+  for (int f = 0; f < NF; ++f)
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
-#pragma unroll
-    for (int f = 0; f < NF; ++f)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[i][f][k] = 0.0;
+    for (int k = 0; k < 4; ++k) acc[f][k] = 0.0;
 #pragma unroll 2
   for (int q = i0; q < i1; ++q) {
     const int4 es = __ldg(sg_e + q);
-    const int64_t p = (int64_t)es.y * 8 + t;
+    const int64_t p = (int64_t)es.y * 8;
     const bool in0 = es.z >> t & 1, in1 = es.z >> t & 16;
     const double* blk = st_A + (int64_t)es.x * (NF * 64) + g * 8 + t;
-    double b[NF][2];
+    double av[4];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      b[f][0] = __ldg(blk + f * 64);
-      b[f][1] = __ldg(blk + f * 64 + 4);
+    for (int h = 0; h < 2; ++h) {
+      av[h] = on[h] && in0 ? __ldg(row[h] + p) : 0.0;
+      av[2 + h] = on[h] && in1 ? __ldg(row[h] + p + 4) : 0.0;
     }
-    double av[NB][4];
 #pragma unroll
-    for (int i = 0; i < NB; ++i)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        av[i][h] = on[i][h] && in0 ? (double)__ldg(row[i][h] + p) : 0.0;
-        av[i][2 + h] = on[i][h] && in1 ? (double)__ldg(row[i][h] + p + 4) : 0.0;
-      }
-#pragma unroll
-    for (int i = 0; i < NB; ++i)
-#pragma unroll
-      for (int f = 0; f < NF; ++f) mma_f64(acc[i][f], av[i], b[f][0], b[f][1]);
+    for (int f = 0; f < NF; ++f) mma_f64(acc[f], av, __ldg(blk + f * 64), __ldg(blk + f * 64 + 4));
   }
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
+  for (int f = 0; f < NF; ++f)
 #pragma unroll
-    for (int f = 0; f < NF; ++f)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) lm_red[warp * NE + ((i * NF + f) * 4 + k) * 32 + lane] = acc[i][f][k];
+    for (int k = 0; k < 4; ++k) red[warp * NE + (f * 4 + k) * 32 + lane] = acc[f][k];
   __syncthreads();
   for (int e = threadIdx.x; e < NE; e += 32 * LM_WARPS) {
-    double v = lm_red[e];
+    double v = red[e];
 #pragma unroll
-    for (int ww = 1; ww < LM_WARPS; ++ww) v += lm_red[ww * NE + e];
-    lm_red[e] = v;
+    for (int ww = 1; ww < LM_WARPS; ++ww) v += red[ww * NE + e];
+    red[e] = v;
   }
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -607,143 +600,91 @@ __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WAR
   for (int e = rank * 32 * LM_WARPS + threadIdx.x; e < NE; e += LM_CLUSTER * 32 * LM_WARPS) {
     double v = 0.0;
 #pragma unroll
-    for (int r = 0; r < LM_CLUSTER; ++r) v += cluster.map_shared_rank(lm_red, r)[e];
-    const int l = e & 31, k = (e >> 5) & 3, f = (e >> 7) % NF, i = (e >> 7) / NF;
-    const int64_t x = x0 + 16 * i + 8 * (k >> 1) + (l >> 2);
+    for (int r = 0; r < LM_CLUSTER; ++r) v += cluster.map_shared_rank(red, r)[e];
+    const int l = e & 31, k = (e >> 5) & 3, f = e >> 7;
+    const int64_t x = x0 + 8 * (k >> 1) + (l >> 2);
     const int m = f * 8 + 2 * (l & 3) + (k & 1);
     if (x < nx && m < nm) {
-      T* cp = c_xM + x * nM + M + m;
-      *cp = (T)fma(dv, v, (double)*cp);
+      double* cp = c_xM + x * nM + M + m;
+      *cp = fma(dv, v, *cp);
     }
   }
   cluster.sync();        // the other CTAs may still be reading this one's sums
 }
 
-template <typename T, int NB, int NF>
+template <int NF>
 __global__ void __launch_bounds__(32 * LM_WARPS)
-    lfc_add_mma_kernel(int ns, const int2* __restrict__ st_sub, const int* __restrict__ st_eoff,
-                       const int2* __restrict__ st_M, const double* __restrict__ st_A, const T* __restrict__ c_xM,
-                       T* __restrict__ a_xG, int64_t nx, int64_t nG, int nM) {
+    lfc_add_mma_kernel(int ns, const int4* __restrict__ st_sub, const int2* __restrict__ st_M,
+                       const double* __restrict__ st_A, const double* __restrict__ c_xM, double* __restrict__ a_xG,
+                       int64_t nx, int64_t nG, int nM) {
   const int s = blockIdx.x * LM_WARPS + (threadIdx.x >> 5);
   if (s >= ns) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int64_t x0 = (int64_t)blockIdx.y * 16 * NB;
-  const int2 sub = st_sub[s];
-  const int e0 = st_eoff[s], e1 = st_eoff[s + 1];
-  const T* row[NB][2];
-  bool on[NB][2];
+  const int64_t x0 = (int64_t)blockIdx.y * 16 + g;
+  // a sub-tile comes with its first entry, so that the loads of coefficients,
+  // block and grid points are one step behind its own
+  const int4 sub = __ldg(st_sub + 2 * s), first = __ldg(st_sub + 2 * s + 1);
+  const bool on[2] = {x0 < nx, x0 + 8 < nx};
+  const double* row[2];
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
+  for (int h = 0; h < 2; ++h) row[h] = c_xM + (on[h] ? x0 + 8 * h : 0) * nM + t;
+  // points 2 t and 2 t + 1 of bands x0 and x0 + 8: the four loads before the
+  // sums, the four stores after them
+  double* const ap = a_xG + x0 * nG + (int64_t)sub.x * 8 + 2 * t;
+  double old[4], acc[4];
+  bool wr[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t x = x0 + 16 * i + 8 * h + g;
-      on[i][h] = x < nx;
-      row[i][h] = c_xM + (on[i][h] ? x : 0) * nM;
-    }
-  double acc[NB][4];
-#pragma unroll
-  for (int i = 0; i < NB; ++i)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) acc[i][k] = 0.0;
-  for (int e = e0; e < e1; ++e) {
-    const int2 mn = st_M[e];
+  for (int k = 0; k < 4; ++k) {
+    wr[k] = on[k >> 1] && (sub.y >> (2 * t + (k & 1)) & 1);
+    old[k] = wr[k] ? ap[8 * (k >> 1) * nG + (k & 1)] : 0.0;
+    acc[k] = 0.0;
+  }
+  int2 mn = make_int2(first.x, first.y);
+  for (int e = sub.z; e < sub.w; ++e) {
     const int nm = mn.y & 255;
     const bool cov[2] = {(mn.y >> (8 + 2 * t) & 1) != 0, (mn.y >> (9 + 2 * t) & 1) != 0};
-    double b[NF][2];
+    double d[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       const double* blk = st_A + ((int64_t)e * NF + f) * 64 + t * 8 + g;
-      b[f][0] = __ldg(blk);
-      b[f][1] = __ldg(blk + 32);
-    }
+      const bool in0 = f * 8 + t < nm, in1 = f * 8 + t + 4 < nm;
+      double cv[4];
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      double d[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const int m = f * 8 + t;
-        const bool in0 = m < nm, in1 = m + 4 < nm;
-        double cv[4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const T* c = row[i][h] + mn.x + m;
-          cv[h] = on[i][h] && in0 ? (double)__ldg(c) : 0.0;
-          cv[2 + h] = on[i][h] && in1 ? (double)__ldg(c + 4) : 0.0;
-        }
-        mma_f64(d, cv, b[f][0], b[f][1]);
+      for (int h = 0; h < 2; ++h) {
+        const double* c = row[h] + mn.x + f * 8;
+        cv[h] = on[h] && in0 ? __ldg(c) : 0.0;
+        cv[2 + h] = on[h] && in1 ? __ldg(c + 4) : 0.0;
       }
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (cov[k & 1]) acc[i][k] += d[k];
+      mma_f64(d, cv, __ldg(blk), __ldg(blk + 32));
     }
+    if (e + 1 < sub.w) mn = __ldg(st_M + e + 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (cov[k & 1]) acc[k] += d[k];
   }
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int pt = 2 * t + (k & 1);
-      const int64_t x = x0 + 16 * i + 8 * (k >> 1) + g;
-      if (x < nx && (sub.y >> pt & 1)) {
-        T* ap = a_xG + x * nG + (int64_t)sub.x * 8 + pt;
-        *ap = (T)((double)*ap + acc[i][k]);
-      }
-    }
+  for (int k = 0; k < 4; ++k)
+    if (wr[k]) ap[8 * (k >> 1) * nG + (k & 1)] = old[k] + acc[k];
 }
 
-// A single grid (a density or potential, not a block of bands) would fill one
-// row of sixteen of every tile and keeps the point-major kernels; the launch
-// grid's second dimension bounds the bands.
-static bool mma_usable(const gb_lfc* l, int64_t nx) { return l->nf && nx > 1 && nx < 65535 * 16; }
+// the launch grid's second dimension bounds the bands
+static bool mma_usable(const gb_lfc* l, int64_t nx) { return l->nf && nx <= 65535 * 16; }
 
-// 16-band tiles per warp: at most 5, the blocks of a call as even as possible
-static int mma_tiles(int64_t nx) {
-  const int64_t tiles = (nx + 15) / 16, blocks = (tiles + 4) / 5;
-  return (int)((tiles + blocks - 1) / blocks);
-}
-
-template <typename T, int NB, int NF>
-static int integrate_mma_nb(const gb_lfc* l, const void* a, void* c, int64_t nx, cudaStream_t st) {
-  constexpr int smem = LM_WARPS * NB * NF * 128 * (int)sizeof(double);
-  auto kern = lfc_integrate_mma_kernel<T, NB, NF>;
-  static bool set = false;
-  if (!set && smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return check_launch("lfc shared memory");
-    set = true;
-  }
-  const dim3 grid((unsigned)(l->ngroups * LM_CLUSTER), (unsigned)((nx + 16 * NB - 1) / (16 * NB)));
-  kern<<<grid, 32 * LM_WARPS, smem, st>>>(l->sg_off, l->sg_e, l->st_A, l->gr_M, l->gr_nm, (const T*)a, (T*)c, nx,
-                                          l->nG, l->nM, l->dv);
+static int integrate_mma(const gb_lfc* l, const double* a, double* c, int64_t nx, cudaStream_t st) {
+  if (l->ngroups == 0) return GB_OK;
+  const dim3 grid((unsigned)(l->ngroups * LM_CLUSTER), (unsigned)((nx + 15) / 16));
+  auto kern = l->nf == 1 ? lfc_integrate_mma_kernel<1> : lfc_integrate_mma_kernel<2>;
+  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->sg_off, l->sg_e, l->st_A, l->gr_M, l->gr_nm, a, c, nx, l->nG, l->nM, l->dv);
   return check_launch("lfc_integrate_mma_kernel");
 }
 
-template <typename T, int NB, int NF>
-static int add_mma_nb(const gb_lfc* l, const void* c, void* a, int64_t nx, cudaStream_t st) {
-  const dim3 grid((unsigned)((l->ns + LM_WARPS - 1) / LM_WARPS), (unsigned)((nx + 16 * NB - 1) / (16 * NB)));
-  lfc_add_mma_kernel<T, NB, NF><<<grid, 32 * LM_WARPS, 0, st>>>(l->ns, l->st_sub, l->st_eoff, l->st_M, l->st_A,
-                                                                (const T*)c, (T*)a, nx, l->nG, l->nM);
+static int add_mma(const gb_lfc* l, const double* c, double* a, int64_t nx, cudaStream_t st) {
+  if (l->ns == 0) return GB_OK;
+  const dim3 grid((unsigned)((l->ns + LM_WARPS - 1) / LM_WARPS), (unsigned)((nx + 15) / 16));
+  auto kern = l->nf == 1 ? lfc_add_mma_kernel<1> : lfc_add_mma_kernel<2>;
+  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->ns, l->st_sub, l->st_M, l->st_A, c, a, nx, l->nG, l->nM);
   return check_launch("lfc_add_mma_kernel");
 }
-
-#define GB_LFC_NB(FN, ...)                                                    \
-  switch (mma_tiles(nx)) {                                                    \
-    case 1: return l->nf == 1 ? FN<T, 1, 1>(__VA_ARGS__) : FN<T, 1, 2>(__VA_ARGS__); \
-    case 2: return l->nf == 1 ? FN<T, 2, 1>(__VA_ARGS__) : FN<T, 2, 2>(__VA_ARGS__); \
-    case 3: return l->nf == 1 ? FN<T, 3, 1>(__VA_ARGS__) : FN<T, 3, 2>(__VA_ARGS__); \
-    case 4: return l->nf == 1 ? FN<T, 4, 1>(__VA_ARGS__) : FN<T, 4, 2>(__VA_ARGS__); \
-    default: return l->nf == 1 ? FN<T, 5, 1>(__VA_ARGS__) : FN<T, 5, 2>(__VA_ARGS__); \
-  }
-template <typename T>
-static int integrate_mma(const gb_lfc* l, const void* a, void* c, int64_t nx, cudaStream_t st) {
-  if (l->ngroups == 0) return GB_OK;
-  GB_LFC_NB(integrate_mma_nb, l, a, c, nx, st)
-}
-template <typename T>
-static int add_mma(const gb_lfc* l, const void* c, void* a, int64_t nx, cudaStream_t st) {
-  if (l->ns == 0) return GB_OK;
-  GB_LFC_NB(add_mma_nb, l, c, a, nx, st)
-}
-#undef GB_LFC_NB
 
 template <typename T, int NM>
 static int integrate_nm(const gb_lfc* l, int gbeg, int gcount, const void* a, void* c, int64_t nx, int q,
@@ -778,7 +719,7 @@ static int integrate_t(const gb_lfc* l, const void* a, void* c, int64_t nx, int 
       return integrate_tiles(l, static_cast<const float*>(a), static_cast<float*>(c), nx, st);
   }
   if constexpr (std::is_same<T, double>::value) {
-    if (mma_usable(l, nx)) return integrate_mma<T>(l, a, c, nx, st);
+    if (mma_usable(l, nx)) return integrate_mma(l, static_cast<const double*>(a), static_cast<double*>(c), nx, st);
   }
   // groups are sorted by nm on the host; one launch per padded class
   int g = 0;
@@ -1204,14 +1145,17 @@ static int add_t(const gb_lfc* l, const void* c, void* a, int64_t nx, int q, cud
     if (l->A32p) return add_bands(l, static_cast<const float*>(c), static_cast<float*>(a), nx, st);
   }
   if constexpr (std::is_same<T, double>::value) {
-    if (mma_usable(l, nx)) return add_mma<T>(l, c, a, nx, st);
+    // one grid (a density or potential) would fill one row of sixteen of every
+    // tile: 71^3, 24 atoms with 5 functions: 8.9 us, point by point 6.6
+    if (nx > 1 && mma_usable(l, nx)) return add_mma(l, static_cast<const double*>(c), static_cast<double*>(a), nx, st);
   }
+  constexpr int XB = std::is_same<T, double>::value ? 1 : 8;      // bands per thread
   switch (nm_class(l->maxnm)) {
-    case 1: return add_nm<T, 8, 1>(l, c, a, nx, q, st, per_q);
-    case 2: return add_nm<T, 8, 2>(l, c, a, nx, q, st, per_q);
-    case 4: return add_nm<T, 8, 4>(l, c, a, nx, q, st, per_q);
-    case 8: return add_nm<T, 8, 8>(l, c, a, nx, q, st, per_q);
-    case 16: return add_nm<T, 4, 16>(l, c, a, nx, q, st, per_q);
+    case 1: return add_nm<T, XB, 1>(l, c, a, nx, q, st, per_q);
+    case 2: return add_nm<T, XB, 2>(l, c, a, nx, q, st, per_q);
+    case 4: return add_nm<T, XB, 4>(l, c, a, nx, q, st, per_q);
+    case 8: return add_nm<T, XB, 8>(l, c, a, nx, q, st, per_q);
+    case 16: return add_nm<T, XB == 1 ? 1 : 4, 16>(l, c, a, nx, q, st, per_q);
     case 32: return add_nm<T, 2, 32>(l, c, a, nx, q, st, per_q);
     case 64: return add_nm<T, 1, 64>(l, c, a, nx, q, st, per_q);
     default: return fail(GB_E_UNSUPPORTED, "lfc: more than 64 functions in one volume");
@@ -1454,9 +1398,9 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     gr_voff.push_back((int)gv_W.size());
   }
   // entries of the tensor-core path, in the order of their sub-tiles
-  std::vector<int2> st_sub, st_M;
-  std::vector<int4> sg_e;
-  std::vector<int> st_eoff, sg_off;
+  std::vector<int2> st_M;
+  std::vector<int4> st_sub, sg_e;
+  std::vector<int> sg_off;
   std::vector<double> st_A;
   if (l->maxnm <= 16 && nW > 0) {
     l->nf = l->maxnm <= 8 ? 1 : 2;
@@ -1478,10 +1422,6 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     std::vector<std::vector<int4>> by_group(ngr);
     for (size_t e = 0; e < ents.size(); ++e) {
       const Ent& n = ents[e];
-      if (st_sub.empty() || st_sub.back().x != n.sub) {
-        st_sub.push_back(make_int2(n.sub, 0));
-        st_eoff.push_back((int)e);
-      }
       const int nm = nm_W[n.W];
       int cov = 0;
       double* blk = st_A.data() + e * (size_t)nblk;
@@ -1491,17 +1431,22 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
         const double* Ar = A_all + aoff[n.W] + (r - row0[n.W]) * nm;
         for (int m = 0; m < nm; ++m) blk[m * 8 + p] = Ar[m];
       }
-      st_sub.back().y |= cov;
       st_M.push_back(make_int2(M_W[n.W], nm | cov << 8));
+      if (e == 0 || ents[e - 1].sub != n.sub) {
+        st_sub.push_back(make_int4(n.sub, 0, (int)e, 0));
+        st_sub.push_back(make_int4(st_M[e].x, st_M[e].y, 0, 0));
+      }
+      int4& sub = st_sub[st_sub.size() - 2];
+      sub.y |= cov;
+      sub.w = (int)e + 1;
       by_group[vol_group[n.W]].push_back(make_int4((int)e, n.sub, cov, 0));
     }
-    st_eoff.push_back((int)ents.size());
     sg_off.push_back(0);
     for (int gi = 0; gi < ngr; ++gi) {
       sg_e.insert(sg_e.end(), by_group[gi].begin(), by_group[gi].end());
       sg_off.push_back((int)sg_e.size());
     }
-    l->ns = (int)st_sub.size();
+    l->ns = (int)st_sub.size() / 2;
   }
   // brick tiling for the FP32 real path
   std::vector<int> tch_c, tch_eoff, te_nm, te_slot, te_lst, te_info, tbr_ch0, tbr_pbase, tps_M, tps_nm, tps_eoff,
@@ -1655,7 +1600,7 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     }
   }
   if (ok && l->nf)
-    ok = upload(l, &l->st_sub, st_sub) && upload(l, &l->st_eoff, st_eoff) && upload(l, &l->st_M, st_M) &&
+    ok = upload(l, &l->st_sub, st_sub) && upload(l, &l->st_M, st_M) &&
          upload(l, &l->st_A, st_A) && upload(l, &l->sg_off, sg_off) && upload(l, &l->sg_e, sg_e);
   if (ok && tiled) {
     ok = upload(l, &l->tch_c, tch_c) && upload(l, &l->tch_eoff, tch_eoff) && upload(l, &l->te_info, te_info) &&

@@ -234,6 +234,11 @@ int gb_spline_to_grid(const gb_spline* s, const int64_t beg_c[3],
  * integrate: c_xM[x][M_W+m] += dv sum_G phase_qW a_xG[x][G] A_W[g][m]
  *            (accumulates, like the reference; callers zero c_xM)
  * q = -1 for real data / no Bloch phase.  Device arrays for a_xG / c_xM.
+ * A row's result has the same bits whatever other rows come with it, with one
+ * exception: FP64 real data of a single row are added to by another kernel
+ * than blocks of rows, whose sums may differ in the last bits.
+ * Non-finite values reach the sums they belong to and no others; in the
+ * chunk-tiled FP32 path below also those of their 8-point sub-tile.
  * ==================================================================== */
 typedef struct gb_lfc gb_lfc;
 int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W,

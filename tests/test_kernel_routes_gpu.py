@@ -55,3 +55,31 @@ def test_fp32_lfc_outside_the_bricks(N, pbc, ls, nx):
     lfc.add_M(one, c[nx - 1:].contiguous())
     assert torch.equal(one, b[nx - 1:])
     assert torch.equal(lfc.integrate(a[nx - 1:].contiguous(), {}), P[nx - 1:])
+
+
+@pytest.mark.parametrize('ls', [(0,), (0, 0, 1), (0, 1, 2)])
+@pytest.mark.parametrize('natoms', [1, 7])
+def test_fp64_lfc_of_one_grid_and_of_many(ls, natoms):
+    """Projections have the same bits for a band alone, in a block of 16 and
+    among 37; so has what add gives a block.  A single grid is added to by
+    another kernel: each sum of up to 7 x 9 products may then round
+    differently, by at most 64 ulp of the sum of their absolute values."""
+    gd, lfc = lfc_on(24, 0, natoms, ls)
+    g = torch.Generator(device='cuda').manual_seed(natoms)
+    a = torch.randn((37,) + tuple(gd.n_c), generator=g, device='cuda', dtype=torch.float64)
+    c = torch.randn((37, lfc.Mmax), generator=g, device='cuda', dtype=torch.float64)
+    P, b = lfc.integrate(a, {}), a.clone()
+    lfc.add_M(b, c)
+    Phi = gd.zeros(lfc.Mmax)
+    lfc.add_M(Phi, torch.eye(lfc.Mmax, dtype=torch.float64, device='cuda'))
+    size = a.abs() + torch.einsum('xM,Mijk->xijk', c.abs(), Phi.abs())
+    for x0, x1 in ((0, 1), (20, 21), (36, 37), (5, 21)):
+        part = a[x0:x1].clone()
+        names = kernels(lambda: lfc.integrate(part, {}))
+        assert any('lfc_integrate_mma_kernel' in k for k in names)
+        assert torch.equal(lfc.integrate(part, {}), P[x0:x1])
+        lfc.add_M(part, c[x0:x1].contiguous())
+        if x1 - x0 > 1:
+            assert torch.equal(part, b[x0:x1])
+        else:
+            assert ((part - b[x0:x1]).abs() <= 64 * 2.3e-16 * size[x0]).all()
