@@ -57,9 +57,9 @@ __device__ __forceinline__ int wrap_index(int i, int n) {
 
 // One term of the stencil, in the order and form of star_core.cuh: centre,
 // axis 0, axis 2, axis 1, offsets ascending; FP32 as differences, axes 0 and 2
-// in pairs of offsets.  A band's result is then the same, bit for bit, in this
-// kernel and in the row kernel, so it does not depend on how many bands a call
-// has.
+// in pairs of offsets, which symmetric stencils of radius 1 and 3 add before
+// they multiply.  A band's result is then the same, bit for bit, in this kernel
+// and in the row kernel, so it does not depend on how many bands a call has.
 template <typename T>
 __device__ __forceinline__ T star_term(T acc, typename Elem<T>::R c, T v, T xc) {
   return fmadd(acc, c, sizeof(typename Elem<T>::R) == 4 ? sub(v, xc) : v);
@@ -388,7 +388,8 @@ static int launch_star(const gb_operator* op, const void* in, void* out, int64_t
                                     std::min<int64_t>(a.n0, ceil_div((int64_t)sm_count() * 16, cols)));
   const unsigned blocks = (unsigned)(cols * a.chunks);
   const bool per = a.pbc0 || a.pbc1 || a.pbc2;
-  if constexpr (std::is_same<T, float>::value) {
+  // FP32: in pairs of offsets where the row kernel has that form too
+  if constexpr (std::is_same<T, float>::value && (H == 1 || H == 3)) {
     if (symmetric_stencil<float>(op)) {
       if (per) march_star_kernel<T, H, true, true><<<blocks, 256, 0, stream>>>(a);
       else march_star_kernel<T, H, false, true><<<blocks, 256, 0, stream>>>(a);

@@ -5,6 +5,8 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import bloch_phases
+
 pytestmark = pytest.mark.gpu
 
 
@@ -16,6 +18,44 @@ def kernels(f):
         f()
         torch.cuda.synchronize()
     return [e.key for e in prof.key_averages()]
+
+
+def stencil_on(n_c, pbc, kind, dtype):
+    """Laplace(gd, -1/2, n) for kind n, the derivative along axis 1 for 'g'."""
+    from gpaw_b200.fd_operators import Gradient, Laplace
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    N = np.array(n_c) + (1 - np.array(pbc))
+    gd = GridDescriptor(N, 0.3 * N, pbc)
+    c = complex if dtype.is_complex else float
+    return Gradient(gd, 1, 1.0, 3, c) if kind == 'g' else Laplace(gd, -0.5, kind, c)
+
+
+def phases_of(pbc, dtype, k=(0.13, -0.21, 0.37)):
+    return bloch_phases(pbc, k) if dtype.is_complex else None
+
+
+def randn(shape, dtype, seed=1):
+    g = torch.Generator(device='cuda').manual_seed(seed)
+    return torch.randn(shape, generator=g, device='cuda', dtype=dtype)
+
+
+@pytest.mark.parametrize('n_c,pbc,nb', [((24, 75, 75), (0, 0, 0), 48), ((30, 40, 77), (1, 1, 1), 48)])
+@pytest.mark.parametrize('kind', [1, 2, 3, 4, 'g'])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64, torch.complex64])
+def test_stencil_of_one_band_and_of_many(n_c, pbc, nb, kind, dtype):
+    """Odd rows: a batch takes the row kernel, a band alone the marching one,
+    and both give it the same bits."""
+    op = stencil_on(n_c, pbc, kind, dtype)
+    ph = phases_of(pbc, dtype)
+    x = randn((nb,) + n_c, dtype)
+    y, one = torch.empty_like(x), torch.empty_like(x[:1])
+    names = kernels(lambda: op.apply(x, y, ph))
+    rows = not (kind == 1 and dtype == torch.float32)
+    assert any(('rows_star_kernel' if rows else 'march_star_kernel') in k for k in names), names
+    assert any('march_star_kernel' in k for k in kernels(lambda: op.apply(x[:1], one, ph)))
+    for b in (0, nb // 2, nb - 1):
+        op.apply(x[b:b + 1], one, ph)
+        assert torch.equal(one, y[b:b + 1])
 
 
 def lfc_on(N, pbc, natoms, ls, seed=3):
