@@ -174,6 +174,9 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
   constexpr int VEC = VB / (int)sizeof(T);   // elements per vector access
   constexpr int HZ = ((H + VEC - 1) / VEC) * VEC;
   constexpr int NQ = 2 * H + 1;
+  // the epilogue's operands are on their way before the sums, except where the
+  // register queue leaves no room for them (radius 4: up to 296 bytes spilled)
+  constexpr bool EARLY = H < 4;
   static_assert(R2 % VEC == 0, "");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -310,13 +313,14 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
         if (cslot < 0) cslot += NS;
         T yv[R1][R2];
         R vv[R1][R2];
-        if (EPI && t >= 2 * H) {
+        auto fetch = [&]() {
 #pragma unroll
           for (int r = 0; r < R1; ++r) {
             if (EPI == 2) ld_run_if<T, R2>(yp + r * n2, yv[r], a.y && on[r]);
             ld_run_if<R, R2>(vp + r * n2, vv[r], a.vpot && on[r]);
           }
-        }
+        };
+        if (EPI && EARLY && t >= 2 * H) fetch();
         if (!mbar_wait(&full[slot], fph)) {
           raise_device_error(102);
           return;
@@ -349,6 +353,7 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
               },
               [](int, int, T v) { return v; });
           // epilogue + streaming stores
+          if (EPI && !EARLY) fetch();
 #pragma unroll
           for (int r = 0; r < R1; ++r) {
 #pragma unroll
@@ -588,43 +593,55 @@ static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int6
   return launch(choice);
 }
 
-// Instantiations: symmetric stencils of the radii the path uses (1 and 3: the
-// kinetic operators of the three multigrid levels) with each epilogue (none,
-// potential, general); first derivatives in FP32; everything else general.
+// Symmetric stencils (of radius 2 and 4 in FP32 only, where their taps cost
+// fewer instructions), first derivatives in FP32, and everything else; each
+// without an epilogue and with the general one, the kinetic operators of radius
+// 3 and 4 with the potential alone too.  Without the first of these plain calls of
+// radius 2 and 4 and the derivatives carried the epilogue's loads and registers
+// along: (160, 60^3) radius 4 in FP32 264 against 122 us, in FP64 213 against
+// 150; derivative in FP64 165 against 107 us.
+template <typename T, int H, int R2, int SYM>
+static int launch_tma(const gb_operator* op, const void* in, void* out, int64_t nin, cudaStream_t st,
+                      const Epilogue& ep) {
+  const int epi = ep.y || ep.alpha != 1.0 || ep.beta != 0.0 ? 2 : ep.vpot ? 1 : 0;
+  if constexpr (H == 1 && SYM == 1) {
+    if (epi < 2) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 1>(op, in, out, nin, st, ep);
+  } else {
+    if (epi == 0) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 0>(op, in, out, nin, st, ep);
+    if constexpr ((H == 3 && SYM == 1) || (H == 4 && SYM >= 0))
+      if (epi == 1) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 1>(op, in, out, nin, st, ep);
+  }
+  return launch_tma_cfg<T, H, 2, R2, 16, SYM, 2>(op, in, out, nin, st, ep);
+}
+
 template <typename T, int R2>
 static int dispatch_tma(const gb_operator* op, const void* in, void* out, int64_t nin, cudaStream_t st,
                         const Epilogue& ep) {
-  bool sym = true, anti = std::is_same<T, float>::value;
-  for (int c = 0; c < 3; ++c)
-    for (int k = 1; k <= HMAX; ++k) {
-      using R = typename Elem<T>::R;
-      const R p = (R)op->a[c][HMAX + k], m = (R)op->a[c][HMAX - k];
-      sym = sym && p == m;
-      anti = anti && p == -m;
-    }
-  const int epi = ep.y || ep.alpha != 1.0 || ep.beta != 0.0 ? 2 : ep.vpot ? 1 : 0;
-  if (sym && (op->H == 1 || op->H == 3)) {
-    if (op->H == 1)
-      return epi == 2 ? launch_tma_cfg<T, 1, 2, R2, 16, 1, 2>(op, in, out, nin, st, ep)
-                      : launch_tma_cfg<T, 1, 2, R2, 16, 1, 1>(op, in, out, nin, st, ep);
-    switch (epi) {
-      case 0: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 0>(op, in, out, nin, st, ep);
-      case 1: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 1>(op, in, out, nin, st, ep);
-      default: return launch_tma_cfg<T, 3, 2, R2, 16, 1, 2>(op, in, out, nin, st, ep);
-    }
+  using R = typename Elem<T>::R;
+  constexpr bool F32 = std::is_same<T, float>::value;
+  if (symmetric_stencil<R>(op)) {
+    if (op->H == 1) return launch_tma<T, 1, R2, 1>(op, in, out, nin, st, ep);
+    if (op->H == 3) return launch_tma<T, 3, R2, 1>(op, in, out, nin, st, ep);
+    if constexpr (F32)
+      return op->H == 2 ? launch_tma<T, 2, R2, 1>(op, in, out, nin, st, ep)
+                        : launch_tma<T, 4, R2, 1>(op, in, out, nin, st, ep);
   }
-  if constexpr (std::is_same<T, float>::value)
+  if constexpr (F32) {
+    bool anti = true;
+    for (int c = 0; c < 3; ++c)
+      for (int k = 1; k <= HMAX; ++k) anti = anti && (R)op->a[c][HMAX + k] == -(R)op->a[c][HMAX - k];
     if (anti) switch (op->H) {
-        case 1: return launch_tma_cfg<T, 1, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
-        case 2: return launch_tma_cfg<T, 2, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
-        case 3: return launch_tma_cfg<T, 3, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
-        default: return launch_tma_cfg<T, 4, 2, R2, 16, -1, 2>(op, in, out, nin, st, ep);
+        case 1: return launch_tma<T, 1, R2, -1>(op, in, out, nin, st, ep);
+        case 2: return launch_tma<T, 2, R2, -1>(op, in, out, nin, st, ep);
+        case 3: return launch_tma<T, 3, R2, -1>(op, in, out, nin, st, ep);
+        default: return launch_tma<T, 4, R2, -1>(op, in, out, nin, st, ep);
       }
+  }
   switch (op->H) {
-    case 1: return launch_tma_cfg<T, 1, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
-    case 2: return launch_tma_cfg<T, 2, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
-    case 3: return launch_tma_cfg<T, 3, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
-    default: return launch_tma_cfg<T, 4, 2, R2, 16, 0, 2>(op, in, out, nin, st, ep);
+    case 1: return launch_tma<T, 1, R2, 0>(op, in, out, nin, st, ep);
+    case 2: return launch_tma<T, 2, R2, 0>(op, in, out, nin, st, ep);
+    case 3: return launch_tma<T, 3, R2, 0>(op, in, out, nin, st, ep);
+    default: return launch_tma<T, 4, R2, 0>(op, in, out, nin, st, ep);
   }
 }
 

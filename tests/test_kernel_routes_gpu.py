@@ -58,6 +58,24 @@ def test_stencil_of_one_band_and_of_many(n_c, pbc, nb, kind, dtype):
         assert torch.equal(one, y[b:b + 1])
 
 
+@pytest.mark.parametrize('kind', [1, 2, 3, 4, 'g'])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64, torch.complex64, torch.complex128])
+def test_plain_stencils_carry_no_epilogue(kind, dtype):
+    """apply() runs a kernel without the general epilogue (last template
+    argument below 2), whatever the radius; a potential is added all the same."""
+    n_c, pbc = (20, 24, 32), (1, 0, 1)
+    op = stencil_on(n_c, pbc, kind, dtype)
+    ph = np.ones((3, 2), complex) if dtype.is_complex else None
+    x = randn((3,) + n_c, dtype)
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    names = [k for k in kernels(lambda: op.apply(x, y, ph)) if 'star_tma_kernel' in k]
+    assert names and not any(', 2>' in k for k in names), names
+    v = randn(n_c, x.real.dtype if dtype.is_complex else dtype, 2)
+    op.apply_potential(x, z, v, ph)
+    tol = 1e-12 if dtype in (torch.float64, torch.complex128) else 1e-5
+    assert (z - (y + v * x)).abs().max() < tol * y.abs().max()
+
+
 def lfc_on(N, pbc, natoms, ls, seed=3):
     from gpaw_b200.grid_descriptor import GridDescriptor
     from gpaw_b200.lfc import LFC
