@@ -342,7 +342,11 @@ static int dispatch_rows(const gb_operator* op, const void* in, void* out, int64
                          cudaStream_t st, const Epilogue& ep, int nk) {
   const bool sym = symmetric_stencil<typename Elem<T>::R>(op);
   const int epi = ep.y || ep.alpha != 1.0 || ep.beta != 0.0 ? 2 : ep.vpot ? 1 : 0;
-  if (std::is_same<T, float>::value && op->H == 1) return 1;   // faster marching (fd_stencil.cu)
+  // faster marching (fd_stencil.cu): 7-point FP32 stencils, and rows so short
+  // that a plane hardly fills a CTA (FP64, radius 1: 300 bands of 15^3 33 us
+  // here, 12 us there; radius 4: 160 bands of 25^3 52 and 35 us)
+  if (std::is_same<T, float>::value && op->H == 1) return 1;
+  if (sizeof(T) < 16 && op->n[2] < 28) return 1;
   if (sym && op->H == 1)
     return epi == 2 ? launch_rows<T, 1, 2, 1, 2>(op, in, out, nin, ph, st, ep, nk)
                     : launch_rows<T, 1, 2, 1, 1>(op, in, out, nin, ph, st, ep, nk);

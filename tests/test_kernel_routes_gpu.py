@@ -76,6 +76,21 @@ def test_plain_stencils_carry_no_epilogue(kind, dtype):
     assert (z - (y + v * x)).abs().max() < tol * y.abs().max()
 
 
+@pytest.mark.parametrize('n,pbc,kind,dtype', [(15, 0, 1, torch.float64), (19, 1, 1, torch.float64),
+                                              (25, 0, 4, torch.float64), (25, 1, 2, torch.complex64),
+                                              (27, 0, 4, torch.float32)])
+def test_short_rows_march(n, pbc, kind, dtype):
+    """Rows of fewer than 28 elements do not fill the row kernel's CTAs
+    (coarse multigrid levels), however many bands there are."""
+    op = stencil_on((n, n, n), (pbc,) * 3, kind, dtype)
+    ph = phases_of((pbc,) * 3, dtype)
+    x = randn((240, n, n, n), dtype)
+    y, one = torch.empty_like(x), torch.empty_like(x[:1])
+    assert any('march_star_kernel' in k for k in kernels(lambda: op.apply(x, y, ph)))
+    op.apply(x[77:78], one, ph)
+    assert torch.equal(one, y[77:78])
+
+
 def lfc_on(N, pbc, natoms, ls, seed=3):
     from gpaw_b200.grid_descriptor import GridDescriptor
     from gpaw_b200.lfc import LFC
