@@ -1,17 +1,22 @@
 // FD stencil operator (replaces _gpaw.Operator: c/operators.c, c/bmgs/fd.c,
 // c/bc.c).  Stencils whose points all lie on the three axes (the reference's
 // "cfd" case: Laplace on orthorhombic cells, Gradient) take, in this order,
-// the TMA kernel of fd_stencil_tma.cu, the row kernel of fd_stencil_rows.cu
-// and the kernel here:
+// the TMA kernel of fd_stencil_tma.cu, the row kernel of fd_stencil_rows.cu,
+// the tile kernel of fd_stencil_tiles.cu and the kernel here:
 //
 //  * march_star_kernel -- any layout, boundary mix, phases and radius up to 6.
 //    One thread per (axis1, axis2) column marches along axis 0 with a
 //    register queue; its in-plane neighbours are read through L1.  There is
 //    no staging and no barrier, so it is the fastest form while a call is too
-//    small to fill the pipelines of the other two (every SM busy for less
-//    than ~16 plane tiles), and with 7-point FP32 stencils, which read too
-//    few neighbours to be bound by L1 (four 31^3 FP64 grids 13 us against
-//    33 us in the row kernel; 160 x 37^3 FP32, radius 1: 33 against 37 us).
+//    small to fill the pipelines of the others (every SM busy for less than
+//    ~16 plane tiles of the row kernel), with 7-point FP32 stencils, which
+//    read too few neighbours to be bound by L1 (four 31^3 FP64 grids 13 us
+//    against 33 us in the row kernel; 160 x 37^3 FP32, radius 1: 33 against
+//    37 us), and on rows of fewer than 28 elements.  It also serves the rows
+//    that the row kernel's copies do not cover (launch_rows: four rows per warp
+//    and plane; radius 3: up to 34 FP64 or complex64 and 68 FP32 elements):
+//    160 FP64 bands of 31^3 43 us, 160 FP32 bands of 55^3 216 us, against 69
+//    and 279 us in the tile kernel (radius 3, zero boundary).
 //
 //  * box_kernel   -- any stencil (off-axis points of GUC Laplacians /
 //    non-orthogonal gradients, c/bmgs/fd.c generic loop).  3-D tile with a
@@ -464,8 +469,9 @@ int op_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int 
     if (rc != 1) return rc;
     if (stencil_path() == 2)
       return fail(GB_E_UNSUPPORTED, std::string("TMA stencil path required but not applicable: ") + tma_reason());
-    const int rr = star_rows_apply(op, in, out, nin, dtype, ph, st, ep, nk);
-    if (rr != 1) return rr;
+    int rr = star_rows_apply(op, in, out, nin, dtype, ph, st, ep, nk);
+    if (rr == USE_TILES) rr = star_tiles_apply(op, in, out, nin, dtype, ph, st, ep, nk);
+    if (rr != USE_MARCH) return rr;
     switch (dtype) {
       case GB_DTYPE_F64: return dispatch_star<double>(op, in, out, nin, ph, st, ep, nk);
       case GB_DTYPE_F32: return dispatch_star<float>(op, in, out, nin, ph, st, ep, nk);

@@ -273,6 +273,10 @@ __global__ void __launch_bounds__(ROWS_NT, 2) rows_star_kernel(const __grid_cons
         case 6: if constexpr (NQ > 5) turn_of(std::integral_constant<int, 6 % NQ>{}); break;
         case 7: if constexpr (NQ > 7) turn_of(std::integral_constant<int, 7 % NQ>{}); break;
         case 8: if constexpr (NQ > 7) turn_of(std::integral_constant<int, 8 % NQ>{}); break;
+        case 9: if constexpr (NQ > 9) turn_of(std::integral_constant<int, 9 % NQ>{}); break;
+        case 10: if constexpr (NQ > 9) turn_of(std::integral_constant<int, 10 % NQ>{}); break;
+        case 11: if constexpr (NQ > 11) turn_of(std::integral_constant<int, 11 % NQ>{}); break;
+        case 12: if constexpr (NQ > 11) turn_of(std::integral_constant<int, 12 % NQ>{}); break;
       }
       if (++turn == NQ) turn = 0;
       if (++slot == NS) slot = 0;
@@ -291,7 +295,7 @@ static int launch_rows(const gb_operator* op, const void* in, void* out, int64_t
   static int regs = -1;
   if (regs < 0) {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return 1;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return USE_MARCH;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     regs = fa.numRegs;
   }
@@ -316,7 +320,26 @@ static int launch_rows(const gb_operator* op, const void* in, void* out, int64_t
     const double score = cw * eff * (ctas > 1 ? 1.0 : 0.7);
     if (score > best) { best = score; bctas = ctas; bty = ty; }
   }
-  if (!bty) return 1;
+  // No tile: rows too short for the copies of a warp (four rows per plane).
+  if (!bty && a.TZ <= 64) return USE_MARCH;
+  // Rows so long that a tile holds few of them, or none: most of what is staged
+  // is halo.  The marching kernel takes over at radius 3 and 4 without wrapped
+  // halos (radius 3, 40 bands of 24 x 25 x 301 where five warps are left per SM:
+  // FP64 119 against 95 us, complex64 148 against 99), in FP32 at radius 5 and 6
+  // too (40 bands of 12 x 13 x 701, periodic: 150 us, 290 in the tile kernel)
+  // and, at any height, complex128 of radius 5 and 6 (160 bands of 44^3 523
+  // against 398 us); the tile kernel the rest (radius 4, 40 periodic complex128 bands of 64 x 64 x
+  // 131: 1454 against 521 us; radius 6, 40 FP64 bands of 96^3, five rows per
+  // tile, zero boundary: 548 against 449).
+  constexpr bool F32 = std::is_same<T, float>::value, C128 = sizeof(T) == 16;
+  const bool per = a.pbc0 || a.pbc1 || a.pbc2;
+  const int T1 = bty * R1, warps = bctas * ((bty * a.TZ + 31) / 32);
+  if (H >= 5) {
+    if (C128 && !per) return USE_MARCH;
+    if (T1 < 3 || (T1 < 6 && !per && !F32)) return F32 ? USE_MARCH : USE_TILES;
+  }
+  if (H == 4 && T1 < (F32 && per ? 2 : 3)) return per ? USE_TILES : USE_MARCH;
+  if (!bty || (H == 3 && bty == 1 && !per && (C128 || warps < 8))) return USE_MARCH;
   a.NTC = bty * a.TZ; a.T1 = bty * R1; a.ROWS = a.T1 + 2 * H;
   a.ytiles = ceil_div(a.n1, a.T1);
   a.c0 = op->center;
@@ -330,7 +353,7 @@ static int launch_rows(const gb_operator* op, const void* in, void* out, int64_t
   const size_t smem = (size_t)C::NS * a.ROWS * a.pitch * sizeof(T);
   const int64_t total = nin * (int64_t)a.ytiles * a.n0;
   // too few plane tiles to fill the pipelines: the marching kernel
-  if (total < 16 * sm_count()) return 1;
+  if (total < 16 * sm_count()) return USE_MARCH;
   int64_t blocks = (int64_t)sm_count() * bctas;
   blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, total / (H + 1)));
   kern<<<(unsigned)blocks, threads, smem, st>>>(a);
@@ -345,8 +368,8 @@ static int dispatch_rows(const gb_operator* op, const void* in, void* out, int64
   // faster marching (fd_stencil.cu): 7-point FP32 stencils, and rows so short
   // that a plane hardly fills a CTA (FP64, radius 1: 300 bands of 15^3 33 us
   // here, 12 us there; radius 4: 160 bands of 25^3 52 and 35 us)
-  if (std::is_same<T, float>::value && op->H == 1) return 1;
-  if (sizeof(T) < 16 && op->n[2] < 28) return 1;
+  if (std::is_same<T, float>::value && op->H == 1) return USE_MARCH;
+  if (sizeof(T) < 16 && op->n[2] < 28) return USE_MARCH;
   if (sym && op->H == 1)
     return epi == 2 ? launch_rows<T, 1, 2, 1, 2>(op, in, out, nin, ph, st, ep, nk)
                     : launch_rows<T, 1, 2, 1, 1>(op, in, out, nin, ph, st, ep, nk);
@@ -360,13 +383,21 @@ static int dispatch_rows(const gb_operator* op, const void* in, void* out, int64
     case 2: return launch_rows<T, 2, 2, 0, 2>(op, in, out, nin, ph, st, ep, nk);
     case 3: return launch_rows<T, 3, 2, 0, 2>(op, in, out, nin, ph, st, ep, nk);
     case 4: return launch_rows<T, 4, 1, 0, 2>(op, in, out, nin, ph, st, ep, nk);
-    default: return 1;
+    // 160 periodic bands of 56^3, marching against here: FP64 1646 -> 410 us,
+    // FP32 1083 -> 293 (radius 6)
+    case 5:
+      return epi ? launch_rows<T, 5, 1, 0, 2>(op, in, out, nin, ph, st, ep, nk)
+                 : launch_rows<T, 5, 1, 0, 0>(op, in, out, nin, ph, st, ep, nk);
+    case 6:
+      return epi ? launch_rows<T, 6, 1, 0, 2>(op, in, out, nin, ph, st, ep, nk)
+                 : launch_rows<T, 6, 1, 0, 0>(op, in, out, nin, ph, st, ep, nk);
+    default: return USE_MARCH;
   }
 }
 
 int star_rows_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype, const double* ph,
                     cudaStream_t st, const Epilogue& ep, int nk) {
-  if (op->n[1] * op->n[2] >= (1LL << 31)) return 1;
+  if (op->n[1] * op->n[2] >= (1LL << 31)) return USE_MARCH;
   switch (dtype) {
     case GB_DTYPE_F64: return dispatch_rows<double>(op, in, out, nin, ph, st, ep, nk);
     case GB_DTYPE_F32: return dispatch_rows<float>(op, in, out, nin, ph, st, ep, nk);

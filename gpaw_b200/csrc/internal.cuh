@@ -4,7 +4,7 @@
 #include "common.cuh"
 
 namespace gb {
-static constexpr int HMAX = 6;   // largest axis radius handled by star_kernel
+static constexpr int HMAX = 6;   // largest axis radius of a stencil
 
 // Bloch phases: a launch covers nk equal groups of bands (k-points), each
 // with its own phase_cd set; ph[k][axis][side][re/im].  Kernels pick the
@@ -102,9 +102,14 @@ int tr_apply(const gb_transformer* t, const void* in, void* out, int64_t nin, in
 // TMA stencil path: returns 1 when the request is not eligible (caller falls back)
 int star_tma_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype,
                    const double* ph, cudaStream_t st, const Epilogue& ep, int nk = 1);
-// row kernel for the layouts the TMA path does not take; returns 1 likewise
+// row kernel for the layouts the TMA path does not take; USE_MARCH or USE_TILES
+// where another kernel is faster
+constexpr int USE_MARCH = 1, USE_TILES = 2;
 int star_rows_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype,
                     const double* ph, cudaStream_t st, const Epilogue& ep, int nk = 1);
+// tile kernel for radius 4 to 6; returns USE_MARCH while a call is too small for it
+int star_tiles_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype,
+                     const double* ph, cudaStream_t st, const Epilogue& ep, int nk = 1);
 void set_stencil_path(int mode);
 const char* tma_reason();
 int stencil_path();

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import bloch_phases
+from conftest import bloch_phases, relerr
+from oracle import fd
 
 pytestmark = pytest.mark.gpu
 
@@ -89,6 +90,46 @@ def test_short_rows_march(n, pbc, kind, dtype):
     assert any('march_star_kernel' in k for k in kernels(lambda: op.apply(x, y, ph)))
     op.apply(x[77:78], one, ph)
     assert torch.equal(one, y[77:78])
+
+
+@pytest.mark.parametrize('n_c,pbc,nb,kind,dtype,kernel', [
+    ((56, 56, 56), (1, 1, 1), 60, 6, torch.float64, 'rows'),      # radius 5 and 6
+    ((45, 52, 61), (0, 1, 0), 60, 6, torch.float32, 'rows'),
+    ((40, 47, 50), (1, 1, 1), 60, 5, torch.complex64, 'rows'),
+    ((40, 41, 43), (1, 0, 1), 60, 6, torch.complex128, 'rows'),
+    ((40, 96, 96), (0, 0, 0), 30, 6, torch.float64, 'tile'),      # few rows per tile
+    ((30, 40, 257), (1, 0, 1), 30, 5, torch.float64, 'tile'),
+    ((24, 25, 301), (1, 1, 1), 30, 6, torch.complex64, 'tile'),
+    ((20, 20, 450), (1, 1, 1), 30, 6, torch.float32, 'march'),
+    ((44, 44, 44), (0, 0, 0), 60, 6, torch.complex128, 'march'),
+    ((24, 24, 24), (1, 1, 1), 10, 6, torch.float64, 'march'),     # a small call
+    ((30, 33, 131), (1, 1, 1), 40, 4, torch.complex128, 'tile'),  # one row per tile, wrapped
+    ((30, 33, 131), (0, 0, 0), 40, 4, torch.complex128, 'march'),
+    ((24, 25, 301), (0, 0, 0), 40, 3, torch.float64, 'march'),
+    ((24, 25, 301), (1, 1, 1), 40, 3, torch.float64, 'rows'),
+])
+def test_large_radius_and_long_rows(n_c, pbc, nb, kind, dtype, kernel):
+    """Radius 5 and 6 and rows of which a tile holds few: the kernel that is
+    the fastest there, the oracle's values with and without a
+    potential, and the bits of a band alone."""
+    op = stencil_on(n_c, pbc, kind, dtype)
+    ph = phases_of(pbc, dtype)
+    x = randn((nb,) + n_c, dtype)
+    y, z, one = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x[:1])
+    names = kernels(lambda: op.apply(x, y, ph))
+    assert any(f'{kernel}_star_kernel' in k for k in names), names
+    v = randn(n_c, x.real.dtype if dtype.is_complex else dtype, 2)
+    op.apply_potential(x, z, v, ph)
+    wide = np.complex128 if dtype.is_complex else np.float64
+    tol = 1e-12 if dtype in (torch.float64, torch.complex128) else 1e-5
+    for b in (0, nb - 1):
+        h = x[b].cpu().numpy().astype(wide)[None]
+        ref = fd.fd_apply(op.coef_p, op.offset_pc, h, pbc, ph)
+        assert relerr(y[b:b + 1].cpu().numpy(), ref) < tol
+        assert relerr(z[b:b + 1].cpu().numpy(), ref + v.cpu().numpy() * h) < tol
+    for b in (0, nb // 2):
+        op.apply(x[b:b + 1], one, ph)
+        assert torch.equal(one, y[b:b + 1])
 
 
 def lfc_on(N, pbc, natoms, ls, seed=3):
