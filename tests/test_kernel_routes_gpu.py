@@ -197,3 +197,27 @@ def test_fp64_lfc_of_one_grid_and_of_many(ls, natoms):
             assert torch.equal(part, b[x0:x1])
         else:
             assert ((part - b[x0:x1]).abs() <= 64 * 2.3e-16 * size[x0]).all()
+
+
+@pytest.mark.parametrize('nn', [2, 3, 4])
+@pytest.mark.parametrize('n0,pbc', [(16, (1, 1, 1)), (20, (0, 1, 0)), (28, (1, 0, 1)), (36, (0, 0, 0))])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64, torch.complex64, torch.complex128])
+def test_interpolation_takes_several_planes(nn, n0, pbc, dtype):
+    """A block interpolates four coarse planes (eight in FP32), so that a
+    plane is read about twice and not once per tap; plane counts around those
+    blocks against the oracle."""
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    from gpaw_b200.transformers import Transformer
+    N = np.array((n0, 20, 44))
+    gf = GridDescriptor(N, 0.3 * N, pbc)
+    gc = gf.coarsen()
+    t = Transformer(gc, gf, nn, complex if dtype.is_complex else float)
+    ph = phases_of(pbc, dtype)
+    x = randn((3,) + tuple(gc.n_c), dtype)
+    names = kernels(lambda: t.apply(x, None, ph))
+    planes = 8 if dtype == torch.float32 else 4
+    assert any(f', {2 * nn}, {planes}, 16' in k for k in names if 'interpolate_x_kernel' in k), names
+    h = x.cpu().numpy().astype(np.complex128 if dtype.is_complex else np.float64)
+    ref = fd.Transformer(*[fd.Grid(d.N_c, d.cell_cv, d.pbc_c) for d in (gc, gf)], nn).apply(h, ph)
+    tol = 1e-12 if dtype in (torch.float64, torch.complex128) else 1e-5
+    assert relerr(t.apply(x, None, ph).cpu().numpy(), ref) < tol
