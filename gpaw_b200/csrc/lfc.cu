@@ -66,13 +66,13 @@ struct gb_lfc {
   std::vector<int> h_gr_nm;
   // tensor-core add / integrate for FP64 real data (every volume has <= 16
   // functions): one entry per (volume, 8-point sub-tile of the flattened grid
-  // it touches) with its values there as nf dense [m][p] 8 x 8 blocks
-  int nf = 0;                 // 1 or 2 blocks per entry; 0 = not built
+  // it touches) with its values there as maxnm dense rows [m][p]
+  int nf = 0;                 // blocks of 8 functions per entry, 1 or 2; 0 = not built
   int ns = 0;                 // sub-tiles with entries
   int4* st_sub = nullptr;     // [ns][2] sub-tile | mask of its covered points | its entries' range,
                               //   then the first entry's st_M
   int2* st_M = nullptr;       // [ne] first function | function count + covered points << 8 of an entry
-  double* st_A = nullptr;     // [ne][nf][8][8]
+  double* st_A = nullptr;     // [ne][maxnm][8]
   int* sg_off = nullptr;      // [ngroups + 1] entries of each function group:
   int4* sg_e = nullptr;       //   entry | sub-tile | covered points, in the order of the sub-tiles
   // brick-tiled FP32 add / integrate for real data (every volume has <= 8
@@ -526,9 +526,9 @@ static __global__ void lfc_pad_rows_kernel(const double* __restrict__ A, const i
 // its sums; in the loop over the stores each load waited for the store before
 // it.  Inputs from HBM, 71^3 points, radius 2.1 A, point-major kernels (gathered
 // rows, one point per thread) against these:
-//   24 atoms x 9 functions, 96 bands:  integrate 127 ->  75 us, add 174 ->  76 us
-//   24 atoms x 5 functions, 160 bands: integrate 120 ->  77 us, add 169 ->  89 us
-//    4 atoms x 9 functions, 32 bands:  integrate  64 ->  36 us, add  22 ->  13 us
+//   24 atoms x 9 functions, 96 bands:  integrate 127 ->  80 us, add 174 ->  76 us
+//   24 atoms x 5 functions, 160 bands: integrate 120 ->  78 us, add 169 ->  96 us
+//    4 atoms x 9 functions, 160 bands: integrate  66 ->  40 us, add  77 ->  31 us
 __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
@@ -543,7 +543,7 @@ constexpr int LM_WARPS = 8;
 template <int NF>
 __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WARPS)
     lfc_integrate_mma_kernel(const int* __restrict__ sg_off, const int4* __restrict__ sg_e,
-                             const double* __restrict__ st_A, const int* __restrict__ gr_M,
+                             const double* __restrict__ st_A, int nr, const int* __restrict__ gr_M,
                              const int* __restrict__ gr_nm, const double* __restrict__ a_xG,
                              double* __restrict__ c_xM, int64_t nx, int64_t nG, int nM, double dv) {
   constexpr int NE = NF * 128;
@@ -573,7 +573,7 @@ __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WAR
     const int4 es = __ldg(sg_e + q);
     const int64_t p = (int64_t)es.y * 8;
     const bool in0 = es.z >> t & 1, in1 = es.z >> t & 16;
-    const double* blk = st_A + (int64_t)es.x * (NF * 64) + g * 8 + t;
+    const double* blk = st_A + ((int64_t)es.x * nr + g) * 8 + t;
     double av[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -581,7 +581,10 @@ __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WAR
       av[2 + h] = on[h] && in1 ? __ldg(row[h] + p + 4) : 0.0;
     }
 #pragma unroll
-    for (int f = 0; f < NF; ++f) mma_f64(acc[f], av, __ldg(blk + f * 64), __ldg(blk + f * 64 + 4));
+    for (int f = 0; f < NF; ++f) {
+      const bool in = f * 8 + g < nr;
+      mma_f64(acc[f], av, in ? __ldg(blk + f * 64) : 0.0, in ? __ldg(blk + f * 64 + 4) : 0.0);
+    }
   }
 #pragma unroll
   for (int f = 0; f < NF; ++f)
@@ -615,8 +618,8 @@ __global__ void __cluster_dims__(LM_CLUSTER, 1, 1) __launch_bounds__(32 * LM_WAR
 template <int NF>
 __global__ void __launch_bounds__(32 * LM_WARPS)
     lfc_add_mma_kernel(int ns, const int4* __restrict__ st_sub, const int2* __restrict__ st_M,
-                       const double* __restrict__ st_A, const double* __restrict__ c_xM, double* __restrict__ a_xG,
-                       int64_t nx, int64_t nG, int nM) {
+                       const double* __restrict__ st_A, int nr, const double* __restrict__ c_xM,
+                       double* __restrict__ a_xG, int64_t nx, int64_t nG, int nM) {
   const int s = blockIdx.x * LM_WARPS + (threadIdx.x >> 5);
   if (s >= ns) return;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -646,7 +649,7 @@ __global__ void __launch_bounds__(32 * LM_WARPS)
     double d[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-      const double* blk = st_A + ((int64_t)e * NF + f) * 64 + t * 8 + g;
+      const double* blk = st_A + ((int64_t)e * nr + f * 8 + t) * 8 + g;
       const bool in0 = f * 8 + t < nm, in1 = f * 8 + t + 4 < nm;
       double cv[4];
 #pragma unroll
@@ -655,7 +658,7 @@ __global__ void __launch_bounds__(32 * LM_WARPS)
         cv[h] = on[h] && in0 ? __ldg(c) : 0.0;
         cv[2 + h] = on[h] && in1 ? __ldg(c + 4) : 0.0;
       }
-      mma_f64(d, cv, __ldg(blk), __ldg(blk + 32));
+      mma_f64(d, cv, in0 ? __ldg(blk) : 0.0, in1 ? __ldg(blk + 32) : 0.0);
     }
     if (e + 1 < sub.w) mn = __ldg(st_M + e + 1);
 #pragma unroll
@@ -667,6 +670,19 @@ __global__ void __launch_bounds__(32 * LM_WARPS)
     if (wr[k]) ap[8 * (k >> 1) * nG + (k & 1)] = old[k] + acc[k];
 }
 
+// st_A[e][m][p]: the rows of an entry are the points it covers, in order;
+// ent_a is the offset of the first one in A
+static __global__ void lfc_blocks_kernel(const double* __restrict__ A, const int64_t* __restrict__ ent_a,
+                                         const int2* __restrict__ st_M, int64_t ne, int nr, double* __restrict__ st_A) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ne * nr * 8;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e = i / (nr * 8);
+    const int m = (int)(i / 8 % nr), p = (int)(i & 7);
+    const int nm = st_M[e].y & 255, cov = st_M[e].y >> 8;
+    st_A[i] = m < nm && (cov >> p & 1) ? A[ent_a[e] + __popc(cov & ((1 << p) - 1)) * nm + m] : 0.0;
+  }
+}
+
 // the launch grid's second dimension bounds the bands
 static bool mma_usable(const gb_lfc* l, int64_t nx) { return l->nf && nx <= 65535 * 16; }
 
@@ -674,7 +690,8 @@ static int integrate_mma(const gb_lfc* l, const double* a, double* c, int64_t nx
   if (l->ngroups == 0) return GB_OK;
   const dim3 grid((unsigned)(l->ngroups * LM_CLUSTER), (unsigned)((nx + 15) / 16));
   auto kern = l->nf == 1 ? lfc_integrate_mma_kernel<1> : lfc_integrate_mma_kernel<2>;
-  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->sg_off, l->sg_e, l->st_A, l->gr_M, l->gr_nm, a, c, nx, l->nG, l->nM, l->dv);
+  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->sg_off, l->sg_e, l->st_A, l->maxnm, l->gr_M, l->gr_nm, a, c, nx, l->nG, l->nM,
+                                       l->dv);
   return check_launch("lfc_integrate_mma_kernel");
 }
 
@@ -682,7 +699,7 @@ static int add_mma(const gb_lfc* l, const double* c, double* a, int64_t nx, cuda
   if (l->ns == 0) return GB_OK;
   const dim3 grid((unsigned)((l->ns + LM_WARPS - 1) / LM_WARPS), (unsigned)((nx + 15) / 16));
   auto kern = l->nf == 1 ? lfc_add_mma_kernel<1> : lfc_add_mma_kernel<2>;
-  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->ns, l->st_sub, l->st_M, l->st_A, c, a, nx, l->nG, l->nM);
+  kern<<<grid, 32 * LM_WARPS, 0, st>>>(l->ns, l->st_sub, l->st_M, l->st_A, l->maxnm, c, a, nx, l->nG, l->nM);
   return check_launch("lfc_add_mma_kernel");
 }
 
@@ -1397,54 +1414,53 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
     for (int W : kv.second) gv_W.push_back(W);
     gr_voff.push_back((int)gv_W.size());
   }
-  // entries of the tensor-core path, in the order of their sub-tiles
+  // entries of the tensor-core path, in the order of their sub-tiles: a volume
+  // meets its sub-tiles in order, so that placing the volumes one after the
+  // other by counted sub-tiles sorts the entries by (sub-tile, volume)
   std::vector<int2> st_M;
   std::vector<int4> st_sub, sg_e;
   std::vector<int> sg_off;
-  std::vector<double> st_A;
+  std::vector<int64_t> ent_a;
   if (l->maxnm <= 16 && nW > 0) {
     l->nf = l->maxnm <= 8 ? 1 : 2;
-    const int nblk = l->nf * 64, ngr = (int)gr_M.size();
-    std::vector<int> vol_group(nW);
+    const int ngr = (int)gr_M.size();
+    std::vector<int> at((size_t)(nG + 7) / 8 + 1, 0), ent_sub, ent_W;
+    for (int W = 0; W < nW; ++W)
+      for (int64_t r = row0[W]; r < row0[W + 1]; ++r)
+        if (r == row0[W] || row_G[r] / 8 != row_G[r - 1] / 8) ++at[row_G[r] / 8 + 1];
+    for (size_t i = 1; i < at.size(); ++i) at[i] += at[i - 1];
+    const int ne = at.back();
+    st_M.resize(ne);
+    ent_a.resize(ne);
+    ent_sub.resize(ne);
+    ent_W.resize(ne);
+    for (int W = 0; W < nW; ++W)
+      for (int64_t r = row0[W]; r < row0[W + 1];) {
+        const int sub = row_G[r] / 8, e = at[sub]++;
+        ent_sub[e] = sub;
+        ent_W[e] = W;
+        ent_a[e] = aoff[W] + (r - row0[W]) * nm_W[W];
+        int cov = 0;
+        for (; r < row0[W + 1] && row_G[r] / 8 == sub; ++r) cov |= 1 << row_G[r] % 8;
+        st_M[e] = make_int2(M_W[W], nm_W[W] | cov << 8);
+      }
+    std::vector<int> vol_group(nW), gat(ngr + 1, 0);
     for (int gi = 0; gi < ngr; ++gi)
       for (int v = gr_voff[gi]; v < gr_voff[gi + 1]; ++v) vol_group[gv_W[v]] = gi;
-    struct Ent { int sub, W; int64_t r0, r1; };          // rows of W in the sub-tile
-    std::vector<Ent> ents;
-    for (int W = 0; W < nW; ++W)
-      for (int64_t r = row0[W]; r < row0[W + 1]; ++r) {
-        const int sub = row_G[r] / 8;
-        if (r == row0[W] || sub != ents.back().sub) ents.push_back({sub, W, r, r});
-        ents.back().r1 = r + 1;
-      }
-    std::sort(ents.begin(), ents.end(),
-              [](const Ent& x, const Ent& y) { return x.sub != y.sub ? x.sub < y.sub : x.W < y.W; });
-    st_A.assign(ents.size() * (size_t)nblk, 0.0);
-    std::vector<std::vector<int4>> by_group(ngr);
-    for (size_t e = 0; e < ents.size(); ++e) {
-      const Ent& n = ents[e];
-      const int nm = nm_W[n.W];
-      int cov = 0;
-      double* blk = st_A.data() + e * (size_t)nblk;
-      for (int64_t r = n.r0; r < n.r1; ++r) {
-        const int p = row_G[r] % 8;
-        cov |= 1 << p;
-        const double* Ar = A_all + aoff[n.W] + (r - row0[n.W]) * nm;
-        for (int m = 0; m < nm; ++m) blk[m * 8 + p] = Ar[m];
-      }
-      st_M.push_back(make_int2(M_W[n.W], nm | cov << 8));
-      if (e == 0 || ents[e - 1].sub != n.sub) {
-        st_sub.push_back(make_int4(n.sub, 0, (int)e, 0));
+    for (int e = 0; e < ne; ++e) ++gat[vol_group[ent_W[e]] + 1];
+    for (int gi = 0; gi < ngr; ++gi) gat[gi + 1] += gat[gi];
+    sg_off = gat;
+    sg_e.resize(ne);
+    for (int e = 0; e < ne; ++e) {
+      const int cov = st_M[e].y >> 8;
+      if (e == 0 || ent_sub[e] != ent_sub[e - 1]) {
+        st_sub.push_back(make_int4(ent_sub[e], 0, e, 0));
         st_sub.push_back(make_int4(st_M[e].x, st_M[e].y, 0, 0));
       }
       int4& sub = st_sub[st_sub.size() - 2];
       sub.y |= cov;
-      sub.w = (int)e + 1;
-      by_group[vol_group[n.W]].push_back(make_int4((int)e, n.sub, cov, 0));
-    }
-    sg_off.push_back(0);
-    for (int gi = 0; gi < ngr; ++gi) {
-      sg_e.insert(sg_e.end(), by_group[gi].begin(), by_group[gi].end());
-      sg_off.push_back((int)sg_e.size());
+      sub.w = e + 1;
+      sg_e[gat[vol_group[ent_W[e]]]++] = make_int4(e, ent_sub[e], cov, 0);
     }
     l->ns = (int)st_sub.size() / 2;
   }
@@ -1599,9 +1615,23 @@ int gb_lfc_new(int nW, const double* A_all, const int64_t* ngm_W, const int* nm_
       ok = cudaDeviceSynchronize() == cudaSuccess;
     }
   }
-  if (ok && l->nf)
-    ok = upload(l, &l->st_sub, st_sub) && upload(l, &l->st_M, st_M) &&
-         upload(l, &l->st_A, st_A) && upload(l, &l->sg_off, sg_off) && upload(l, &l->sg_e, sg_e);
+  if (ok && l->nf) {
+    const int64_t ne = (int64_t)st_M.size();
+    ok = upload(l, &l->st_sub, st_sub) && upload(l, &l->st_M, st_M) && upload(l, &l->sg_off, sg_off) &&
+         upload(l, &l->sg_e, sg_e);
+    l->st_A = ok ? dalloc<double>(l, ne * l->maxnm * 8) : nullptr;
+    int64_t* d_a = nullptr;
+    ok = l->st_A && cudaMalloc(&d_a, std::max<size_t>(1, ne) * sizeof(int64_t)) == cudaSuccess;
+    if (ok && ne) {
+      ok = cudaMemcpy(d_a, ent_a.data(), ne * sizeof(int64_t), cudaMemcpyHostToDevice) == cudaSuccess;
+      if (ok) {
+        lfc_blocks_kernel<<<(unsigned)std::min<int64_t>((ne * l->maxnm * 8 + 255) / 256, 16384), 256>>>(
+            l->A64, d_a, l->st_M, ne, l->maxnm, l->st_A);
+        ok = cudaDeviceSynchronize() == cudaSuccess;
+      }
+    }
+    cudaFree(d_a);
+  }
   if (ok && tiled) {
     ok = upload(l, &l->tch_c, tch_c) && upload(l, &l->tch_eoff, tch_eoff) && upload(l, &l->te_info, te_info) &&
          upload(l, &l->te_A, te_A) && upload(l, &l->tbr_ch0, tbr_ch0) && upload(l, &l->tbr_pbase, tbr_pbase) &&

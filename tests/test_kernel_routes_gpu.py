@@ -221,3 +221,27 @@ def test_interpolation_takes_several_planes(nn, n0, pbc, dtype):
     ref = fd.Transformer(*[fd.Grid(d.N_c, d.cell_cv, d.pbc_c) for d in (gc, gf)], nn).apply(h, ph)
     tol = 1e-12 if dtype in (torch.float64, torch.complex128) else 1e-5
     assert relerr(t.apply(x, None, ph).cpu().numpy(), ref) < tol
+
+
+def test_lfc_object_size():
+    """An object of one function per atom (a local potential, an ion charge)
+    keeps about 95 bytes on the device per covered point and atom: 8 + 4 of
+    values, 30 of indices, 32 of padded FP32 rows, and 8-point blocks with as
+    many rows as there are functions; 20 allocations may round up by 2 MB."""
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    from gpaw_b200.lfc import LFC
+    from gpaw_b200.spline import Spline
+    rc = 3.6
+    spl = Spline.from_data(0, rc, np.exp(-np.linspace(0, rc, 41)**2))
+    gd = GridDescriptor((96, 96, 96), (96 * 0.19,) * 3, True)
+    lfc = LFC(gd, [[spl]] * 40, cut=True)
+    lfc.set_positions(np.random.default_rng(2).random((40, 3)))
+    rows = int(lfc.lfc.ngm.sum())
+    del lfc.lfc
+    lfc.my_atom_indices = None
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    lfc.set_positions(np.random.default_rng(2).random((40, 3)))
+    torch.cuda.synchronize()
+    assert rows > 5e5
+    assert before - torch.cuda.mem_get_info()[0] < 97 * rows + 20 * 2**21
