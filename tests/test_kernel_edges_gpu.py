@@ -18,21 +18,28 @@ TOL = {torch.float64: 1e-12, torch.complex128: 1e-12,
        torch.float32: 1e-5, torch.complex64: 1e-5}
 
 
-@pytest.mark.parametrize('n_c,pbc,nb', [
-    ((31, 31, 31), (0, 0, 0), 48),       # odd rows, several row tiles, zero boundaries
-    ((24, 75, 75), (0, 0, 0), 32),       # a last row tile of few rows
-    ((40, 7, 33), (1, 0, 1), 80),        # one tile, fewer rows than a tile
-    ((20, 29, 98), (0, 1, 0), 64),       # rows of more than three warps
-    ((17, 36, 21), (1, 1, 1), 96),       # odd rows with wrapped halo columns
+ROWS = [((24, 75, 75), (0, 0, 0), 48),   # a last row tile of few rows
+        ((20, 26, 77), (1, 0, 1), 100),  # one tile, wrapped halo columns
+        ((20, 29, 101), (0, 1, 0), 80),  # rows of more than three warps, wrapped halo rows
+        ((17, 36, 75), (1, 1, 1), 96)]   # everything wrapped
+
+
+@pytest.mark.parametrize('n_c,pbc,nb', ROWS + [
+    ((31, 31, 31), (0, 0, 0), 48),       # rows too short for the row kernel's copies
+    ((24, 75, 75), (0, 0, 0), 32),
+    ((40, 7, 33), (1, 0, 1), 80),
+    ((20, 29, 98), (0, 1, 0), 64),
+    ((17, 36, 21), (1, 1, 1), 96),
 ])
 @pytest.mark.parametrize('dtype', [torch.float64, torch.float32, torch.complex128,
                                    torch.complex64])
 @pytest.mark.parametrize('kind', ['laplace3', 'laplace1', 'gradient'])
 def test_row_stencil(n_c, pbc, nb, dtype, kind):
-    """Batches large enough for the row kernel: every band of apply equals
-    the marching kernel's result on that band alone, two bands equal the
-    oracle, and the potential is added (k-point batches of phases for
-    complex data)."""
+    """Every band of apply equals the result on that band alone (a call so
+    small that it marches), three bands equal the oracle, and the potential is
+    added (k-point batches of phases for complex data).  The batches of ROWS
+    take the row kernel, but for 7-point FP32 stencils, which march, and
+    complex128 without phases, whose rows suit the TMA kernel."""
     from gpaw_b200.fd_operators import Gradient, Laplace
     from gpaw_b200.grid_descriptor import GridDescriptor
     N = np.array(n_c) + (1 - np.array(pbc))
@@ -46,6 +53,13 @@ def test_row_stencil(n_c, pbc, nb, dtype, kind):
     ks = [(0.13, -0.21, 0.37), (0.4, 0.1, -0.3)]
     ph = np.array([bloch_phases(pbc, k) for k in ks]) if dtype.is_complex else None
     y, yv = torch.empty_like(x), torch.empty_like(x)
+    if (n_c, pbc, nb) in ROWS:
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            op.apply(x, y, ph)
+            torch.cuda.synchronize()
+        want = 'march_star_kernel' if kind == 'laplace1' and dtype == torch.float32 else \
+               'star_tma_kernel' if dtype == torch.complex128 and not any(pbc) else 'rows_star_kernel'
+        assert any(want in e.key for e in prof.key_averages())
     op.apply(x, y, ph)
     op.apply_potential(x, yv, v, ph)
     wide = np.complex128 if dtype.is_complex else np.float64
