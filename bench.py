@@ -708,7 +708,7 @@ def main():
     ap.add_argument('--no-scf', action='store_true',
                     help='skip the Si64 SCF time-to-solution comparison')
     ap.add_argument('--stencil-path', type=int, default=0,
-                    help='0 auto (TMA where possible), 1 cp.async kernel, 2 TMA only')
+                    help='0 auto (TMA where possible), 1 never TMA, 2 TMA only')
     ap.add_argument('--bands', type=int, default=NB,
                     help='grids per step (256 is the benchmark workload; smaller '
                          'values give the small case that ncu captures)')
@@ -798,10 +798,10 @@ def main():
         kernel = (f'star_tma_kernel<{cname},H=3,R1=2,R2=2>' if args.dtype == 'f64'
                   else f'star_tma_kernel<{cname},H=3,R1=2,R2=4>')
     except nat.GPAWB200Error:
-        kernel = f'star_kernel<{cname},H=3>'
+        kernel = f'rows_star_kernel<{cname},H=3>'
     nat.check(nat.lib().gb_set_stencil_path(args.stencil_path), 'stencil path')
     if args.stencil_path == 1:
-        kernel = f'star_kernel<{cname},H=3>'
+        kernel = f'rows_star_kernel<{cname},H=3>'
 
     for _ in range(max(args.warmup, 3)):
         lap.apply(x, y)

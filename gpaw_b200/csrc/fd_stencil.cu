@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 16 ? 2 : 3) march_star_kerne
   using R = typename Elem<T>::R;
   constexpr bool CPLX = Elem<T>::cplx;
   constexpr bool DIFF = sizeof(R) == 4;
-  constexpr int R1 = 1;                     // rows per thread (2 and 3 were slower: fewer warps)
   constexpr int NQ = 2 * H + 2;             // 2H + 1 planes in use, one on its way
+  // one row per thread (two and three were slower: fewer warps)
   const int n0 = a.n0, n1 = a.n1, n2 = a.n2;
   const int64_t n12 = (int64_t)n1 * n2;
   unsigned u0 = blockIdx.x;
@@ -98,32 +98,24 @@ __global__ void __launch_bounds__(256, sizeof(T) == 16 ? 2 : 3) march_star_kerne
   const int64_t band = u0 / a.chunks;
   const int64_t f = (int64_t)tile * 256 + threadIdx.x;
   int z;
-  const int y0 = (int)div_mod(f, n2, z) * R1;
-  if (y0 >= n1) return;
+  const int y = (int)div_mod(f, n2, z);
+  if (y >= n1) return;
   const int p_begin = (int)((int64_t)n0 * chunk / a.chunks), p_end = (int)((int64_t)n0 * (chunk + 1) / a.chunks);
 
-  const T* __restrict__ src = reinterpret_cast<const T*>(a.in) + band * n12 * n0 + ((int64_t)y0 * n2 + z);
+  const T* __restrict__ src = reinterpret_cast<const T*>(a.in) + band * n12 * n0 + f;
   const auto& PH = a.phs.ph[phase_set_of(a.phs, band)];
   const bool phased = CPLX && PER && a.phs.any;
 
-  // Row y0 + d relative to the thread's own point: the flat offset (wrapped on
-  // a periodic axis), whether it holds data, and whether it wraps
-  auto row = [&](int d, int64_t& off, bool& ok, int& side) {
-    const int y = y0 + d;
-    off = (int64_t)d * n2;
-    side = y < 0 ? 1 : y >= n1 ? 0 : -1;
-    ok = side < 0;
+  // value of the point's plane at row y + d / column z + d: wrapped on a
+  // periodic axis, zero outside the others
+  auto ld_row = [&](const T* c, int d) -> T {
+    int64_t off = (int64_t)d * n2;
+    const int side = y + d < 0 ? 1 : y + d >= n1 ? 0 : -1;
+    bool ok = side < 0;
     if (PER && a.pbc1 && !ok) {
       off += side ? n12 : -n12;
       ok = true;
     }
-  };
-  // value of the centre plane's row d (rows of the own block come from the queue)
-  auto ld_row = [&](const T* c, int d) -> T {
-    int64_t off;
-    int side;
-    bool ok;
-    row(d, off, ok, side);
     T v = zero<T>();
     if (ok) v = ld_nc(c + off);
     if (phased && side >= 0) v = phase_mul(v, PH[1][side][0], PH[1][side][1]);
@@ -143,106 +135,74 @@ __global__ void __launch_bounds__(256, sizeof(T) == 16 ? 2 : 3) march_star_kerne
     if (phased && side >= 0) v = phase_mul(v, PH[2][side][0], PH[2][side][1]);
     return v;
   };
-  // own block of plane j (any j; zero or wrapped outside the grid)
-  int64_t ooff[R1];
-  bool ook[R1];
-  int oside[R1];
-#pragma unroll
-  for (int r = 0; r < R1; ++r) row(r, ooff[r], ook[r], oside[r]);
-  auto ld_plane = [&](int j, T (&v)[R1]) {
+  // the point itself in plane j (any j; zero or wrapped outside the grid)
+  auto ld_plane = [&](int j) -> T {
     int side = j < 0 ? 1 : j >= n0 ? 0 : -1;
     bool in = side < 0;
     if (PER && a.pbc0 && !in) {
       j += side ? n0 : -n0;
       in = true;
     }
-    const T* c = src + (int64_t)j * n12;
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      v[r] = zero<T>();
-      if (in && ook[r]) v[r] = ld_nc(c + ooff[r]);
-      if (phased) {
-        if (oside[r] >= 0) v[r] = phase_mul(v[r], PH[1][oside[r]][0], PH[1][oside[r]][1]);
-        if (side >= 0) v[r] = phase_mul(v[r], PH[0][side][0], PH[0][side][1]);
-      }
-    }
+    T v = zero<T>();
+    if (in) v = ld_nc(src + (int64_t)j * n12);
+    if (phased && side >= 0) v = phase_mul(v, PH[0][side][0], PH[0][side][1]);
+    return v;
   };
 
   const bool epi = a.alpha != 1.0 || a.beta != 0.0 || a.y != nullptr || a.vpot != nullptr;
   const R c0 = DIFF ? (R)a.c0diff : (R)a.c0;
-  const int64_t obase = band * n12 * n0 + ((int64_t)y0 * n2 + z);
-  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + obase;
-  const T* __restrict__ ysrc = a.y ? reinterpret_cast<const T*>(a.y) + obase : nullptr;
-  const R* __restrict__ vsrc = a.vpot ? reinterpret_cast<const R*>(a.vpot) + ((int64_t)y0 * n2 + z) : nullptr;
+  T* __restrict__ dst = reinterpret_cast<T*>(a.out) + band * n12 * n0 + f;
+  const T* __restrict__ ysrc = a.y ? reinterpret_cast<const T*>(a.y) + band * n12 * n0 + f : nullptr;
+  const R* __restrict__ vsrc = a.vpot ? reinterpret_cast<const R*>(a.vpot) + f : nullptr;
 
   // q[(s + H) % NQ]: plane p_begin + s
-  T q[NQ][R1];
+  T q[NQ];
 #pragma unroll
-  for (int s = -H; s <= H; ++s) ld_plane(p_begin + s, q[s + H]);
+  for (int s = -H; s <= H; ++s) q[s + H] = ld_plane(p_begin + s);
   for (int pb = p_begin; pb < p_end; pb += NQ) {
 #pragma unroll
     for (int u = 0; u < NQ; ++u) {
       const int p = pb + u;
       if (p < p_end) {
-        if (p + 1 < p_end) ld_plane(p + 1 + H, q[(u + 2 * H + 1) % NQ]);
+        if (p + 1 < p_end) q[(u + 2 * H + 1) % NQ] = ld_plane(p + 1 + H);
         const int64_t po = (int64_t)p * n12;
         const T* c = src + po;
-        const int cu = (u + H) % NQ;
-        T yv[R1];
-        R vv[R1];
+        const T xc = q[(u + H) % NQ];
+        T yv;
+        R vv;
         if (epi) {
+          if (ysrc) yv = __ldcs(ysrc + po);
+          if (vsrc) vv = __ldg(vsrc + po);
+        }
+        T x = scale(c0, xc);
 #pragma unroll
-          for (int r = 0; r < R1; ++r) {
-            if (ysrc && y0 + r < n1) yv[r] = __ldcs(ysrc + po + r * n2);
-            if (vsrc && y0 + r < n1) vv[r] = __ldg(vsrc + po + r * n2);
+        for (int m = -H; m <= H; ++m) {
+          if constexpr (std::is_same<T, float>::value) {
+            if (m > 0)
+              x = star_pair<SYM>(x, (R)a.a[0][HMAX + m], (R)a.a[0][HMAX - m], q[(u + H + m + NQ) % NQ],
+                                 q[(u + H - m + NQ) % NQ], xc);
+          } else {
+            if (m) x = star_term(x, (R)a.a[0][m + HMAX], q[(u + H + m + NQ) % NQ], xc);
           }
         }
-        T acc[R1];
 #pragma unroll
-        for (int r = 0; r < R1; ++r) {
-          const T xc = q[cu][r];
-          T x = scale(c0, xc);
-#pragma unroll
-          for (int m = -H; m <= H; ++m) {
-            if constexpr (std::is_same<T, float>::value) {
-              if (m > 0)
-                x = star_pair<SYM>(x, (R)a.a[0][HMAX + m], (R)a.a[0][HMAX - m], q[(u + H + m + NQ) % NQ][r],
-                                   q[(u + H - m + NQ) % NQ][r], xc);
-            } else {
-              if (m) x = star_term(x, (R)a.a[0][m + HMAX], q[(u + H + m + NQ) % NQ][r], xc);
-            }
+        for (int m = -H; m <= H; ++m) {
+          if constexpr (std::is_same<T, float>::value) {
+            if (m > 0)
+              x = star_pair<SYM>(x, (R)a.a[2][HMAX + m], (R)a.a[2][HMAX - m], ld_col(c, m), ld_col(c, -m), xc);
+          } else {
+            if (m) x = star_term(x, (R)a.a[2][m + HMAX], ld_col(c, m), xc);
           }
-#pragma unroll
-          for (int m = -H; m <= H; ++m) {
-            if constexpr (std::is_same<T, float>::value) {
-              if (m > 0)
-                x = star_pair<SYM>(x, (R)a.a[2][HMAX + m], (R)a.a[2][HMAX - m], ld_col(c + ooff[r], m),
-                                   ld_col(c + ooff[r], -m), xc);
-            } else {
-              if (m) x = star_term(x, (R)a.a[2][m + HMAX], ld_col(c + ooff[r], m), xc);
-            }
-          }
-          acc[r] = x;
         }
 #pragma unroll
-        for (int d = -H; d < R1 + H; ++d) {
-          const T v = d >= 0 && d < R1 ? q[cu][d < 0 ? 0 : d < R1 ? d : 0] : ld_row(c, d);
-#pragma unroll
-          for (int r = 0; r < R1; ++r)
-            if (d != r && d - r >= -H && d - r <= H)
-              acc[r] = star_term(acc[r], (R)a.a[1][d - r + HMAX], v, q[cu][r]);
+        for (int d = -H; d <= H; ++d)
+          if (d) x = star_term(x, (R)a.a[1][d + HMAX], ld_row(c, d), xc);
+        if (epi) {
+          x = fmadd(scale((R)a.alpha, x), (R)a.beta, xc);
+          if (ysrc) x = fmadd(x, (R)a.gamma, yv);
+          if (vsrc) x = fmadd(x, vv, xc);
         }
-#pragma unroll
-        for (int r = 0; r < R1; ++r) {
-          if (y0 + r >= n1) continue;
-          T v = acc[r];
-          if (epi) {
-            v = fmadd(scale((R)a.alpha, v), (R)a.beta, q[cu][r]);
-            if (ysrc) v = fmadd(v, (R)a.gamma, yv[r]);
-            if (vsrc) v = fmadd(v, vv[r], q[cu][r]);
-          }
-          st_cs(dst + po + r * n2, v);
-        }
+        st_cs(dst + po, x);
       }
     }
   }

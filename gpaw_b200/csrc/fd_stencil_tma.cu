@@ -1,6 +1,7 @@
-// FD star stencil, TMA + warp-specialised pipeline (the default path on
-// sm_100a whenever the layout allows it; fd_stencil.cu keeps the cp.async
-// kernel for the other cases: odd row pitches, Bloch phases, radius > 4).
+// FD star stencil, TMA + warp-specialised pipeline: the default path whenever
+// the layout allows it (whole 16-byte chunks per row, no Bloch phases, radius
+// up to 4; fd_stencil_rows.cu, fd_stencil_tiles.cu and fd_stencil.cu take the
+// rest).
 //
 // Tile = a band of T1 full rows of the (axis1, axis2) plane: because a CTA
 // holds whole rows, the axis-2 halo of a periodic grid is read from the other
@@ -101,8 +102,6 @@ struct TmaArgs {
   double c0;
   double c0diff;    // c0 + sum of the neighbour coefficients (difference form)
   double a[3][2 * HMAX + 1];
-  float c0f, c0difff;
-  float af[3][2 * HMAX + 1];
   double alpha, beta, gamma;
 };
 
@@ -111,24 +110,6 @@ struct TmaArgs {
 // out-of-bounds fill (zeros); on a zero-boundary axis 2 the pitch keeps at
 // least 16 such bytes, and the halo chunks left of column 0 / right of column
 // n2 - 1 read them, so the consumers have no boundary branches at all.
-// shared-memory vector loads of VB bytes (16: float4, 8: float2)
-template <typename T, int N, int VB>
-__device__ __forceinline__ void ldv(const T* p, T (&v)[N]) {
-  if constexpr (VB == 16) {
-    lds_vec<T, N>(p, v);
-  } else {
-    constexpr int V = 8 / (int)sizeof(T);
-    static_assert(N % V == 0, "");
-#pragma unroll
-    for (int i = 0; i < N / V; ++i) {
-      const float2 x = *reinterpret_cast<const float2*>(p + i * V);
-      const T* e = reinterpret_cast<const T*>(&x);
-#pragma unroll
-      for (int k = 0; k < V; ++k) v[i * V + k] = e[k];
-    }
-  }
-}
-
 // N consecutive elements from global memory, zeros if !on: 16-byte loads when
 // N elements make whole 16-byte chunks (the caller guarantees the alignment)
 template <typename V, int N>
@@ -164,14 +145,14 @@ __device__ __forceinline__ void st_run_if(T* p, const T (&v)[N], bool on) {
   }
 }
 
-template <typename T, int H, int R1, int R2, int VB, int SYM, int EPI>
+template <typename T, int H, int R1, int R2, int SYM, int EPI>
 __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ CUtensorMap tmA,
                                                         const __grid_constant__ CUtensorMap tmH,
                                                         const __grid_constant__ CUtensorMap tmB,
                                                         const __grid_constant__ CUtensorMap tmL,
                                                         const __grid_constant__ TmaArgs a) {
   using R = typename Elem<T>::R;
-  constexpr int VEC = VB / (int)sizeof(T);   // elements per vector access
+  constexpr int VEC = 16 / (int)sizeof(T);   // elements per vector access
   constexpr int HZ = ((H + VEC - 1) / VEC) * VEC;
   constexpr int NQ = 2 * H + 1;
   // the epilogue's operands are on their way before the sums, except where the
@@ -328,7 +309,7 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
         const unsigned char* P = slots + (int64_t)slot * a.slot_bytes;
 #pragma unroll
         for (int r = 0; r < R1; ++r)
-          ldv<T, R2, VB>(reinterpret_cast<const T*>(P + own_row + r * pitch + own_col), q[u][r]);
+          lds_vec<T, R2>(reinterpret_cast<const T*>(P + own_row + r * pitch + own_col), q[u][r]);
 
         if (t >= 2 * H) {
           const int cu = (u + NQ - H) % NQ;     // centre plane in the queue (static after unrolling)
@@ -339,17 +320,17 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
               [&](int r, T(&w)[HZ]) {
 #pragma unroll
                 for (int ch = 0; ch < HZ / VEC; ++ch)
-                  ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + lcol[ch] + r * pitch),
+                  lds_vec<T, VEC>(reinterpret_cast<const T*>(Pc + lcol[ch] + r * pitch),
                                   *reinterpret_cast<T(*)[VEC]>(&w[ch * VEC]));
               },
               [&](int r, T(&w)[HZ]) {
 #pragma unroll
                 for (int ch = 0; ch < HZ / VEC; ++ch)
-                  ldv<T, VEC, VB>(reinterpret_cast<const T*>(Pc + rcol[ch] + r * pitch),
+                  lds_vec<T, VEC>(reinterpret_cast<const T*>(Pc + rcol[ch] + r * pitch),
                                   *reinterpret_cast<T(*)[VEC]>(&w[ch * VEC]));
               },
               [&](int rr, T(&v)[R2]) {
-                if (rr < 0 || rr >= R1) ldv<T, R2, VB>(reinterpret_cast<const T*>(Pc + own_row + rr * pitch + own_col), v);
+                if (rr < 0 || rr >= R1) lds_vec<T, R2>(reinterpret_cast<const T*>(Pc + own_row + rr * pitch + own_col), v);
               },
               [](int, int, T v) { return v; });
           // epilogue + streaming stores
@@ -395,13 +376,13 @@ __global__ void __launch_bounds__(512) star_tma_kernel(const __grid_constant__ C
 }
 
 // ------------------------------------------------------------------ host
-template <typename T, int H, int R1, int R2, int VB, int SYM, int EPI>
+template <typename T, int H, int R1, int R2, int SYM, int EPI>
 static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int64_t nin, cudaStream_t st,
                           const Epilogue& ep) {
   using R = typename Elem<T>::R;
   const int n0 = (int)op->n[0], n1 = (int)op->n[1], n2 = (int)op->n[2];
   const int TZ = n2 / R2;
-  auto kern = star_tma_kernel<T, H, R1, R2, VB, SYM, EPI>;
+  auto kern = star_tma_kernel<T, H, R1, R2, SYM, EPI>;
   static int regs = -1;
   if (regs < 0) {
     cudaFuncAttributes fa;
@@ -493,10 +474,6 @@ static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int6
     for (int cc = 0; cc < 3; ++cc)
       for (int m = 0; m < 2 * HMAX + 1; ++m) a.c0diff += op->a[cc][m];
     memcpy(a.a, op->a, sizeof(a.a));
-    a.c0f = (float)a.c0;
-    a.c0difff = (float)a.c0diff;
-    for (int cc = 0; cc < 3; ++cc)
-      for (int m = 0; m < 2 * HMAX + 1; ++m) a.af[cc][m] = (float)op->a[cc][m];
     a.alpha = ep.alpha; a.beta = ep.beta; a.gamma = ep.gamma;
     const size_t smem = 256 + 128 + (size_t)a.NS * a.slot_bytes;
     // tensor maps over (n2 scalars, n1, n0, nbatch); the box spans the whole
@@ -535,8 +512,8 @@ static int launch_tma_cfg(const gb_operator* op, const void* in, void* out, int6
   // fails, the model's best candidate is used without tuning.
   const int epi_kind = (ep.vpot ? 4 : 0) | (ep.y ? 2 : 0) | ((ep.alpha != 1.0 || ep.beta != 0.0) ? 1 : 0);
   char keyb[160];
-  snprintf(keyb, sizeof keyb, "%d:%d:%d:%d:%d:%d:%d:%d:%d:%d:%d:%lld", (int)sizeof(T), Elem<T>::cplx ? 1 : 0, H, n0,
-           n1, n2, op->pbc[0] * 4 + op->pbc[1] * 2 + op->pbc[2], epi_kind, (int)VB, R2, SYM, (long long)nin);
+  snprintf(keyb, sizeof keyb, "%d:%d:%d:%d:%d:%d:%d:%d:%d:%d:%lld", (int)sizeof(T), Elem<T>::cplx ? 1 : 0, H, n0,
+           n1, n2, op->pbc[0] * 4 + op->pbc[1] * 2 + op->pbc[2], epi_kind, R2, SYM, (long long)nin);
   const std::string key(keyb);
   int choice = -1;
   {
@@ -605,13 +582,13 @@ static int launch_tma(const gb_operator* op, const void* in, void* out, int64_t 
                       const Epilogue& ep) {
   const int epi = ep.y || ep.alpha != 1.0 || ep.beta != 0.0 ? 2 : ep.vpot ? 1 : 0;
   if constexpr (H == 1 && SYM == 1) {
-    if (epi < 2) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 1>(op, in, out, nin, st, ep);
+    if (epi < 2) return launch_tma_cfg<T, H, 2, R2, SYM, 1>(op, in, out, nin, st, ep);
   } else {
-    if (epi == 0) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 0>(op, in, out, nin, st, ep);
+    if (epi == 0) return launch_tma_cfg<T, H, 2, R2, SYM, 0>(op, in, out, nin, st, ep);
     if constexpr ((H == 3 && SYM == 1) || (H == 4 && SYM >= 0))
-      if (epi == 1) return launch_tma_cfg<T, H, 2, R2, 16, SYM, 1>(op, in, out, nin, st, ep);
+      if (epi == 1) return launch_tma_cfg<T, H, 2, R2, SYM, 1>(op, in, out, nin, st, ep);
   }
-  return launch_tma_cfg<T, H, 2, R2, 16, SYM, 2>(op, in, out, nin, st, ep);
+  return launch_tma_cfg<T, H, 2, R2, SYM, 2>(op, in, out, nin, st, ep);
 }
 
 template <typename T, int R2>
@@ -645,13 +622,13 @@ static int dispatch_tma(const gb_operator* op, const void* in, void* out, int64_
   }
 }
 
-static int g_stencil_path = 0;   // 0 auto, 1 cp.async only, 2 TMA required
+static int g_stencil_path = 0;   // 0 automatic, 1 never TMA, 2 TMA required
 const char* tma_reason() { return g_tma_reason; }
 
 int star_tma_apply(const gb_operator* op, const void* in, void* out, int64_t nin, int dtype, const double* ph,
                    cudaStream_t st, const Epilogue& ep, int nk) {
   g_tma_reason = "";
-  if (g_stencil_path == 1) { g_tma_reason = "cp.async path forced"; return 1; }
+  if (g_stencil_path == 1) { g_tma_reason = "TMA path switched off"; return 1; }
   if (!op->cfd || op->H > 4) { g_tma_reason = "stencil not on axes or radius > 4"; return 1; }
   if (ph) {
     for (int i = 0; i < 6 * (nk > 1 ? nk : 1); ++i)

@@ -1,7 +1,8 @@
 // TMA (cp.async.bulk.tensor) and mbarrier helpers for sm_100a, written as
-// inline PTX.  Every wait is bounded: after WAIT_LIMIT polls the caller gets
-// `false`, records an error code in a device flag and leaves, so a fault in
-// the pipeline protocol can never hang the GPU.
+// inline PTX.  Every wait is bounded: after WAIT_LIMIT_HINT polls (WAIT_LIMIT
+// where a caller polls by itself) the caller gets `false`, records an error
+// code in a device flag and leaves, so a fault in the pipeline protocol can
+// never hang the GPU.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -1,5 +1,6 @@
-"""Both stencil kernels (the cp.async kernel and the TMA pipeline) against
-the oracle on layouts where both apply, plus the bounded-wait error flag."""
+"""The TMA stencil and the kernels that serve without it (rows, marching)
+against the oracle on layouts where both apply, plus the bounded-wait error
+flag."""
 import ctypes
 
 import numpy as np
