@@ -57,7 +57,7 @@ def peaks():
 # (dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture of a 64-grid
 # launch of the same kernel, divided by 64; the capture is summarised in
 # profiles/star_tma_kernel_f64_laplace_96cubed.txt)
-STENCIL_TRAFFIC_PER_GRID = 16.35e6
+STENCIL_TRAFFIC_PER_GRID = 16.32e6
 
 
 def profiled_traffic(nb):

@@ -15,12 +15,13 @@
 // the centre plane.  Ring: H + 1 planes in use and two on their way, one
 // barrier per plane (deeper rings measured the same).
 //
-// Bound by issue slots, 107 per 32 points in FP64, and by instruction fetch
-// (the 32 x 32 tiles it replaces spent most of theirs on addresses, boundaries
-// and the unused part of edge tiles): (160, 75^3) FP64 zero boundary 1080 ->
-// 433 us (2.5 TB/s), with a potential 1680 -> 506 us; FP32 768 -> 305 us;
-// (64, 60^3) complex128 with phases 597 -> 225 us, all before the compute part
-// alone was unrolled.
+// On 60 FP64 grids of 75^3 the shared-memory data pipe is 62 % busy, issue
+// slots 49 % (111 instructions per 32 points), DRAM 33 %: 16 warps per SM wait
+// for their shared-memory reads.  (The 32 x 32 tiles before it spent most
+// instructions on addresses, boundaries and the unused part of edge tiles:
+// (160, 75^3) FP64 zero boundary 1080 -> 433 us, with a potential 1680 -> 506
+// us; FP32 768 -> 305 us; (64, 60^3) complex128 with phases 597 -> 225 us, all
+// before the compute part alone was unrolled.)
 #include <algorithm>
 #include <cstring>
 #include "star_core.cuh"
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(ROWS_NT, 2) rows_star_kernel(const __grid_cons
   using R = typename Elem<T>::R;
   using C = RowsCfg<T, H>;
   constexpr bool CPLX = Elem<T>::cplx;
-    constexpr int VEC = C::VEC, R2 = C::R2, HZ = C::HZ, D = C::D, NS = C::NS;
+  constexpr int VEC = C::VEC, R2 = C::R2, HZ = C::HZ, D = C::D, NS = C::NS;
   constexpr int NQ = 2 * H + 1;
   constexpr int RPW = RowsCfg<T, H>::RPW;
   extern __shared__ __align__(16) unsigned char smem_raw[];

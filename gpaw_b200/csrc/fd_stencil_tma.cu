@@ -19,12 +19,16 @@
 // through an mbarrier when its last reader is done.  All waits are bounded
 // (tma.cuh).
 //
-// Bound by issue slots more than by HBM: 78 instructions per 32 FP64 points
-// (19 points, radius 3), 94 before the coefficients stayed in registers, the
-// stores and epilogue loads became predicated and the loads moved ahead of
-// the wait.  256 x 96^3 FP64 803 -> 715 us (5.1 of the measured 6.55 TB/s),
-// with a potential 1557 -> 1030 us; 160 x 56^3 FP32 with a potential 120 ->
-// 81 us.  One row per thread instead of two (more warps) was 11 % slower.
+// No one unit is full on 64 FP64 grids of 96^3 (19 points, radius 3): the
+// shared-memory data pipe 72 %, DRAM 69 %, issue slots 55 %, FP64 arithmetic
+// 40 %; warps wait for their shared-memory reads, and DRAM delivers 1.41 times
+// the input, since a CTA reaches the neighbouring row tile a whole column of
+// planes later, when its halo rows have left L2.  Keeping the coefficients in
+// registers, predicating the stores and epilogue loads and issuing the loads
+// ahead of the wait took 118 -> 97 M warp instructions there; (256, 96^3) FP64
+// back to back 779 -> 726 us (5.0 of the measured 6.55 TB/s), with a potential
+// 1557 -> 1030 us; 160 x 56^3 FP32 with a potential 120 -> 81 us.  One row per
+// thread instead of two (more warps) was 11 % slower.
 #include <algorithm>
 #include <cstring>
 #include <cstdio>

@@ -18,8 +18,8 @@ namespace gb {
 // A value the compiler must keep in a register.  sm_100 arithmetic takes
 // constants through the uniform registers, and the FP64 and packed FP32
 // instructions need them moved to ordinary ones first: re-read from the
-// parameter bank the 19-point FP64 kernel spent 14 of its 94 instructions
-// per 32 points on such moves, with every unit but the issue slots idle.
+// parameter bank the 19-point FP64 kernel spent a seventh of its instructions
+// on such moves.
 __device__ __forceinline__ double in_register(double v) {
   asm volatile("" : "+d"(v));
   return v;

@@ -50,8 +50,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // bounded wait on phase `parity`; false on timeout.  The suspend hint lets
-// the hardware park the warp until the phase completes: polling warps of the
-// marching stencil took 7 of its 94 issue slots per 32 points.
+// the hardware park the warp until the phase completes: polls took about one
+// in thirteen issue slots of the FP64 stencil.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = (uint32_t)__cvta_generic_to_shared(bar);
   for (int i = 0; i < WAIT_LIMIT_HINT; ++i) {
